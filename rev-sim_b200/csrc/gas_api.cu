@@ -59,13 +59,14 @@ struct revsim_gas_handle {
     double fwd_dt = 0, fwd_gamma = 0;
     std::vector<double> centres, Eloss, Rloss;
     bool fwd_has_E = false, fwd_has_R = false;
-    // RDF term of the water atoms: the terms, their targets and scratch (histogram with the
-    // normaliser behind it, dL/dh), the one-box table {atom0, n_mol} / box, dL/dx of the
+    // RDF term of the water atoms: the terms, their targets and scratch (slice sums with the
+    // normaliser behind them, gradient weights), the one-box table {atom0, n_mol} / box, dL/dx of the
     // water atoms, and the per-loss-point losses of the forward pass
     struct RdfDev {
         revsim_rdf_term t;
         int off = 0;
-        double *d_target = nullptr, *d_hist = nullptr, *d_dLdh = nullptr;
+        double *d_target = nullptr, *d_sum = nullptr, *d_wt = nullptr;   // d_sum: slice sums, then pre
+        rs::RdfDen den;
     };
     std::vector<RdfDev> rdf;
     int *d_rdf_int = nullptr;
@@ -438,8 +439,8 @@ int ensure_eloss(revsim_gas_handle *h, size_t n) {
 void free_rdf(revsim_gas_handle *h) {
     for (auto &T : h->rdf) {
         if (T.d_target) cudaFree(T.d_target);
-        if (T.d_hist) cudaFree(T.d_hist);
-        if (T.d_dLdh) cudaFree(T.d_dLdh);
+        if (T.d_sum) cudaFree(T.d_sum);
+        if (T.d_wt) cudaFree(T.d_wt);
     }
     h->rdf.clear();
 }
@@ -450,7 +451,6 @@ void free_rdf(revsim_gas_handle *h) {
 int rdf_point(revsim_gas_handle *h, bool grad, double *d_loss) {
     for (auto &T : h->rdf) {
         const revsim_rdf_term &t = T.t;
-        CK(cudaMemsetAsync(T.d_hist, 0, sizeof(double) * t.n_grid, h->st));
         rs::RdfArgs a;
         a.x = h->d_x;
         a.rep_atom0 = h->d_rdf_int;
@@ -464,18 +464,15 @@ int rdf_point(revsim_gas_handle *h, bool grad, double *d_loss) {
         a.cutoff = t.exp_cutoff;
         a.n_grid = t.n_grid;
         a.off = T.off;
-        a.hist = T.d_hist;
-        a.dLdh = T.d_dLdh;
+        a.hist = nullptr;
         a.dLdx = h->d_rdf_dx;
         const int n1 = t.sel1 == 0 ? h->nw : 2 * h->nw, n2 = t.sel2 == 0 ? h->nw : 2 * h->nw;
-        CK(rs::launch_rdf(a, 1, n1, n2, false, h->st));
-        CK(rs::launch_rdf_finalize(a, 1, T.d_hist + t.n_grid, T.d_target, t.slice_start, t.slice_stride,
-                                   t.n_target, t.norm, t.weight, d_loss, T.d_dLdh, h->st));
-        h->launches += 2;
-        if (grad) {
-            CK(rs::launch_rdf(a, 1, n1, n2, true, h->st));
-            h->launches++;
-        }
+        rs::RdfSlice sl = rs::rdf_slice(t.slice_start, t.slice_stride, t.n_target, t.step, t.width, t.exp_cutoff);
+        sl.sum = T.d_sum;
+        sl.wt = T.d_wt;
+        CK(rs::launch_rdf_loss(a, sl, T.den, 1, n1, n2, T.d_sum + t.n_target, T.d_target, t.norm, t.weight, grad,
+                               d_loss, h->st));
+        h->launches += grad ? 3 : 2;
     }
     return REVSIM_OK;
 }
@@ -688,18 +685,19 @@ int32_t revsim_gas_set_rdf(revsim_gas_handle *h, int32_t n_terms, const revsim_r
         revsim_gas_handle::RdfDev T;
         T.t = t;
         T.off = (int)std::llround(t.x_min / t.step) - 1;
+        T.den = rs::rdf_den_poly(t.step, t.width, t.exp_cutoff);
         h->rdf.push_back(T);
         auto &D = h->rdf.back();
-        if (dalloc(&D.d_target, t.n_target) != cudaSuccess || dalloc(&D.d_hist, (size_t)t.n_grid + 1) != cudaSuccess ||
-            dalloc(&D.d_dLdh, t.n_grid) != cudaSuccess) {
+        if (dalloc(&D.d_target, t.n_target) != cudaSuccess || dalloc(&D.d_sum, (size_t)t.n_target + 1) != cudaSuccess ||
+            dalloc(&D.d_wt, t.n_target) != cudaSuccess) {
             free_rdf(h);
             return fail(h, REVSIM_ERR_NOMEM, "RDF scratch");
         }
-        // the normaliser V / (4 pi n1 n2 step) behind the histogram (rdf_differentiable, 725)
+        // the normaliser V / (4 pi n1 n2 step) behind the slice sums (rdf_differentiable, 725)
         const double n1 = t.sel1 == 0 ? h->nw : 2.0 * h->nw, n2 = t.sel2 == 0 ? h->nw : 2.0 * h->nw;
         const double pre = h->L * h->L * h->L / (4 * pi * n1 * n2 * t.step);
         CK(cudaMemcpy(D.d_target, targets[i], sizeof(double) * t.n_target, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(D.d_hist + t.n_grid, &pre, sizeof(double), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(D.d_sum + t.n_target, &pre, sizeof(double), cudaMemcpyHostToDevice));
     }
     return REVSIM_OK;
 }

@@ -50,7 +50,8 @@ struct Term {
     int off;
     double *d_target = nullptr;   // [R * n_target]
     double *d_hist = nullptr;     // [R * n_grid + R]  (histogram, then pre[R])
-    double *d_dLdh = nullptr;     // [R * n_grid]
+    double *d_wt = nullptr;       // [R * n_target] gradient weights of the slice points
+    RdfDen den;
 };
 
 }  // namespace
@@ -720,6 +721,29 @@ int enth_dev(revsim_handle *h, double *acc, double *ev_acc, bool grad_x, bool gr
     return REVSIM_OK;
 }
 
+RdfArgs rdf_args(revsim_handle *h, const Term &T, int &n1, int &n2) {
+    const revsim_rdf_term &t = T.t;
+    RdfArgs a;
+    a.x = h->d_x;
+    a.rep_atom0 = h->d_rep_atom0;
+    a.rep_nmol = h->d_rep_nmol;
+    a.rep_box = h->d_rep_box;
+    a.sel1 = t.sel1;
+    a.sel2 = t.sel2;
+    a.x_min = t.x_min;
+    a.step = t.step;
+    a.width = t.width;
+    a.cutoff = t.exp_cutoff;
+    a.n_grid = t.n_grid;
+    a.off = T.off;
+    a.hist = T.d_hist;
+    a.dLdx = h->d_dLdx;
+    const int mx = *std::max_element(h->nmol.begin(), h->nmol.end());
+    n1 = t.sel1 == 0 ? mx : 2 * mx;
+    n2 = t.sel2 == 0 ? mx : 2 * mx;
+    return a;
+}
+
 // loss_fn / loss_and_grads at the current positions: adds the per-replica loss to acc
 // (device [R]) and the enthalpy part to ev_acc (may be null); if grad writes dL/dx into
 // d_dLdx; if grad_p adds the enthalpy term's direct parameter gradient to d_ev_grad /
@@ -728,33 +752,14 @@ int loss_dev(revsim_handle *h, bool grad, double *acc, double *ev_acc = nullptr,
     if (grad) CK(cudaMemsetAsync(h->d_dLdx, 0, sizeof(double) * 3 * (size_t)h->N, h->st));
     for (Term &T : h->terms) {
         const revsim_rdf_term &t = T.t;
-        RdfArgs a;
-        a.x = h->d_x;
-        a.rep_atom0 = h->d_rep_atom0;
-        a.rep_nmol = h->d_rep_nmol;
-        a.rep_box = h->d_rep_box;
-        a.sel1 = t.sel1;
-        a.sel2 = t.sel2;
-        a.x_min = t.x_min;
-        a.step = t.step;
-        a.width = t.width;
-        a.cutoff = t.exp_cutoff;
-        a.n_grid = t.n_grid;
-        a.off = T.off;
-        a.hist = T.d_hist;
-        a.dLdh = T.d_dLdh;
-        a.dLdx = h->d_dLdx;
-        int mx = *std::max_element(h->nmol.begin(), h->nmol.end());
-        const int n1 = t.sel1 == 0 ? mx : 2 * mx, n2 = t.sel2 == 0 ? mx : 2 * mx;
-        CK(cudaMemsetAsync(T.d_hist, 0, sizeof(double) * (size_t)h->R * t.n_grid, h->st));
-        CK(launch_rdf(a, h->R, n1, n2, false, h->st));
-        CK(launch_rdf_finalize(a, h->R, T.d_hist + (size_t)h->R * t.n_grid, T.d_target, t.slice_start,
-                               t.slice_stride, t.n_target, t.norm, t.weight, acc, T.d_dLdh, h->st));
-        h->launches += 2;
-        if (grad) {
-            CK(launch_rdf(a, h->R, n1, n2, true, h->st));
-            h->launches++;
-        }
+        int n1, n2;
+        const RdfArgs a = rdf_args(h, T, n1, n2);
+        RdfSlice sl = rdf_slice(t.slice_start, t.slice_stride, t.n_target, t.step, t.width, t.exp_cutoff);
+        sl.sum = T.d_hist;   // n_target <= n_grid entries of it
+        sl.wt = T.d_wt;
+        CK(launch_rdf_loss(a, sl, T.den, h->R, n1, n2, T.d_hist + (size_t)h->R * t.n_grid, T.d_target, t.norm,
+                           t.weight, grad, acc, h->st));
+        if (t.n_target > 0) h->launches += grad ? 3 : 2;
     }
     if (h->ev_on) return enth_dev(h, acc, ev_acc, grad, grad_p);
     return REVSIM_OK;
@@ -1160,7 +1165,7 @@ void free_all(revsim_handle *h) {
     for (Term &T : h->terms) {
         dfree(T.d_target);
         dfree(T.d_hist);
-        dfree(T.d_dLdh);
+        dfree(T.d_wt);
     }
     for (int w = 0; w < 2; w++)
         for (cudaEvent_t e : h->ev[w]) cudaEventDestroy(e);
@@ -1459,7 +1464,7 @@ int32_t revsim_set_loss(revsim_handle *h, int32_t n_terms, const revsim_rdf_term
     for (Term &T : h->terms) {
         dfree(T.d_target);
         dfree(T.d_hist);
-        dfree(T.d_dLdh);
+        dfree(T.d_wt);
     }
     h->terms.clear();
     for (int i = 0; i < n_terms; i++) {
@@ -1478,12 +1483,13 @@ int32_t revsim_set_loss(revsim_handle *h, int32_t n_terms, const revsim_rdf_term
         Term T;
         T.t = t;
         T.off = (int)std::llround(q) - 1;
+        T.den = rdf_den_poly(t.step, t.width, t.exp_cutoff);
         if (dalloc(&T.d_target, (size_t)h->R * std::max(t.n_target, 1)) != cudaSuccess ||
             dalloc(&T.d_hist, (size_t)h->R * t.n_grid + h->R) != cudaSuccess ||
-            dalloc(&T.d_dLdh, (size_t)h->R * t.n_grid) != cudaSuccess) {
+            dalloc(&T.d_wt, (size_t)h->R * std::max(t.n_target, 1)) != cudaSuccess) {
             dfree(T.d_target);
             dfree(T.d_hist);
-            dfree(T.d_dLdh);
+            dfree(T.d_wt);
             return fail(h, REVSIM_ERR_NOMEM, "loss buffers");
         }
         h->terms.push_back(T);
@@ -1771,16 +1777,12 @@ int32_t revsim_rdf(revsim_handle *h, int32_t term, int32_t replica, double *hist
         return REVSIM_ERR_BADARG;
     if (!h->have_state) return fail(h, REVSIM_ERR_STATE, "state not set");
     CK(cudaSetDevice(h->dev));
-    std::vector<Term> keep = h->terms;
-    const bool ev = h->ev_on;
-    h->terms.assign(1, keep[term]);
-    h->ev_on = false;
-    CK(cudaMemsetAsync(h->d_loss, 0, sizeof(double) * h->R, h->st));
-    int rc = loss_dev(h, false, h->d_loss);
-    h->terms = keep;
-    h->ev_on = ev;
-    if (rc) return rc;
     const Term &T = h->terms[term];
+    int n1, n2;
+    const RdfArgs a = rdf_args(h, T, n1, n2);
+    CK(cudaMemsetAsync(T.d_hist, 0, sizeof(double) * (size_t)h->R * T.t.n_grid, h->st));
+    CK(launch_rdf(a, h->R, n1, n2, T.d_hist + (size_t)h->R * T.t.n_grid, h->st));
+    h->launches += 2;
     CK(cudaMemcpyAsync(hist, T.d_hist + (size_t)replica * T.t.n_grid, sizeof(double) * T.t.n_grid,
                        cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));

@@ -190,10 +190,26 @@ struct RdfArgs {
     int sel1, sel2;
     double x_min, step, width, cutoff;
     int n_grid, off;
-    double *hist;      // [R * n_grid] raw sums, then h
-    const double *dLdh; // [R * n_grid]
+    double *hist;      // [R * n_grid] raw sums, then h (the whole histogram only)
     double *dLdx;      // [3N]
 };
+
+// The grid points a loss term reads, s0 + t sd for t < nt: their sums and, after the value
+// pass, their gradient weights dL/dh pre / x^2.  recur: consecutive slice points' Gaussians
+// may follow from one another (the ratio stays finite).
+struct RdfSlice {
+    int s0, sd, nt, recur;
+    double *sum, *wt;   // [R * nt] each
+};
+
+// The normaliser den(d) of a pair whose window the grid does not clip, as a polynomial in d's
+// offset from the middle of its grid cell, one per window (rdf_den_poly in rs_loss.cu).
+struct RdfDen {
+    static constexpr int kMaxTerms = 16;
+    int n, M;   // floor(cutoff / step); terms (0: no polynomial, sum the window)
+    double c[4][kMaxTerms];
+};
+RdfDen rdf_den_poly(double step, double width, double cutoff);
 
 // The RDF kernels form consecutive Gaussians by a recurrence whose ratio at a window's
 // anchor is exp(-(2 e step + step^2) / width) with |e| <= exp_cutoff + 2 step; it must stay
@@ -202,6 +218,10 @@ struct RdfArgs {
 inline bool rdf_term_recurrence_ok(double step, double width, double exp_cutoff) {
     const double worst = (2.0 * (exp_cutoff + 2.0 * step) * step + step * step) / width;
     return worst <= 700.0;
+}
+
+inline RdfSlice rdf_slice(int s0, int sd, int nt, double step, double width, double exp_cutoff) {
+    return RdfSlice{s0, sd, nt, rdf_term_recurrence_ok(sd * step, width, exp_cutoff) ? 1 : 0, nullptr, nullptr};
 }
 
 // Launchers (return cudaError_t of the launch).
@@ -321,10 +341,11 @@ cudaError_t launch_noise(int N, const int *atom_rep, const int *rep_atom0, const
                          const double *rep_sdH, const uint64_t *seeds, double *xi,
                          cudaStream_t st);
 
-cudaError_t launch_rdf(const RdfArgs &a, int R, int max_n1, int max_n2, bool grad,
-                       cudaStream_t st);
-cudaError_t launch_rdf_finalize(const RdfArgs &a, int R, const double *pre, const double *target,
-                                int slice_start, int slice_stride, int n_target, int norm,
-                                double weight, double *loss, double *dLdh, cudaStream_t st);
+// The whole histogram h of every replica (hist cleared by the caller).
+cudaError_t launch_rdf(const RdfArgs &a, int R, int max_n1, int max_n2, const double *pre, cudaStream_t st);
+// One term's loss added to loss [R] and, when grad, dL/dx added to a.dLdx.
+cudaError_t launch_rdf_loss(const RdfArgs &a, const RdfSlice &sl, const RdfDen &dn, int R, int max_n1, int max_n2,
+                            const double *pre, const double *target, int norm, double weight, bool grad,
+                            double *loss, cudaStream_t st);
 
 }  // namespace rs

@@ -8,8 +8,10 @@
 // The loss (loss_rdf_part, water.jl:693-697) compares a strided slice of h with a
 // target; the gradient is the analytic derivative of the same windowed sums (the
 // quantity Enzyme differentiates in the reference's pullback, water.jl:715-736).
-// One thread per ordered atom pair, shared-memory histogram, FP64 throughout; the window's
-// Gaussians by a two-multiplication recurrence re-anchored on exp every 16 points.
+// The loss and its gradient read h at the slice points only, so the loss kernels (k_rdf_loss)
+// smear only the pairs those points can see onto those points; the whole histogram
+// (revsim_rdf) is k_rdf's.  FP64 throughout; the window's Gaussians by a two-multiplication
+// recurrence re-anchored on exp every 16 points.
 #include <cmath>
 #include <mutex>
 
@@ -62,11 +64,12 @@ struct Gauss {
     double g, r;
 };
 
-__device__ __forceinline__ void gauss_anchor(const RdfArgs &a, double d, int k, double inv_w,
+// S: the spacing of the points the recurrence visits (a grid step, or a slice stride).
+__device__ __forceinline__ void gauss_anchor(const RdfArgs &a, double d, int k, double S, double inv_w,
                                              Gauss &G) {
     const double e = __dsub_rn(grid_x(a, k), d);
     G.g = exp(-__dmul_rn(__dmul_rn(e, e), inv_w));
-    G.r = exp(-__dmul_rn(__fma_rn(__dmul_rn(2.0, e), a.step, __dmul_rn(a.step, a.step)), inv_w));
+    G.r = exp(-__dmul_rn(__fma_rn(__dmul_rn(2.0, e), S, __dmul_rn(S, S)), inv_w));
 }
 
 __device__ __forceinline__ void gauss_next(Gauss &G, double q) {
@@ -81,7 +84,7 @@ __device__ __forceinline__ void den_sums(const RdfArgs &a, double d, double inv_
     double s = 0.0, ds = 0.0;
     Gauss G{0.0, 0.0};
     for (int k = lo; k <= hi; k++) {
-        if (((k - lo) % kGaussAnchor) == 0) gauss_anchor(a, d, k, inv_w, G);
+        if (((k - lo) % kGaussAnchor) == 0) gauss_anchor(a, d, k, a.step, inv_w, G);
         const double e = __dsub_rn(grid_x(a, k), d);
         s = __dadd_rn(s, G.g);
         ds = __fma_rn(__dmul_rn(__dmul_rn(G.g, 2.0), e), inv_w, ds);
@@ -91,8 +94,30 @@ __device__ __forceinline__ void den_sums(const RdfArgs &a, double d, double inv_
     dden = ds;
 }
 
-template <bool GRAD>
-__global__ void k_rdf(RdfArgs a, const double *pre) {
+// The same sums from the polynomial of the pair's window (RdfDen); false where the window is
+// clipped by the grid, is not one of the four of an unclipped pair, or there is no polynomial.
+__device__ __forceinline__ bool den_poly(const RdfArgs &a, const RdfDen &dn, double d, double &den, double &dden) {
+    if (dn.M == 0) return false;
+    const long long s = (long long)ceil(__ddiv_rn(__dsub_rn(d, a.cutoff), a.step));
+    const long long e = (long long)floor(__ddiv_rn(__dadd_rn(d, a.cutoff), a.step));
+    if (s - a.off < 1 || e - a.off > a.n_grid) return false;
+    const double j = floor(__ddiv_rn(d, a.step));
+    const int ca = (int)(s - (long long)j) + dn.n, cb = (int)(e - (long long)j) - dn.n;
+    if (ca < 0 || ca > 1 || cb < 0 || cb > 1) return false;
+    const double u = __dsub_rn(d, __dmul_rn(__dadd_rn(j, 0.5), a.step));
+    const double *c = dn.c[2 * ca + cb];
+    double v = c[dn.M - 1], dv = 0.0;
+    for (int m = dn.M - 2; m >= 0; m--) {
+        dv = __fma_rn(dv, u, v);
+        v = __fma_rn(v, u, c[m]);
+    }
+    den = v;
+    dden = dv;
+    return true;
+}
+
+// The whole histogram: one thread per ordered atom pair, shared-memory histogram.
+__global__ void k_rdf(RdfArgs a) {
     extern __shared__ double s_hist[];
     const int r = blockIdx.y;
     const int nm = a.rep_nmol[r];
@@ -100,7 +125,7 @@ __global__ void k_rdf(RdfArgs a, const double *pre) {
     const long long n1 = a.sel1 == 0 ? nm : 2LL * nm;
     const long long n2 = a.sel2 == 0 ? nm : 2LL * nm;
     const double L = a.rep_box[r];
-    const bool use_smem = !GRAD && a.n_grid <= 6144;
+    const bool use_smem = a.n_grid <= 6144;
     double *hist = a.hist + (size_t)r * a.n_grid;
     if (use_smem) {
         for (int k = threadIdx.x; k < a.n_grid; k += blockDim.x) s_hist[k] = 0.0;
@@ -129,40 +154,14 @@ __global__ void k_rdf(RdfArgs a, const double *pre) {
         den_sums(a, d, inv_w, q, den, dden);
         const double inv_den = __drcp_rn(den);
         Gauss G{0.0, 0.0};
-        if (!GRAD) {
-            for (int k = lo; k <= hi; k++) {
-                if (((k - lo) % kGaussAnchor) == 0) gauss_anchor(a, d, k, inv_w, G);
-                const double g = __dmul_rn(G.g, inv_den);
-                if (use_smem)
-                    atomicAdd(s_hist + k, g);
-                else
-                    atomicAdd(hist + k, g);
-                gauss_next(G, q);
-            }
-        } else {
-            const double *dLdh = a.dLdh + (size_t)r * a.n_grid;
-            const double dd2 = __dmul_rn(dden, __dmul_rn(inv_den, inv_den));
-            double dLdd = 0.0;
-            for (int k = lo; k <= hi; k++) {
-                if (((k - lo) % kGaussAnchor) == 0) gauss_anchor(a, d, k, inv_w, G);
-                const double w = dLdh[k];
-                if (w != 0.0) {
-                    const double xk = grid_x(a, k), e = __dsub_rn(xk, d);
-                    const double g = G.g;
-                    const double gp = __dmul_rn(__dmul_rn(__dmul_rn(g, 2.0), e), inv_w);
-                    const double t = __dsub_rn(__dmul_rn(gp, inv_den), __dmul_rn(g, dd2));
-                    dLdd = __dadd_rn(dLdd, __dmul_rn(__ddiv_rn(__dmul_rn(w, pre[r]), __dmul_rn(xk, xk)), t));
-                }
-                gauss_next(G, q);
-            }
-            if (dLdd != 0.0) {
-#pragma unroll
-                for (int u = 0; u < 3; u++) {
-                    const double gu = __ddiv_rn(__dmul_rn(dLdd, dr[u]), d);
-                    atomicAdd(a.dLdx + 3 * (size_t)ib + u, gu);
-                    atomicAdd(a.dLdx + 3 * (size_t)ia + u, -gu);
-                }
-            }
+        for (int k = lo; k <= hi; k++) {
+            if (((k - lo) % kGaussAnchor) == 0) gauss_anchor(a, d, k, a.step, inv_w, G);
+            const double g = __dmul_rn(G.g, inv_den);
+            if (use_smem)
+                atomicAdd(s_hist + k, g);
+            else
+                atomicAdd(hist + k, g);
+            gauss_next(G, q);
         }
     }
     if (use_smem) {
@@ -172,65 +171,303 @@ __global__ void k_rdf(RdfArgs a, const double *pre) {
     }
 }
 
-// h_k = pre * sum_k / x_k^2; loss += weight * sum |h - target|^norm over the slice;
-// dL/dh at the slice points.  One CTA per replica.
-__global__ void k_rdf_finalize(RdfArgs a, const double *pre, const double *target, int s0, int sd,
-                               int nt, int norm, double weight, double *loss, double *dLdh) {
-    const int r = blockIdx.x;
-    double *h = a.hist + (size_t)r * a.n_grid;
-    double *gh = dLdh + (size_t)r * a.n_grid;
-    for (int k = threadIdx.x; k < a.n_grid; k += blockDim.x) {
-        const double xk = grid_x(a, k);
-        h[k] = __ddiv_rn(__dmul_rn(pre[r], h[k]), __dmul_rn(xk, xk));
-        gh[k] = 0.0;
+// The slice points' sums (GRAD false) and the loss gradient from their weights (true).
+//
+// A warp owns one atom i of the first set; the CTA's eight stage the second set in tiles of
+// 256 FP32 positions, and each lane tests one tile atom against the distances the slice can
+// see (an FP32 test with a margin far above its rounding).  The atoms that pass are queued
+// per warp and evaluated 32 at a time in FP64, so the window loops run with full warps
+// whatever the fraction in range (5 % in the 4.5 nm box).  Equal sets take each unordered
+// pair once (half ring: i with the next n/2 atoms, modulo n) and count it twice.  Deposits go
+// to one of a few shared-memory copies of the slice sums (lanes that share a copy are eight
+// apart).  The gradient sums atom i's share in registers.
+//
+// Bound by the shared-memory FP64 atomics (value) and the FP64 pipe (gradient).  Smearing every
+// ordered pair over the whole grid, as k_rdf does, took 567 us a value and 535 us a gradient on
+// the 895-water box and the experimental grid (4,801 points, of which the loss reads 248 and
+// 281), and 215 / 298 us on the 3,000-water box with the 200-bin O-O term; this form takes
+// 63 / 44 us and 67 / 76 us (mean over the O-O and O-H terms).
+constexpr int kRlWarps = 8, kRlTile = 256;
+
+template <bool GRAD>
+__global__ void __launch_bounds__(32 * kRlWarps) k_rdf_loss(RdfArgs a, RdfSlice sl, RdfDen dn, int split,
+                                                            int ncopy) {
+    extern __shared__ double s_sum[];   // GRAD false: [nt][ncopy] partial sums (ncopy 0: none)
+    __shared__ float s_x[3][kRlTile];
+    __shared__ int s_q[kRlWarps][64];
+    const int r = blockIdx.y, nm = a.rep_nmol[r], atom0 = a.rep_atom0[r];
+    const bool same = a.sel1 == a.sel2;
+    const int n1 = a.sel1 == 0 ? nm : 2 * nm, n2 = a.sel2 == 0 ? nm : 2 * nm;
+    const int i0 = (int)(blockIdx.x / split) * kRlWarps, part = (int)(blockIdx.x % split);
+    if (i0 >= n1) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = i0 + warp;
+    // tile positions p of the CTA: atom (i0 + 1 + p) mod n for equal sets, atom p otherwise
+    const int half = n1 / 2;
+    const int np = same ? half + kRlWarps - 1 : n2;
+    const int ntile = (np + kRlTile - 1) / kRlTile;
+    const int t0 = (int)((long long)ntile * part / split), t1 = (int)((long long)ntile * (part + 1) / split);
+    if (t0 >= t1) return;
+    const double L = a.rep_box[r];
+    const float Lf = (float)L, hLf = 0.5f * Lf;
+    const double inv_w = __drcp_rn(a.width);
+    const double S = __dmul_rn(a.step, (double)sl.sd);   // slice spacing
+    const double q1 = exp(-__dmul_rn(__dmul_rn(2.0, __dmul_rn(a.step, a.step)), inv_w));
+    const double qS = exp(-__dmul_rn(__dmul_rn(2.0, __dmul_rn(S, S)), inv_w));
+    const double dmin = __dsub_rn(__dsub_rn(grid_x(a, sl.s0), a.cutoff), a.step);
+    const double dmax = __dadd_rn(__dadd_rn(grid_x(a, sl.s0 + (sl.nt - 1) * sl.sd), a.cutoff), a.step);
+    // FP32 distances err by < 1e-6 L: a margin that no pair in range can miss
+    const float marg = 1e-3f + 1e-5f * Lf;
+    const float far = (float)dmax + marg, near = fmaxf(0.f, (float)dmin - marg);
+    const float far2 = far * far, near2 = near * near;
+    const double pair_w = same ? 2.0 : 1.0;
+    if (!GRAD && ncopy > 0) {
+        for (int k = threadIdx.x; k < sl.nt * ncopy; k += blockDim.x) s_sum[k] = 0.0;
     }
-    __syncthreads();
+    double xi[3] = {0.0, 0.0, 0.0};
+    float xf[3] = {0.f, 0.f, 0.f};
+    const bool live = i < n1;
+    const int ia = rdf_atom(a.sel1, atom0, live ? i : 0);
+    if (live) {
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+            xi[u] = a.x[3 * (size_t)ia + u];
+            xf[u] = (float)xi[u];
+        }
+    }
+    // equal sets: atom i takes the pairs (i, i + k mod n), k = 1 .. n/2, the last of them (n
+    // even) only for i < n/2, so that each unordered pair comes once
+    const int kmax = !live ? -1 : (n1 % 2 == 0 && i >= half ? half - 1 : half);
+    double gi[3] = {0.0, 0.0, 0.0};
+    double *sums = sl.sum + (size_t)r * sl.nt;
+    const double *wt = sl.wt + (size_t)r * sl.nt;
+
+    auto eval = [&](int j) {
+        const int ib = rdf_atom(a.sel2, atom0, j);
+        const double *xb = a.x + 3 * (size_t)ib;
+        double dr[3];
+#pragma unroll
+        for (int u = 0; u < 3; u++) dr[u] = vec1d(xi[u], xb[u], L);
+        const double d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dr[0], dr[0]), __dmul_rn(dr[1], dr[1])),
+                                              __dmul_rn(dr[2], dr[2])));
+        if (d == 0.0 || d < dmin || d > dmax) return;
+        int lo, hi;
+        hist_window(a, d, lo, hi);
+        if (lo > hi) return;
+        // the slice points of the window
+        const int ta = lo <= sl.s0 ? 0 : (lo - sl.s0 + sl.sd - 1) / sl.sd;
+        const int tb = hi < sl.s0 ? -1 : min((hi - sl.s0) / sl.sd, sl.nt - 1);
+        if (ta > tb) return;
+        double den, dden;
+        if (!den_poly(a, dn, d, den, dden)) den_sums(a, d, inv_w, q1, den, dden);
+        const double inv_den = __drcp_rn(den);
+        Gauss G{0.0, 0.0};
+        if (!GRAD) {
+            const double c = __dmul_rn(pair_w, inv_den);
+            for (int t = ta; t <= tb; t++) {
+                if (!sl.recur || ((t - ta) % kGaussAnchor) == 0) gauss_anchor(a, d, sl.s0 + t * sl.sd, S, inv_w, G);
+                const double g = __dmul_rn(G.g, c);
+                if (ncopy > 0)
+                    atomicAdd(s_sum + (size_t)t * ncopy + (lane & (ncopy - 1)), g);
+                else
+                    atomicAdd(sums + t, g);
+                gauss_next(G, qS);
+            }
+        } else {
+            const double dd2 = __dmul_rn(dden, __dmul_rn(inv_den, inv_den));
+            double dLdd = 0.0;
+            for (int t = ta; t <= tb; t++) {
+                if (!sl.recur || ((t - ta) % kGaussAnchor) == 0) gauss_anchor(a, d, sl.s0 + t * sl.sd, S, inv_w, G);
+                const double e = __dsub_rn(grid_x(a, sl.s0 + t * sl.sd), d);
+                const double gp = __dmul_rn(__dmul_rn(__dmul_rn(G.g, 2.0), e), inv_w);
+                dLdd = __fma_rn(wt[t], __dsub_rn(__dmul_rn(gp, inv_den), __dmul_rn(G.g, dd2)), dLdd);
+                gauss_next(G, qS);
+            }
+            if (dLdd != 0.0) {
+                const double s = __ddiv_rn(__dmul_rn(pair_w, dLdd), d);
+#pragma unroll
+                for (int u = 0; u < 3; u++) {
+                    const double gu = __dmul_rn(s, dr[u]);
+                    atomicAdd(a.dLdx + 3 * (size_t)ib + u, gu);
+                    gi[u] = __dsub_rn(gi[u], gu);
+                }
+            }
+        }
+    };
+
+    int nq = 0;
+    for (int t = t0; t < t1; t++) {
+        __syncthreads();
+        {
+            const int p = t * kRlTile + threadIdx.x;
+            if (p < np) {
+                const int j = same ? (i0 + 1 + p) % n1 : p;
+                const double *xj = a.x + 3 * (size_t)rdf_atom(a.sel2, atom0, j);
+#pragma unroll
+                for (int u = 0; u < 3; u++) s_x[u][threadIdx.x] = (float)xj[u];
+            }
+        }
+        __syncthreads();
+        for (int b = 0; b < kRlTile; b += 32) {
+            const int p = t * kRlTile + b + lane;
+            // equal sets: k = j - i before the ring's wrap
+            const int k = i0 + 1 + p - i;
+            bool ok = p < np && (same ? k >= 1 && k <= kmax : live);
+            if (ok) {
+                float r2 = 0.f;
+#pragma unroll
+                for (int u = 0; u < 3; u++) {
+                    float d = s_x[u][b + lane] - xf[u];
+                    d = d > hLf ? d - Lf : (d < -hLf ? d + Lf : d);
+                    r2 = fmaf(d, d, r2);
+                }
+                ok = r2 <= far2 && r2 >= near2;
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, ok);
+            if (ok) {
+                const int j = !same ? p : (i + k < n1 ? i + k : i + k - n1);
+                s_q[warp][nq + __popc(m & ((1u << lane) - 1u))] = j;
+            }
+            nq += __popc(m);
+            __syncwarp();
+            if (nq >= 32) {
+                nq -= 32;
+                eval(s_q[warp][nq + lane]);
+                __syncwarp();
+            }
+        }
+    }
+    if (lane < nq) eval(s_q[warp][lane]);
+    if (GRAD) {
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 3; u++) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) gi[u] += __shfl_xor_sync(0xffffffffu, gi[u], o);
+            if (lane == 0 && live && gi[u] != 0.0) atomicAdd(a.dLdx + 3 * (size_t)ia + u, gi[u]);
+        }
+    } else if (ncopy > 0) {
+        __syncthreads();
+        for (int t = threadIdx.x; t < sl.nt; t += blockDim.x) {
+            double v = 0.0;
+            for (int c = 0; c < ncopy; c++) v += s_sum[(size_t)t * ncopy + c];
+            if (v != 0.0) atomicAdd(sums + t, v);
+        }
+    }
+}
+
+// h = pre sum / x^2 at the slice points, loss += weight sum |h - target|^norm, and the
+// gradient's weights dL/dh pre / x^2.  One CTA per replica.
+__global__ void __launch_bounds__(256) k_rdf_loss_finalize(RdfArgs a, RdfSlice sl, const double *pre,
+                                                           const double *target, int norm, double weight,
+                                                           double *loss) {
     __shared__ double s_l[256];
+    const int r = blockIdx.x;
+    const double *sum = sl.sum + (size_t)r * sl.nt;
+    double *wt = sl.wt + (size_t)r * sl.nt;
     double l = 0.0;
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-        const int k = s0 + t * sd;
-        const double e = __dsub_rn(h[k], target[(size_t)r * nt + t]);
+    for (int t = threadIdx.x; t < sl.nt; t += blockDim.x) {
+        const double xk = grid_x(a, sl.s0 + t * sl.sd), x2 = __dmul_rn(xk, xk);
+        const double e = __dsub_rn(__ddiv_rn(__dmul_rn(pre[r], sum[t]), x2), target[(size_t)r * sl.nt + t]);
+        double g;
         if (norm == 1) {
             l = __dadd_rn(l, fabs(e));
-            gh[k] = weight * (e > 0.0 ? 1.0 : (e < 0.0 ? -1.0 : 0.0));
+            g = weight * (e > 0.0 ? 1.0 : (e < 0.0 ? -1.0 : 0.0));
         } else {
             l = __dadd_rn(l, __dmul_rn(e, e));
-            gh[k] = __dmul_rn(weight, __dmul_rn(2.0, e));
+            g = __dmul_rn(weight, __dmul_rn(2.0, e));
         }
+        wt[t] = __ddiv_rn(__dmul_rn(g, pre[r]), x2);
     }
     s_l[threadIdx.x] = l;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int t = 0; t < blockDim.x; t++) s = __dadd_rn(s, s_l[t]);
-        loss[r] = __dadd_rn(loss[r], __dmul_rn(weight, s));
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) s_l[threadIdx.x] = __dadd_rn(s_l[threadIdx.x], s_l[threadIdx.x + o]);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) loss[r] = __dadd_rn(loss[r], __dmul_rn(weight, s_l[0]));
+}
+
+// h_k = pre * sum_k / x_k^2.  One CTA per replica.
+__global__ void k_rdf_scale(RdfArgs a, const double *pre) {
+    const int r = blockIdx.x;
+    double *h = a.hist + (size_t)r * a.n_grid;
+    for (int k = threadIdx.x; k < a.n_grid; k += blockDim.x) {
+        const double xk = grid_x(a, k);
+        h[k] = __ddiv_rn(__dmul_rn(pre[r], h[k]), __dmul_rn(xk, xk));
     }
 }
 
 }  // namespace
 
-// pre [R] is stashed by the caller at a.hist + R*n_grid (scratch behind the histogram).
-cudaError_t launch_rdf(const RdfArgs &a, int R, int max_n1, int max_n2, bool grad,
-                       cudaStream_t st) {
+cudaError_t launch_rdf(const RdfArgs &a, int R, int max_n1, int max_n2, const double *pre, cudaStream_t st) {
     const long long pairs = (long long)max_n1 * max_n2;
     long long blocks = (pairs + 255) / 256;
     if (blocks > 4096) blocks = 4096;
     if (blocks < 1) blocks = 1;
-    const double *pre = a.hist + (size_t)R * a.n_grid;
-    if (grad) {
-        k_rdf<true><<<dim3((unsigned)blocks, R), 256, 0, st>>>(a, pre);
-    } else {
-        const size_t smem = a.n_grid <= 6144 ? sizeof(double) * a.n_grid : 0;
-        k_rdf<false><<<dim3((unsigned)blocks, R), 256, smem, st>>>(a, pre);
-    }
+    const size_t smem = a.n_grid <= 6144 ? sizeof(double) * a.n_grid : 0;
+    k_rdf<<<dim3((unsigned)blocks, R), 256, smem, st>>>(a);
+    k_rdf_scale<<<R, 256, 0, st>>>(a, pre);
     return cudaGetLastError();
 }
 
-cudaError_t launch_rdf_finalize(const RdfArgs &a, int R, const double *pre, const double *target,
-                                int slice_start, int slice_stride, int n_target, int norm,
-                                double weight, double *loss, double *dLdh, cudaStream_t st) {
-    k_rdf_finalize<<<R, 256, 0, st>>>(a, pre, target, slice_start, slice_stride, n_target, norm,
-                                      weight, loss, dLdh);
+// den(d) of an unclipped pair depends only on where d lies in its grid cell: with j the cell,
+// u = d - (j + 1/2) step, the window is [j - n + a, j + n + b], a, b in {0, 1}, and
+// exp(-(e - u)^2 / w) = sum_m A_m(e) u^m with A_0 = exp(-e^2 / w), A_1 = (2 e / w) A_0,
+// A_{m+1} = ((2 e / w) A_m - (2 / w) A_{m-1}) / (m + 1) (Hermite's recurrence).  The series is
+// cut where its terms at |u| = step / 2 fall below 1e-18 of the sum; a grid too coarse for
+// that within kMaxTerms keeps the direct sum (M = 0).
+RdfDen rdf_den_poly(double step, double width, double cutoff) {
+    constexpr int T = RdfDen::kMaxTerms;
+    RdfDen dn;
+    dn.M = 0;
+    const double cells = std::floor(cutoff / step);
+    if (!(cells < 4096.0)) return dn;
+    dn.n = (int)cells;
+    double inner[T + 2] = {}, edge[2][T + 2] = {}, mag[T + 2] = {};   // edge: k = -n and n + 1
+    for (int k = -dn.n; k <= dn.n + 1; k++) {
+        const double e = (k - 0.5) * step, w2 = 2.0 / width;
+        double *c = k == -dn.n ? edge[0] : (k == dn.n + 1 ? edge[1] : inner);
+        double p0 = 0.0, p1 = std::exp(-e * e / width), h = 1.0;
+        for (int m = 0; m < T + 2; m++) {
+            c[m] += p1;
+            mag[m] += std::fabs(p1) * h;
+            const double p2 = (w2 * e * p1 - w2 * p0) / (m + 1);
+            p0 = p1;
+            p1 = p2;
+            h *= 0.5 * step;
+        }
+    }
+    for (int m = 1; m <= T; m++)
+        if (mag[m] < 1e-18 * mag[0] && mag[m + 1] < 1e-18 * mag[0]) {
+            dn.M = m;
+            break;
+        }
+    for (int ca = 0; ca < 2; ca++)
+        for (int cb = 0; cb < 2; cb++)
+            for (int m = 0; m < T; m++)
+                dn.c[2 * ca + cb][m] = inner[m] + (ca ? 0.0 : edge[0][m]) + (cb ? edge[1][m] : 0.0);
+    return dn;
+}
+
+// split: CTAs per eight first atoms, so that small boxes still fill the SMs; ncopy: as many
+// shared-memory copies of the slice sums (a power of two, at most 8) as 32 KB hold.
+cudaError_t launch_rdf_loss(const RdfArgs &a, const RdfSlice &sl, const RdfDen &dn, int R, int max_n1, int max_n2,
+                            const double *pre, const double *target, int norm, double weight, bool grad,
+                            double *loss, cudaStream_t st) {
+    if (sl.nt < 1) return cudaSuccess;
+    const int groups = (max_n1 + kRlWarps - 1) / kRlWarps;
+    const int tiles = ((a.sel1 == a.sel2 ? max_n1 / 2 + kRlWarps : max_n2) + kRlTile - 1) / kRlTile;
+    int split = 1;
+    while (split < tiles && (long long)groups * R * split < 2 * 148) split++;
+    int ncopy = 8;
+    while (ncopy > 0 && sizeof(double) * ncopy * (size_t)sl.nt > 32768) ncopy >>= 1;
+    const dim3 grid(groups * split, R);
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(sl.sum, 0, sizeof(double) * (size_t)R * sl.nt, st))) return e;
+    k_rdf_loss<false><<<grid, 32 * kRlWarps, sizeof(double) * ncopy * sl.nt, st>>>(a, sl, dn, split, ncopy);
+    k_rdf_loss_finalize<<<R, 256, 0, st>>>(a, sl, pre, target, norm, weight, loss);
+    if (grad) k_rdf_loss<true><<<grid, 32 * kRlWarps, 0, st>>>(a, sl, dn, split, 0);
     return cudaGetLastError();
 }
 
@@ -242,7 +479,7 @@ cudaError_t launch_rdf_finalize(const RdfArgs &a, int R, const double *pre, cons
 // hands out device pointers), a loop that must not hit the device-wide
 // synchronisation cudaMalloc/cudaFree imply, or a service whose memory is budgeted
 // in full before it starts.  For them this entry point takes the caller's device
-// buffers and keeps its scratch (the histogram, dL/dh, the normalisation constant
+// buffers and keeps its scratch (the slice sums, the gradient weights, the normalisation constant
 // and a one-box table, at most kNoallocMaxGrid grid points) in the file-scope
 // array g_rdf_scratch, which every GPU that loads the library holds until the
 // process exits.  Host code cannot use the array's name as a device address: the
@@ -257,8 +494,8 @@ cudaError_t launch_rdf_finalize(const RdfArgs &a, int R, const double *pre, cons
 namespace {
 
 constexpr int kNoallocMaxGrid = 8192;
-// layout (doubles): hist [kNoallocMaxGrid + 1] (the normaliser V / (4 pi n1 n2 step)
-// sits right after the n_grid used entries) | dL/dh [kNoallocMaxGrid] | box [1] |
+// layout (doubles): slice sums [kNoallocMaxGrid + 1] (the normaliser V / (4 pi n1 n2 step)
+// sits after n_grid entries) | gradient weights [kNoallocMaxGrid] | box [1] |
 // {atom0, n_mol} as two ints [1]
 constexpr int kNoallocDLdh = kNoallocMaxGrid + 1;
 constexpr int kNoallocBox = 2 * kNoallocMaxGrid + 1;
@@ -312,8 +549,7 @@ extern "C" int32_t revsim_rdf_loss_grad_noalloc(const double *d_x, int32_t n_mol
     const double pre = box * box * box / (4 * 3.14159265358979323846 * n1 * n2 * t->step);
     k_noalloc_tables<<<1, 1, 0, st>>>(s, t->n_grid, pre, box, n_mol);
     if (cudaGetLastError() != cudaSuccess) return REVSIM_ERR_CUDA;
-    if (cudaMemsetAsync(s, 0, sizeof(double) * t->n_grid, st) != cudaSuccess ||
-        cudaMemsetAsync(d_loss, 0, sizeof(double), st) != cudaSuccess ||
+    if (cudaMemsetAsync(d_loss, 0, sizeof(double), st) != cudaSuccess ||
         cudaMemsetAsync(d_dLdx, 0, sizeof(double) * 9 * (size_t)n_mol, st) != cudaSuccess)
         return REVSIM_ERR_CUDA;
     RdfArgs a;
@@ -329,13 +565,13 @@ extern "C" int32_t revsim_rdf_loss_grad_noalloc(const double *d_x, int32_t n_mol
     a.cutoff = t->exp_cutoff;
     a.n_grid = t->n_grid;
     a.off = (int)std::llround(q) - 1;
-    a.hist = s;
-    a.dLdh = s + kNoallocDLdh;
+    a.hist = nullptr;
     a.dLdx = d_dLdx;
-    if (launch_rdf(a, 1, (int)n1, (int)n2, false, st) != cudaSuccess ||
-        launch_rdf_finalize(a, 1, s + t->n_grid, d_target, t->slice_start, t->slice_stride, t->n_target,
-                            t->norm, t->weight, d_loss, s + kNoallocDLdh, st) != cudaSuccess ||
-        launch_rdf(a, 1, (int)n1, (int)n2, true, st) != cudaSuccess)
+    RdfSlice sl = rdf_slice(t->slice_start, t->slice_stride, t->n_target, t->step, t->width, t->exp_cutoff);
+    sl.sum = s;
+    sl.wt = s + kNoallocDLdh;
+    if (launch_rdf_loss(a, sl, rdf_den_poly(t->step, t->width, t->exp_cutoff), 1, (int)n1, (int)n2, s + t->n_grid,
+                        d_target, t->norm, t->weight, true, d_loss, st) != cudaSuccess)
         return REVSIM_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? REVSIM_OK : REVSIM_ERR_CUDA;
 }
