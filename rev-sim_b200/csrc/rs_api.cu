@@ -1383,23 +1383,25 @@ int set_mlp(revsim_handle *h, const double *theta_mlp) {
 
 // The accumulated interval-coefficient adjoints of every replica -> dtheta_mlp [R][MLP_NPARAMS].
 int mlp_grads(revsim_handle *h, std::vector<double> &out) {
-    for (int r = 0; r < h->R; r++) {
-        const double *cadj = h->d_mlp_adj + (size_t)r * MLP_NCOPY * MLP_NT * MLP_NG * 4;
-        double *grad = h->d_mlp_grad + (size_t)r * MLP_NPARAMS;
-        cudaError_t e;
-        if (h->mlp_mode == 1) {
+    cudaError_t e = cudaSuccess;
+    if (h->mlp_mode == 1) {
+        for (int r = 0; r < h->R && e == cudaSuccess; r++) {
+            const double *cadj = h->d_mlp_adj + (size_t)r * MLP_NCOPY * MLP_NT * MLP_NG * 4;
+            double *grad = h->d_mlp_grad + (size_t)r * MLP_NPARAMS;
             e = launch_mlp_node_adjoints(cadj, MLP_NCOPY, h->rc, h->d_mlp_scratch, h->st);
             if (e == cudaSuccess)
                 e = launch_mlp_tc_backprop(h->d_mlp_theta, MLP_NT, h->rc, MLP_WIDTH,
                                            mlp_scratch_nodes(h->d_mlp_scratch, 2),
                                            mlp_scratch_nodes(h->d_mlp_scratch, 3), h->d_mlp_tc, grad, h->st);
             h->launches += 4;
-        } else {
-            e = launch_mlp_backprop(h->d_mlp_theta, h->rc, cadj, MLP_NCOPY, h->d_mlp_scratch, grad, h->st);
-            h->launches += 3;
         }
-        if (e != cudaSuccess) return fail(h, REVSIM_ERR_CUDA, std::string("MLP backprop: ") + cudaGetErrorString(e));
+    } else {
+        int nk = 0;
+        e = launch_mlp_backprop(h->d_mlp_theta, h->rc, h->d_mlp_adj, h->R, MLP_NCOPY, h->d_mlp_scratch, h->d_mlp_grad,
+                                h->st, &nk);
+        h->launches += nk;
     }
+    if (e != cudaSuccess) return fail(h, REVSIM_ERR_CUDA, std::string("MLP backprop: ") + cudaGetErrorString(e));
     out.resize((size_t)h->R * MLP_NPARAMS);
     CK(cudaMemcpyAsync(out.data(), h->d_mlp_grad, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));

@@ -302,11 +302,12 @@ size_t mlp_scratch_doubles();
 // default; the Stillinger-Weber radial term uses one type.
 cudaError_t launch_mlp_table(int prec, const double *theta, double rc, double *scratch, void *tab,
                              cudaStream_t st, int nt = MLP_NT, double w = MLP_WIDTH);
-// Interval-coefficient adjoints (the sum of ncopy accumulators) -> dtheta [MLP_NPARAMS]
-// (after launch_mlp_table with the same theta and scratch).
-cudaError_t launch_mlp_backprop(const double *theta, double rc, const double *cadj, int ncopy,
-                                double *scratch, double *dtheta, cudaStream_t st, int nt = MLP_NT,
-                                double w = MLP_WIDTH);
+// Interval-coefficient adjoints [R][ncopy][nt][MLP_NG][4] (the sum of each replica's ncopy
+// accumulators) -> dtheta [R][nt * MLP_PER_TYPE] (after launch_mlp_table with the same theta and
+// scratch).
+cudaError_t launch_mlp_backprop(const double *theta, double rc, const double *cadj, int R, int ncopy,
+                                double *scratch, double *dtheta, cudaStream_t st, int *n_kernels,
+                                int nt = MLP_NT, double w = MLP_WIDTH);
 
 // Node values -> interval table, the scratch's node arrays (0 u, 1 du, 2 au, 3 ad), and the
 // coefficient adjoints -> node adjoints alone (rs_mlp.cu).

@@ -10,6 +10,8 @@
 // interval coefficients; k_mlp_* below carry them back to the weights once per pass.
 // The same code serves the Stillinger-Weber path's learned radial term (one type, its own
 // cutoff and width): the type count nt and width w are arguments.
+#include <algorithm>
+
 #include "rs_internal.h"
 
 namespace rs {
@@ -51,51 +53,92 @@ __device__ __forceinline__ void rbf(double r, double rc, double w, int k, double
     dphi = -e / (w * w) * phi;
 }
 
-// Sum over the 64 threads of a block in a fixed tree.
-__device__ __forceinline__ double block_sum64(double v, double *s) {
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 32; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-        __syncthreads();
-    }
-    const double r = s[0];
-    __syncthreads();
-    return r;
+// The node batch: kNodes nodes per CTA, thread (i, q) = hidden unit i of nodes q and q + 4, so
+// that W2 is read once per eight nodes, from shared memory (rows padded to 65: lanes of one
+// warp read one column of 32 rows without bank conflicts).  FP64-pipe work of ~3 us for the
+// three types; one 64-thread CTA per node, which read W2 from L2 with a 512-byte lane stride,
+// took 66 us for the water model's 3 x 1,025 nodes.
+constexpr int kNodes = 8, kMlpThreads = 256, kQ = kMlpThreads / H, kPer = kNodes / kQ;
+constexpr int kW2Ld = H + 1;
+
+__device__ __forceinline__ void load_w2(const View &m, double *s_w2) {
+    for (int k = threadIdx.x; k < H * H; k += kMlpThreads) s_w2[(k / H) * kW2Ld + k % H] = m.W2[k];
 }
 
-// One block (64 threads = hidden units) per (node g, type t): value and r-tangent streams.
-__global__ void __launch_bounds__(64) k_mlp_nodes(const double *theta, double rc, double w, double *act,
-                                                  double *u, double *du) {
-    __shared__ double s_phi[NR], s_dphi[NR], s_h1[H], s_dh1[H], s_red[H];
-    const int g = blockIdx.x, t = blockIdx.y, i = threadIdx.x;
+__global__ void __launch_bounds__(kMlpThreads) k_mlp_nodes(const double *theta, double rc, double w, double *act,
+                                                           double *u, double *du) {
+    extern __shared__ double s_w2[];   // [H][kW2Ld]
+    __shared__ double s_phi[kNodes][NR], s_dphi[kNodes][NR], s_h[kNodes][H], s_dh[kNodes][H];
+    __shared__ double s_red[kNodes][2][2];
+    const int t = blockIdx.y, g0 = blockIdx.x * kNodes, i = threadIdx.x % H, q = threadIdx.x / H;
     const View m = view(theta, t);
-    const double r = g * (rc / NG);
-    if (i < NR) rbf(r, rc, w, i, s_phi[i], s_dphi[i]);
+    load_w2(m, s_w2);
+    if (threadIdx.x < kNodes * NR) {
+        const int n = threadIdx.x / NR, k = threadIdx.x % NR;
+        rbf((g0 + n) * (rc / NG), rc, w, k, s_phi[n][k], s_dphi[n][k]);
+    }
     __syncthreads();
-    double z1 = m.b1[i], dz1 = 0.0;
+    double z1[kPer], dz1[kPer], z2[kPer], dz2[kPer];
+#pragma unroll
+    for (int p = 0; p < kPer; p++) {
+        z1[p] = m.b1[i];
+        dz1[p] = 0.0;
+    }
     for (int k = 0; k < NR; k++) {
-        z1 += m.W1[i * NR + k] * s_phi[k];
-        dz1 += m.W1[i * NR + k] * s_dphi[k];
+        const double wk = m.W1[i * NR + k];
+#pragma unroll
+        for (int p = 0; p < kPer; p++) {
+            z1[p] += wk * s_phi[q + kQ * p][k];
+            dz1[p] += wk * s_dphi[q + kQ * p][k];
+        }
     }
-    s_h1[i] = silu0(z1);
-    s_dh1[i] = silu1(z1) * dz1;
+#pragma unroll
+    for (int p = 0; p < kPer; p++) {
+        s_h[q + kQ * p][i] = silu0(z1[p]);
+        s_dh[q + kQ * p][i] = silu1(z1[p]) * dz1[p];
+        z2[p] = m.b2[i];
+        dz2[p] = 0.0;
+    }
     __syncthreads();
-    double z2 = m.b2[i], dz2 = 0.0;
+#pragma unroll 8
     for (int j = 0; j < H; j++) {
-        z2 += m.W2[i * H + j] * s_h1[j];
-        dz2 += m.W2[i * H + j] * s_dh1[j];
+        const double wj = s_w2[i * kW2Ld + j];
+#pragma unroll
+        for (int p = 0; p < kPer; p++) {
+            z2[p] += wj * s_h[q + kQ * p][j];
+            dz2[p] += wj * s_dh[q + kQ * p][j];
+        }
     }
-    const double y = m.b3[0] + block_sum64(m.w3[i] * silu0(z2), s_red);
-    const double dy = block_sum64(m.w3[i] * silu1(z2) * dz2, s_red);
-    double *a = act + ((size_t)t * (NG + 1) + g) * NA;
-    a[i] = z1;
-    a[H + i] = dz1;
-    a[2 * H + i] = z2;
-    a[3 * H + i] = dz2;
-    if (i == 0) {
-        const double x = 3.14159265358979323846 * r / rc;
+    const double w3 = m.w3[i];
+#pragma unroll
+    for (int p = 0; p < kPer; p++) {
+        // y and y' over the 64 units: the unit's two warps, then their sum
+        double y = w3 * silu0(z2[p]), dy = w3 * silu1(z2[p]) * dz2[p];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            y += __shfl_xor_sync(0xffffffffu, y, o);
+            dy += __shfl_xor_sync(0xffffffffu, dy, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            s_red[q + kQ * p][i / 32][0] = y;
+            s_red[q + kQ * p][i / 32][1] = dy;
+        }
+        const int g = g0 + q + kQ * p;
+        if (g <= NG) {
+            double *a = act + ((size_t)t * (NG + 1) + g) * NA;
+            a[i] = z1[p];
+            a[H + i] = dz1[p];
+            a[2 * H + i] = z2[p];
+            a[3 * H + i] = dz2[p];
+        }
+    }
+    __syncthreads();
+    const int n = threadIdx.x, g = g0 + n;
+    if (n < kNodes && g <= NG) {
+        const double y = m.b3[0] + (s_red[n][0][0] + s_red[n][1][0]), dy = s_red[n][0][1] + s_red[n][1][1];
+        const double r = g * (rc / NG), x = 3.14159265358979323846 * r / rc;
         const double fc = 0.5 * (cos(x) + 1.0), dfc = -0.5 * 3.14159265358979323846 / rc * sin(x);
+        double *a = act + ((size_t)t * (NG + 1) + g) * NA;
         a[4 * H] = y;
         a[4 * H + 1] = dy;
         a[4 * H + 2] = fc;
@@ -138,6 +181,9 @@ __device__ __forceinline__ void sum_copies(const double *cadj, int ncopy, int nt
 __global__ void k_mlp_adj_nodes(const double *cadj, int ncopy, int nt, double rc, double *au, double *ad) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nt * (NG + 1)) return;
+    cadj += (size_t)blockIdx.y * ncopy * nt * NG * 4;   // one replica per grid row
+    au += (size_t)blockIdx.y * nt * (NG + 1);
+    ad += (size_t)blockIdx.y * nt * (NG + 1);
     const int t = k / (NG + 1), g = k % (NG + 1);
     const double h = rc / NG;
     double a = 0.0, d = 0.0, c[4];
@@ -155,97 +201,165 @@ __global__ void k_mlp_adj_nodes(const double *cadj, int ncopy, int nt, double rc
     ad[k] = d;
 }
 
-// Per node: adjoints of z2, dz2, z1, dz1 and of y, dy (reverse mode through both streams).
-__global__ void __launch_bounds__(64) k_mlp_node_bwd(const double *theta, const double *act,
-                                                     const double *au, const double *ad,
-                                                     double *bwd) {
-    __shared__ double s_z2b[H], s_dz2b[H];
-    const int g = blockIdx.x, t = blockIdx.y, i = threadIdx.x;
+// Backward pass and weight gradients: CTA (chunk c, type t, replica r) takes the nodes of its
+// chunk eight at a time -- the node adjoints of z2, z2', z1, z1' (reverse mode through both
+// streams; W2 from shared memory), then the outer products, W2's as a 4 x 4 tile and W1's as
+// four entries per thread, kept in registers over the chunk -- and writes its partial
+// gradient; k_mlp_wgrad_sum adds the chunks in order.  All replicas run in one launch.
+// FP64-pipe bound.  One thread per parameter and replica, summing over the nodes with the
+// activations formed again for each of the 4,096 W2 entries, took 712 us for the water
+// model's three types and 484 us per replica for the diamond's one.
+__global__ void __launch_bounds__(kMlpThreads) k_mlp_wgrad(const double *theta, double rc, double w, int nt,
+                                                           const double *act, const double *au,
+                                                           const double *ad, double *part) {
+    extern __shared__ double s_dyn[];   // W2 [H][kW2Ld], then seven [kNodes][H] arrays
+    double *s_w2 = s_dyn;
+    using Row = double[H];
+    Row *s_h = (Row *)(s_dyn + H * kW2Ld), *s_dh = s_h + kNodes, *s_z2 = s_dh + kNodes, *s_dz2 = s_z2 + kNodes,
+        *s_z1 = s_dz2 + kNodes, *s_dz1 = s_z1 + kNodes;
+    __shared__ double s_phi[kNodes][NR], s_dphi[kNodes][NR], s_y[kNodes][2];
+    const int C = gridDim.x, c = blockIdx.x, t = blockIdx.y, r = blockIdx.z;
+    const int g_lo = (int)((long long)(NG + 1) * c / C), g_hi = (int)((long long)(NG + 1) * (c + 1) / C);
+    const int i = threadIdx.x % H, q = threadIdx.x / H;
     const View m = view(theta, t);
-    const double *a = act + ((size_t)t * (NG + 1) + g) * NA;
-    double *b = bwd + ((size_t)t * (NG + 1) + g) * NA;
-    const int n = t * (NG + 1) + g;
-    const double fc = a[4 * H + 2], dfc = a[4 * H + 3];
-    // u = y fc, u' = y' fc + y fc'
-    const double yb = au[n] * fc + ad[n] * dfc, dyb = ad[n] * fc;
-    const double z2 = a[2 * H + i], dz2 = a[3 * H + i];
-    const double h2b = yb * m.w3[i], dh2b = dyb * m.w3[i];
-    s_z2b[i] = h2b * silu1(z2) + dh2b * silu2(z2) * dz2;
-    s_dz2b[i] = dh2b * silu1(z2);
-    __syncthreads();
-    double h1b = 0.0, dh1b = 0.0;
-    for (int q = 0; q < H; q++) {
-        h1b += m.W2[q * H + i] * s_z2b[q];
-        dh1b += m.W2[q * H + i] * s_dz2b[q];
+    load_w2(m, s_w2);
+    const double w3 = m.w3[i];
+    const double *aur = au + ((size_t)r * nt + t) * (NG + 1), *adr = ad + ((size_t)r * nt + t) * (NG + 1);
+    const int ti = 4 * (threadIdx.x / 16), tj = 4 * (threadIdx.x % 16);   // W2 tile
+    const int vi = threadIdx.x / 4, vk = 4 * (threadIdx.x % 4);           // W1 entries
+    double aw2[4][4] = {}, aw1[4] = {}, ab1 = 0.0, ab2 = 0.0, aw3 = 0.0, ab3 = 0.0;
+    for (int g0 = g_lo; g0 < g_hi; g0 += kNodes) {
+        __syncthreads();
+        if (threadIdx.x < kNodes * NR) {
+            const int n = threadIdx.x / NR, k = threadIdx.x % NR;
+            rbf((g0 + n) * (rc / NG), rc, w, k, s_phi[n][k], s_dphi[n][k]);
+        }
+        double s1[kPer], s2[kPer];   // silu'(z1), silu''(z1) z1'
+#pragma unroll
+        for (int p = 0; p < kPer; p++) {
+            const int n = q + kQ * p, g = g0 + n;
+            // nodes past the chunk: zero adjoints, finite activations
+            const bool in = g < g_hi;
+            const double *a = act + ((size_t)t * (NG + 1) + (in ? g : g_lo)) * NA;
+            const double fc = a[4 * H + 2], dfc = a[4 * H + 3];
+            const double un = in ? aur[g] : 0.0, dn = in ? adr[g] : 0.0;
+            // u = y fc, u' = y' fc + y fc'
+            const double yb = un * fc + dn * dfc, dyb = dn * fc;
+            const double z1 = a[i], dz1 = a[H + i], z2 = a[2 * H + i], dz2 = a[3 * H + i];
+            const double f2 = silu1(z2);
+            s1[p] = silu1(z1);
+            s2[p] = silu2(z1) * dz1;
+            s_h[n][i] = silu0(z1);
+            s_dh[n][i] = s1[p] * dz1;
+            const double h2b = yb * w3, dh2b = dyb * w3;
+            const double z2b = h2b * f2 + dh2b * silu2(z2) * dz2;
+            s_z2[n][i] = z2b;
+            s_dz2[n][i] = dh2b * f2;
+            ab2 += z2b;
+            aw3 += yb * silu0(z2) + dyb * f2 * dz2;
+            if (i == 0) ab3 += yb;
+        }
+        __syncthreads();
+        double h1b[kPer], dh1b[kPer];
+#pragma unroll
+        for (int p = 0; p < kPer; p++) h1b[p] = dh1b[p] = 0.0;
+#pragma unroll 8
+        for (int k = 0; k < H; k++) {
+            const double wk = s_w2[k * kW2Ld + i];
+#pragma unroll
+            for (int p = 0; p < kPer; p++) {
+                h1b[p] += wk * s_z2[q + kQ * p][k];
+                dh1b[p] += wk * s_dz2[q + kQ * p][k];
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < kPer; p++) {
+            const double z1b = h1b[p] * s1[p] + dh1b[p] * s2[p];
+            s_z1[q + kQ * p][i] = z1b;
+            s_dz1[q + kQ * p][i] = dh1b[p] * s1[p];
+            ab1 += z1b;
+        }
+        __syncthreads();
+        for (int n = 0; n < kNodes; n++) {
+            double zb[4], db[4], hv[4], dv[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                zb[k] = s_z2[n][ti + k];
+                db[k] = s_dz2[n][ti + k];
+                hv[k] = s_h[n][tj + k];
+                dv[k] = s_dh[n][tj + k];
+            }
+#pragma unroll
+            for (int x = 0; x < 4; x++)
+#pragma unroll
+                for (int y = 0; y < 4; y++) aw2[x][y] += zb[x] * hv[y] + db[x] * dv[y];
+            const double z1b = s_z1[n][vi], dz1b = s_dz1[n][vi];
+#pragma unroll
+            for (int k = 0; k < 4; k++) aw1[k] += z1b * s_phi[n][vk + k] + dz1b * s_dphi[n][vk + k];
+        }
     }
-    const double z1 = a[i], dz1 = a[H + i];
-    b[i] = h1b * silu1(z1) + dh1b * silu2(z1) * dz1;   // z1 adjoint
-    b[H + i] = dh1b * silu1(z1);                        // dz1 adjoint
-    b[2 * H + i] = s_z2b[i];
-    b[3 * H + i] = s_dz2b[i];
-    if (i == 0) {
-        b[4 * H] = yb;
-        b[4 * H + 1] = dyb;
+    double *out = part + (((size_t)r * nt + t) * C + c) * MLP_PER_TYPE;
+#pragma unroll
+    for (int k = 0; k < 4; k++) out[vi * NR + vk + k] = aw1[k];
+    double *o2 = out + H * NR + H;
+#pragma unroll
+    for (int x = 0; x < 4; x++)
+#pragma unroll
+        for (int y = 0; y < 4; y++) o2[(ti + x) * H + tj + y] = aw2[x][y];
+    // the four threads of a unit, in order
+    __syncthreads();
+    s_h[q][i] = ab1;
+    s_dh[q][i] = ab2;
+    s_z2[q][i] = aw3;
+    if (i == 0) s_y[q][0] = ab3;
+    __syncthreads();
+    if (threadIdx.x < H) {
+        double b1 = 0.0, b2 = 0.0, v3 = 0.0;
+        for (int k = 0; k < kQ; k++) {
+            b1 += s_h[k][i];
+            b2 += s_dh[k][i];
+            v3 += s_z2[k][i];
+        }
+        out[H * NR + i] = b1;
+        o2[H * H + i] = b2;
+        o2[H * H + H + i] = v3;
+        if (i == 0) o2[H * H + 2 * H] = s_y[0][0] + s_y[1][0] + s_y[2][0] + s_y[3][0];
     }
 }
 
-// One thread per parameter: sum over the nodes in order (deterministic).
-__global__ void k_mlp_wgrad(double rc, double w, int nt, const double *act, const double *bwd,
-                            double *dtheta) {
+// dtheta of (replica, type) = blockIdx.y: the chunks' partials in order.
+__global__ void k_mlp_wgrad_sum(int C, const double *part, double *dtheta) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nt * MLP_PER_TYPE) return;
-    const int t = k / MLP_PER_TYPE, q = k % MLP_PER_TYPE;
-    const double *A = act + (size_t)t * (NG + 1) * NA;
-    const double *B = bwd + (size_t)t * (NG + 1) * NA;
+    if (k >= MLP_PER_TYPE) return;
+    const double *p = part + (size_t)blockIdx.y * C * MLP_PER_TYPE + k;
     double s = 0.0;
-    if (q < H * NR) {                              // W1[i][kk]
-        const int i = q / NR, kk = q % NR;
-        for (int g = 0; g <= NG; g++) {
-            double phi, dphi;
-            rbf(g * (rc / NG), rc, w, kk, phi, dphi);
-            s += B[g * NA + i] * phi + B[g * NA + H + i] * dphi;
-        }
-    } else if (q < H * NR + H) {                   // b1[i]
-        const int i = q - H * NR;
-        for (int g = 0; g <= NG; g++) s += B[g * NA + i];
-    } else if (q < H * NR + H + H * H) {           // W2[i][j]
-        const int i = (q - H * NR - H) / H, j = (q - H * NR - H) % H;
-        for (int g = 0; g <= NG; g++) {
-            const double z1 = A[g * NA + j], dz1 = A[g * NA + H + j];
-            s += B[g * NA + 2 * H + i] * silu0(z1) + B[g * NA + 3 * H + i] * silu1(z1) * dz1;
-        }
-    } else if (q < H * NR + H + H * H + H) {       // b2[i]
-        const int i = q - H * NR - H - H * H;
-        for (int g = 0; g <= NG; g++) s += B[g * NA + 2 * H + i];
-    } else if (q < MLP_PER_TYPE - 1) {             // w3[i]
-        const int i = q - H * NR - H - H * H - H;
-        for (int g = 0; g <= NG; g++) {
-            const double z2 = A[g * NA + 2 * H + i], dz2 = A[g * NA + 3 * H + i];
-            s += B[g * NA + 4 * H] * silu0(z2) + B[g * NA + 4 * H + 1] * silu1(z2) * dz2;
-        }
-    } else {                                       // b3
-        for (int g = 0; g <= NG; g++) s += B[g * NA + 4 * H];
-    }
-    dtheta[k] = s;
+    for (int c = 0; c < C; c++) s += p[(size_t)c * MLP_PER_TYPE];
+    dtheta[(size_t)blockIdx.y * MLP_PER_TYPE + k] = s;
 }
+
+// Scratch of the FP64 network: activations, the weight-gradient partials of one launch (two
+// CTAs per SM), the node arrays u, du, au, ad and the node adjoints of a batch of replicas.
+constexpr int kWgradCtas = 296, kWgradReps = 16;
+constexpr size_t kActLen = (size_t)MLP_NT * (NG + 1) * NA, kPartLen = (size_t)kWgradCtas * MLP_PER_TYPE,
+                 kNodeLen = (size_t)MLP_NT * (NG + 1);
+constexpr size_t kNodesSmem = sizeof(double) * H * kW2Ld,
+                 kWgradSmem = sizeof(double) * (H * kW2Ld + 6 * kNodes * H);
 
 }  // namespace
 
-// scratch layout: act [NT][NG+1][NA], bwd [NT][NG+1][NA], u, du, au, ad [NT][NG+1]
-size_t mlp_scratch_doubles() { return (size_t)2 * MLP_NT * (NG + 1) * NA + 4 * (size_t)MLP_NT * (NG + 1); }
+// scratch layout: act | partials | u, du, au, ad [NT][NG+1] | au, ad of kWgradReps replicas
+size_t mlp_scratch_doubles() { return kActLen + kPartLen + 4 * kNodeLen + 2 * kWgradReps * kNodeLen; }
+
+double *mlp_scratch_nodes(double *scratch, int which) {
+    return scratch + kActLen + kPartLen + (size_t)which * kNodeLen;   // 0: u, 1: du, 2: au, 3: ad
+}
 
 cudaError_t launch_mlp_table(int prec, const double *theta, double rc, double *scratch, void *tab,
                              cudaStream_t st, int nt, double w) {
     if (nt < 1 || nt > MLP_NT) return cudaErrorInvalidValue;
-    const size_t S = (size_t)MLP_NT * (NG + 1) * NA, NN = (size_t)MLP_NT * (NG + 1);
-    double *act = scratch, *u = scratch + 2 * S, *du = u + NN;
-    k_mlp_nodes<<<dim3(NG + 1, nt), 64, 0, st>>>(theta, rc, w, act, u, du);
-    const int n = nt * NG;
-    if (prec == 1)
-        k_mlp_coef<float4><<<(n + 255) / 256, 256, 0, st>>>(u, du, rc, nt, (float4 *)tab);
-    else
-        k_mlp_coef<double4><<<(n + 255) / 256, 256, 0, st>>>(u, du, rc, nt, (double4 *)tab);
-    return cudaGetLastError();
+    k_mlp_nodes<<<dim3((NG + kNodes) / kNodes, nt), kMlpThreads, kNodesSmem, st>>>(
+        theta, rc, w, scratch, mlp_scratch_nodes(scratch, 0), mlp_scratch_nodes(scratch, 1));
+    return launch_mlp_table_from_nodes(prec, scratch, rc, tab, st, nt);
 }
 
 // The tensor-core path (rs_mlp_tc.cu) shares the node arrays of this scratch: the interval
@@ -253,19 +367,13 @@ cudaError_t launch_mlp_table(int prec, const double *theta, double rc, double *s
 cudaError_t launch_mlp_table_from_nodes(int prec, double *scratch, double rc, void *tab, cudaStream_t st,
                                         int nt) {
     if (nt < 1 || nt > MLP_NT) return cudaErrorInvalidValue;
-    const size_t S = (size_t)MLP_NT * (NG + 1) * NA, NN = (size_t)MLP_NT * (NG + 1);
-    double *u = scratch + 2 * S, *du = u + NN;
+    const double *u = mlp_scratch_nodes(scratch, 0), *du = mlp_scratch_nodes(scratch, 1);
     const int n = nt * NG;
     if (prec == 1)
         k_mlp_coef<float4><<<(n + 255) / 256, 256, 0, st>>>(u, du, rc, nt, (float4 *)tab);
     else
         k_mlp_coef<double4><<<(n + 255) / 256, 256, 0, st>>>(u, du, rc, nt, (double4 *)tab);
     return cudaGetLastError();
-}
-
-double *mlp_scratch_nodes(double *scratch, int which) {
-    const size_t S = (size_t)MLP_NT * (NG + 1) * NA, NN = (size_t)MLP_NT * (NG + 1);
-    return scratch + 2 * S + (size_t)which * NN;   // 0: u, 1: du, 2: au, 3: ad
 }
 
 cudaError_t launch_mlp_node_adjoints(const double *cadj, int ncopy, double rc, double *scratch, cudaStream_t st,
@@ -277,16 +385,26 @@ cudaError_t launch_mlp_node_adjoints(const double *cadj, int ncopy, double rc, d
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_backprop(const double *theta, double rc, const double *cadj, int ncopy,
-                                double *scratch, double *dtheta, cudaStream_t st, int nt, double w) {
+// Chunks per (replica, type): as many as give every SM two CTAs, at most one per node batch.
+cudaError_t launch_mlp_backprop(const double *theta, double rc, const double *cadj, int R, int ncopy,
+                                double *scratch, double *dtheta, cudaStream_t st, int *n_kernels, int nt, double w) {
     if (nt < 1 || nt > MLP_NT) return cudaErrorInvalidValue;
-    const size_t S = (size_t)MLP_NT * (NG + 1) * NA, NN = (size_t)MLP_NT * (NG + 1);
-    double *act = scratch, *bwd = scratch + S;
-    double *au = scratch + 2 * S + 2 * NN, *ad = au + NN;
-    const int nn = nt * (NG + 1), np = nt * MLP_PER_TYPE;
-    k_mlp_adj_nodes<<<(nn + 255) / 256, 256, 0, st>>>(cadj, ncopy, nt, rc, au, ad);
-    k_mlp_node_bwd<<<dim3(NG + 1, nt), 64, 0, st>>>(theta, act, au, ad, bwd);
-    k_mlp_wgrad<<<(np + 127) / 128, 128, 0, st>>>(rc, w, nt, act, bwd, dtheta);
+    cudaError_t e = cudaFuncSetAttribute(k_mlp_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgradSmem);
+    if (e != cudaSuccess) return e;
+    double *part = scratch + kActLen, *au = mlp_scratch_nodes(scratch, 4);
+    const int nn = nt * (NG + 1);
+    *n_kernels = 0;
+    for (int r0 = 0; r0 < R; r0 += kWgradReps) {
+        const int rb = std::min(kWgradReps, R - r0);
+        const int C = std::min((NG + kNodes) / kNodes, kWgradCtas / (rb * nt));
+        double *ad = au + (size_t)rb * nn;
+        k_mlp_adj_nodes<<<dim3((nn + 255) / 256, rb), 256, 0, st>>>(cadj + (size_t)r0 * ncopy * nt * NG * 4, ncopy, nt,
+                                                                    rc, au, ad);
+        k_mlp_wgrad<<<dim3(C, nt, rb), kMlpThreads, kWgradSmem, st>>>(theta, rc, w, nt, scratch, au, ad, part);
+        k_mlp_wgrad_sum<<<dim3((MLP_PER_TYPE + 255) / 256, rb * nt), 256, 0, st>>>(
+            C, part, dtheta + (size_t)r0 * nt * MLP_PER_TYPE);
+        *n_kernels += 3;
+    }
     return cudaGetLastError();
 }
 

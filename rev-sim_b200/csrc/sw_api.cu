@@ -481,14 +481,11 @@ int grads_out(revsim_sw_handle *h, double scale, double *out) {
     RC(reduce_part(h, sw));
     std::vector<double> ml;
     if (h->mlp) {
-        for (int r = 0; r < h->R; r++) {
-            cudaError_t e = launch_mlp_backprop(h->d_mlp_theta, MLP_RC,
-                                                h->d_mlp_adj + (size_t)r * MLP_NCOPY * MLP_NG * 4, MLP_NCOPY,
-                                                h->d_mlp_scratch, h->d_mlp_grad + (size_t)r * MLP_PER_TYPE,
-                                                h->st, 1, MLP_W);
-            h->launches += 3;
-            if (e != cudaSuccess) return fail(h, REVSIM_ERR_CUDA, std::string("MLP backprop: ") + cudaGetErrorString(e));
-        }
+        int nk = 0;
+        const cudaError_t e = launch_mlp_backprop(h->d_mlp_theta, MLP_RC, h->d_mlp_adj, h->R, MLP_NCOPY, h->d_mlp_scratch,
+                                                  h->d_mlp_grad, h->st, &nk, 1, MLP_W);
+        h->launches += nk;
+        if (e != cudaSuccess) return fail(h, REVSIM_ERR_CUDA, std::string("MLP backprop: ") + cudaGetErrorString(e));
         ml.resize((size_t)h->R * MLP_PER_TYPE);
         CK(cudaMemcpyAsync(ml.data(), h->d_mlp_grad, sizeof(double) * ml.size(), cudaMemcpyDeviceToHost, h->st));
         CK(cudaStreamSynchronize(h->st));
