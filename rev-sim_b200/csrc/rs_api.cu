@@ -85,9 +85,14 @@ struct revsim_handle {
     // CTA -> (replica, first molecule, molecule count) table.
     struct Shape {
         int G = 32, mpc = 8, U = 1, n_blk = 0;
+        // molecules per CTA of the table: the default's (step_default) until a shape is set, then
+        // mpc or as many as fit with the update warps
+        int cta = 8;
+        bool set = false;
         int *d_blk_rep = nullptr, *d_blk_mol0 = nullptr, *d_blk_nmol = nullptr;
     } shp[2];
     bool shift_ok = false;   // one periodic image per molecule pair is exact for every box
+    double shift_min() const { return 2 * (rc + 2 * kRext) + 0.02; }
     int cap = 0;
 
     // tables
@@ -420,7 +425,9 @@ int launch_step_k(revsim_handle *h, bool rev, const StepArgs &a_in) {
     a.blk_rep = sh.d_blk_rep;
     a.blk_mol0 = sh.d_blk_mol0;
     a.blk_nmol = sh.d_blk_nmol;
-    const int threads = sh.G * sh.mpc;
+    const int threads = sh.G * sh.cta;
+    a.n_pair = threads;
+    a.shift_box = h->shift_min();
     const BondConsts bc = bond_consts(h);
     const bool timed = h->ktime && !(a.mode & MODE_FORCES_ONLY);
     const int which = rev ? 0 : 1;
@@ -445,11 +452,11 @@ int launch_step_k(revsim_handle *h, bool rev, const StepArgs &a_in) {
                         h->st);
         h->launches++;
     } else if (h->prec == REVSIM_MIXED)
-        e = launch_step<float>(rev, h->mlp ? (int)F_LJ_MLP : h->form, sh.G, sh.U, h->shift_ok, sh.n_blk,
-                               threads, a, nb_consts<float>(h), bc, h->st);
+        e = launch_step<float>(rev, h->mlp ? (int)F_LJ_MLP : h->form, sh.G, sh.U, sh.n_blk, sh.cta, a,
+                               nb_consts<float>(h), bc, h->st);
     else
-        e = launch_step<double>(rev, h->mlp ? (int)F_LJ_MLP : h->form, sh.G, sh.U, h->shift_ok, sh.n_blk,
-                                threads, a, nb_consts<double>(h), bc, h->st);
+        e = launch_step<double>(rev, h->mlp ? (int)F_LJ_MLP : h->form, sh.G, sh.U, sh.n_blk, sh.cta, a,
+                                nb_consts<double>(h), bc, h->st);
     h->launches++;
     if (e != cudaSuccess) return fail(h, REVSIM_ERR_CUDA, std::string("step kernel: ") + cudaGetErrorString(e));
     if (timed) {
@@ -464,11 +471,12 @@ int launch_step_k(revsim_handle *h, bool rev, const StepArgs &a_in) {
 int build_block_table(revsim_handle *h, int dir) {
     revsim_handle::Shape &sh = h->shp[dir];
     std::vector<int> br, bm, bn;
+    if (sh.set) sh.cta = step_cta_mols(h->prec == REVSIM_MIXED, dir == 0, sh.U, sh.G, sh.mpc);
     for (int r = 0; r < h->R; r++)
-        for (int m = 0; m < h->nmol[r]; m += sh.mpc) {
+        for (int m = 0; m < h->nmol[r]; m += sh.cta) {
             br.push_back(r);
             bm.push_back(h->mol0[r] + m);
-            bn.push_back(std::min(sh.mpc, h->nmol[r] - m));
+            bn.push_back(std::min(sh.cta, h->nmol[r] - m));
         }
     sh.n_blk = (int)br.size();
     dfree(sh.d_blk_rep);
@@ -810,7 +818,7 @@ int set_cells(revsim_handle *h) {
         coff[r] = ncell;
         ncell += nc[r] * nc[r] * nc[r];
         lmax = std::max(lmax, h->box[r]);
-        if (!(h->box[r] > 2 * (h->rc + 2 * kRext) + 0.02)) h->shift_ok = false;
+        if (!(h->box[r] > h->shift_min())) h->shift_ok = false;
     }
     h->band = (float)(2e-5 * std::max(1.0, lmax / 4.0));
     if (nc == h->nc) return REVSIM_OK;
@@ -1230,7 +1238,7 @@ int32_t revsim_create(const revsim_system_desc *d, revsim_handle **out) {
     h->Pt = h->P + (h->mlp ? MLP_NPARAMS : 0);
     h->shift_ok = true;
     for (int r = 0; r < h->R; r++)
-        if (!(h->box[r] > 2 * (h->rc + 2 * kRext) + 0.02)) h->shift_ok = false;
+        if (!(h->box[r] > h->shift_min())) h->shift_ok = false;
 
     if (cudaSetDevice(h->dev) != cudaSuccess || cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess) {
         delete h;
@@ -1316,6 +1324,12 @@ int32_t revsim_create(const revsim_system_desc *d, revsim_handle **out) {
          cudaMemset(h->d_C, 0, sizeof(double) * n3) == cudaSuccess &&
          cudaMemset(h->d_A, 0, sizeof(double) * n3) == cudaSuccess;
     if (!ok) return cfail("upload");
+    for (int dir = 0; dir < 2; dir++) {
+        const StepShape d0 = step_default(h->prec == REVSIM_MIXED, dir == 0, h->M);
+        h->shp[dir].G = d0.G;
+        h->shp[dir].U = d0.U;
+        h->shp[dir].cta = d0.cta;
+    }
     if (build_block_table(h, 0) != REVSIM_OK || build_block_table(h, 1) != REVSIM_OK ||
         alloc_nbr(h, cap) != REVSIM_OK)
         return cfail("tables");
@@ -2140,7 +2154,7 @@ bool shape_ok(const revsim_handle *h, int dir, int G, int m, int U) {
           !(U == 3 && thr > 256)))
         return false;
     if (half_eff(h) && thr > half_max_threads(dir == 0)) return false;
-    return thr <= step_max_threads(h->prec == REVSIM_MIXED, dir == 0, U);
+    return thr <= shape_max_threads(h->prec == REVSIM_MIXED, dir == 0, U);
 }
 
 // Shape of one step kernel (dir 0 reverse, 1 forward), after shape_ok.
@@ -2149,11 +2163,9 @@ int set_shape_dir(revsim_handle *h, int dir, int G, int m, int U) {
     h->gen++;
     sh.G = G;
     sh.U = U;
-    if (m != sh.mpc || !sh.d_blk_rep) {
-        sh.mpc = m;
-        int rc = build_block_table(h, dir);
-        if (rc) return rc;
-    }
+    sh.mpc = m;
+    sh.set = true;
+    if (step_cta_mols(h->prec == REVSIM_MIXED, dir == 0, U, G, m) != sh.cta || !sh.d_blk_rep) return build_block_table(h, dir);
     return REVSIM_OK;
 }
 
@@ -2172,10 +2184,11 @@ int32_t revsim_set_pair_mode(revsim_handle *h, int32_t mode) {
     h->half_req = want;
     h->gen++;
     h->fwd_valid = false;
-    // the half-shell reverse kernel allows fewer threads per CTA: shrink a shape beyond it
+    // the half-shell reverse kernel allows fewer threads per CTA: shrink a shape beyond it (and
+    // give up the default CTA size, which is the fused kernels')
     for (int dir = 0; dir < 2; dir++) {
         revsim_handle::Shape &sh = h->shp[dir];
-        if (shape_ok(h, dir, sh.G, sh.mpc, sh.U)) continue;
+        if (shape_ok(h, dir, sh.G, sh.mpc, sh.U) && sh.set) continue;
         int m = sh.mpc;
         while (m > 1 && !shape_ok(h, dir, sh.G, m, 1)) m--;
         if (int rc = set_shape_dir(h, dir, sh.G, m, 1)) return rc;

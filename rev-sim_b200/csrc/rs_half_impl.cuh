@@ -13,7 +13,7 @@
 //                   own partials and bonded terms go to a per-molecule record.
 //   k_water_gather  the molecule's lanes sum the slots listed at the back of its split row,
 //                   in row order, with a fixed butterfly, add the own partial and finish the
-//                   atoms exactly as the fused kernel's epilogue does (atom_update).
+//                   atoms exactly as the fused kernel's epilogue does (atom_finish).
 //
 // Pair terms are the fused kernel's (water.jl:892-913 forces, 1212-1433 VJP and dtheta): for
 // the pair (a, b) the VJP of atom b is the negated VJP of atom a (the pair's second
@@ -29,6 +29,48 @@
 namespace rs {
 
 namespace {
+
+// The O-O Lennard-Jones form of pair_form on both halves of a register pair at once (the
+// packed instructions round each half as the scalar ones do, so the halves carry the bits of
+// pair_form<R, F_LJ>).  c[0] = sigma^2, c[1] = 24 eps, c[2] = 144 eps / sigma, c[3] = 1/eps.
+template <typename R, bool GRAD>
+__device__ __forceinline__ void lj_form2(const FormConsts<R> &fc, typename PkT<R>::T rinv,
+                                         typename PkT<R>::T invr2, typename PkT<R>::T &F,
+                                         typename PkT<R>::T &dF, typename PkT<R>::T g[2]) {
+    using P = typename PkT<R>::T;
+    P six = xmul(pk1(fc.c[0]), invr2);
+    six = xmul(xmul(six, six), six);
+    const P twelve = xmul(six, six);
+    F = xmul(xmul(pk1(fc.c[1]), rinv), xsub(xadd(twelve, twelve), six));
+    if (GRAD) {
+        dF = xneg(xmul(xmul(pk1(fc.c[1]), invr2), xsub(xmul(pk1(R(26)), twelve), xmul(pk1(R(7)), six))));
+        g[0] = xmul(xmul(pk1(fc.c[2]), rinv), xsub(xmul(pk1(R(4)), twelve), six));
+        g[1] = xmul(F, pk1(fc.c[3]));
+    }
+}
+
+// Displacement of one slot for both entries (FP32 kernels): cx / cy = the neighbour atom's
+// gather coordinate in entry x / y, c = the own atom's; formed per half (the two results land
+// in one register pair) and packed from there on.  The gather coordinates are offsets from
+// per-molecule cell origins (gather_f32) and s carries the entries' origin differences (exact
+// multiples of 0.5 nm).  SHIFT: s also carries one periodic image per molecule pair (chosen
+// from the O-O vector) for all nine atom pairs, the minimum one for every pair within the
+// cutoff whenever L > 2 (cutoff + 2 * max O-H distance); s stays exact, so d + s is the one
+// rounding of a vector within the cutoff.  Otherwise the image is chosen per slot from d + s
+// and applied to s first (s - L rint((d + s) / L), exact), then added to d.
+template <typename R, bool SHIFT>
+__device__ __forceinline__ typename PkT<R>::T slot_d2(R c, R cx, R cy, typename PkT<R>::T s, R L, R invL) {
+    using P = typename PkT<R>::T;
+    const P d = pk(xsub(cx, c), xsub(cy, c));
+    if (SHIFT) return xadd(d, s);
+    const P q = xmul(xadd(d, s), pk1(invL));
+    return xadd(d, xfma(pk(-r_rint(q.x), -r_rint(q.y)), pk1(L), s));
+}
+
+template <typename R>
+__device__ __forceinline__ R image_shift(R d, R L, R hL) {
+    return d > hL ? -L : (d < -hL ? L : R(0));
+}
 
 // One (own atom KA, partner atom KB) slot of two owned entries (halves x and y): as
 // pair_term, with (cx, cy, cz) = ca_a - ca_b for the dtheta contraction, and the partner's
@@ -138,9 +180,9 @@ __device__ __forceinline__ void half_col(uint32_t mx, uint32_t my, const float4 
             cz = pk(xsub(ca[KA][2], cbx[2]), xsub(ca[KA][2], cby[2]));                                \
         }                                                                                             \
         half_term<FORM, REV, KA, KB>((mx >> (3 * KA + KB)) & 1u, (my >> (3 * KA + KB)) & 1u,          \
-                                     slot_d<float, true>(pa[KA].x, pbx.x, pby.x, sh[0], L, invL),     \
-                                     slot_d<float, true>(pa[KA].y, pbx.y, pby.y, sh[1], L, invL),     \
-                                     slot_d<float, true>(pa[KA].z, pbx.z, pby.z, sh[2], L, invL), ex, \
+                                     slot_d2<float, true>(pa[KA].x, pbx.x, pby.x, sh[0], L, invL),     \
+                                     slot_d2<float, true>(pa[KA].y, pbx.y, pby.y, sh[1], L, invL),     \
+                                     slot_d2<float, true>(pa[KA].z, pbx.z, pby.z, sh[2], L, invL), ex, \
                                      ey, ez, cx, cy, cz, nb, f[KA], g[KA], th, pf, pg, madj);         \
     }
     RS_HSLOT(0);
@@ -400,7 +442,9 @@ __global__ void __launch_bounds__(512) k_water_gather(StepArgs a) {
                 Gv[u] = __dadd_rn((double)xadd(o[9 + 3 * k + u], pick3(k, pg[0][u], pg[1][u], pg[2][u])),
                                   (double)o[27 + 3 * k + u]);
         }
-        atom_update<R, REV>(a, I, k, rep, Ld, F, Gv, n2, xn, wpos);
+        AtomState st;
+        atom_load<REV>(a, I, k, rep, st);
+        atom_finish<R, REV>(a, I, k, Ld, st, F, Gv, n2, xn, wpos);
     }
 
     // gather buffer of the next step (as the fused kernel: H atoms next to their O)

@@ -76,40 +76,78 @@ struct BondConsts {
 };
 
 // Register budget per thread of the step kernels (__maxnreg__), by precision, direction and
-// loop form U.  FP32 (two entries per lane step in packed arithmetic): forward 128, reverse
-// 168 (U = 1) and 200 (U = 2, 3); FP64 (one entry per step): 128, and 255 for U = 3.
+// loop form U; a scheduler's 16,384 registers then hold: FP32 forward seven warps, reverse five
+// (U = 1) or four; FP64 forward four, reverse three (U = 1) or two.
 #ifndef RS_NREG_F_FWD
-#define RS_NREG_F_FWD 128
+#define RS_NREG_F_FWD 72
 #endif
 #ifndef RS_NREG_F_REV1
-#define RS_NREG_F_REV1 168
+#define RS_NREG_F_REV1 96
 #endif
 #ifndef RS_NREG_F_REV2
-#define RS_NREG_F_REV2 200
+#define RS_NREG_F_REV2 128
 #endif
-#ifndef RS_NREG_F_REV3
-#define RS_NREG_F_REV3 200
+#ifndef RS_NREG_D_FWD
+#define RS_NREG_D_FWD 128
+#endif
+#ifndef RS_NREG_D_REV1
+#define RS_NREG_D_REV1 168
 #endif
 constexpr int step_nreg(bool fp32, bool rev, int U) {
-    return !fp32 ? (U == 3 ? 255 : 128)
-                 : (!rev ? RS_NREG_F_FWD : (U == 3 ? RS_NREG_F_REV3 : (U == 1 ? RS_NREG_F_REV1 : RS_NREG_F_REV2)));
+    return fp32 ? (!rev ? RS_NREG_F_FWD : (U == 1 ? RS_NREG_F_REV1 : RS_NREG_F_REV2))
+                : (U == 3 ? 255 : (!rev ? RS_NREG_D_FWD : (U == 1 ? RS_NREG_D_REV1 : 255)));
 }
+// Entries a lane of the step kernels takes per iteration: the FP64 reverse kernel has registers
+// for one only, and its U = 2 form spends them on fewer, spill-free warps instead.
+constexpr int step_entries(bool fp32, bool rev, int U) { return U == 2 && (fp32 || !rev) ? 2 : 1; }
 // The largest CTA a kernel of nreg registers per thread can be launched with: a CTA's warps
 // are spread over the SM's four schedulers, each with a quarter (16,384) of the registers, a
 // thread's registers allocated in units of 8.  128 registers: 512 threads; 168: 384; 200 or
 // 255: 256.
 constexpr int max_threads_for(int nreg) { return 32 * 4 * (16384 / (32 * ((nreg + 7) / 8 * 8))); }
 constexpr int step_max_threads(bool fp32, bool rev, int U) { return max_threads_for(step_nreg(fp32, rev, U)); }
-// Row entries of the FP32 step kernels' neighbour loop are loaded this many iterations ahead.
-#ifndef RS_ROW_AHEAD
-#define RS_ROW_AHEAD 1
-#endif
+// The largest shape (pair threads, lanes times molecules) revsim_set_launch_shape takes; a CTA
+// holds as many of its molecules as step_cta_mols allows.
+constexpr int shape_max_threads(bool fp32, bool rev, int U) {
+    return !fp32 ? (U == 3 ? 256 : 512) : (!rev ? 512 : (U == 1 ? 384 : 256));
+}
+// Update warps of the step kernels: ten molecules each, one lane per atom.
+constexpr int kMolsPerUpdateWarp = 10;
+constexpr int update_warps(int mols) { return (mols + kMolsPerUpdateWarp - 1) / kMolsPerUpdateWarp; }
+// Molecules a CTA of the step kernels takes when mols are asked for at G lanes each: the
+// largest count (in whole pair warps) whose pair and update threads fit the register budget.
+constexpr int step_cta_mols(bool fp32, bool rev, int U, int G, int mols) {
+    const int whole = 32 / G;
+    while (mols > whole && G * mols + 32 * update_warps(mols) > step_max_threads(fp32, rev, U)) mols -= whole;
+    return mols;
+}
 // Half-shell pair kernels (k_water_half): forward 128, reverse 168 registers.
 #ifndef RS_NREG_HALF_REV
 #define RS_NREG_HALF_REV 168
 #endif
-constexpr int half_nreg(bool rev) { return rev ? RS_NREG_HALF_REV : RS_NREG_F_FWD; }
+constexpr int half_nreg(bool rev) { return rev ? RS_NREG_HALF_REV : 128; }
 constexpr int half_max_threads(bool rev) { return max_threads_for(half_nreg(rev)); }
+
+// The shape a handle's step kernels start with (revsim_set_launch_shape and revsim_autotune
+// replace it): lanes per molecule G (one count for both directions), loop form U and molecules
+// per CTA, by the molecules M of all replicas.  Few molecules: 32 lanes each and one CTA per SM,
+// as many molecules as that takes (at least three, so that an update warp is not alone); from
+// there on 16 lanes (fewer idle lanes at the rows' ends) in CTAs of four or five pair warps that
+// fill the register file.  The lines lie between the sizes measured (event-timed us per step,
+// 32 | 16 lanes, forward + reverse): mixed 895 12.8 + 16.7 | 15.1 + 19.2, 1,500 14.7 + 19.5 |
+// 16.8 + 22.8, 3,000 20.9 + 31.1 | 18.8 + 28.9, 14,320 56 + 101 | 52 + 90, 73,720 244 + 515 |
+// 224 + 425; FP64 895 16.5 + 20.9 | 18.8 + 25, 2,001 22.9 + 39 | 25 + 40, 3,000 29 + 50 | 28 + 54,
+// 14,320 98 + 205 | 90 + 185.  Before: 32 lanes and eight molecules at every size.
+struct StepShape {
+    int G, U, cta;
+};
+constexpr StepShape step_default(bool fp32, bool rev, int M) {
+    const bool few = M <= (fp32 ? 2200 : 4000);
+    const int per_sm = (M + 147) / 148;
+    if (!few) return {16, 1, !fp32 && rev ? 10 : 8};
+    const int U = rev && (!fp32 || M <= 1200) ? 2 : 1;
+    return {32, U, step_cta_mols(fp32, rev, U, 32, per_sm < 3 ? 3 : (per_sm > 14 ? 14 : per_sm))};
+}
 
 // Everything the step kernels read or write.
 struct StepArgs {
@@ -135,6 +173,8 @@ struct StepArgs {
     // when set it replaces the Philox draw of seed_cur / seed_next.
     const double *noise_cur, *noise_next;
     int mode;
+    int n_pair;        // pair threads per CTA (step kernels; the update warps follow them)
+    double shift_box;  // replicas in boxes above it take one periodic image per molecule pair
     int exact;         // 1: the exactly reversible integrator (grid increments, rs_device.cuh)
     // Half-shell pair evaluation (FP32 kernels, rs_half.cu): each unordered molecule pair is
     // evaluated once, by its owner, which writes the partner's share into a slot; a second
@@ -236,17 +276,14 @@ cudaError_t launch_half(bool rev, int form, int G, int n_blk, int threads, const
 template <typename R, int FORM>
 cudaError_t launch_half_form(bool rev, int G, int n_blk, int threads, const StepArgs &a,
                              const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st);
-// Fused step kernels: lanes per molecule G (8/16/32), entries per iteration unroll (1/2),
-// shift = one periodic image per molecule pair (valid when every box side exceeds
-// 2 (cutoff + 2 * max O-H distance)).
+// Fused step kernels: lanes per molecule G (8/16/32), entries per iteration unroll (1/2/3),
+// mols molecules per CTA.
 template <typename R>
-cudaError_t launch_step(bool rev, int form, int G, int unroll, bool shift, int n_blk, int threads,
-                        const StepArgs &a, const NbConsts<R> &nb, const BondConsts &bc,
-                        cudaStream_t st);
+cudaError_t launch_step(bool rev, int form, int G, int unroll, int n_blk, int mols, const StepArgs &a,
+                        const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st);
 template <typename R, int FORM>
-cudaError_t launch_form(bool rev, int G, int unroll, bool shift, int n_blk, int threads,
-                        const StepArgs &a, const NbConsts<R> &nb, const BondConsts &bc,
-                        cudaStream_t st);
+cudaError_t launch_form(bool rev, int G, int unroll, int n_blk, int mols, const StepArgs &a,
+                        const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st);
 
 // Potential energy and its parameter gradient (rs_energy.cu), one thread per molecule.
 struct EnergyArgs {

@@ -166,16 +166,15 @@ __global__ void k_noise(int N, const int *atom_rep, const int *rep_atom0, const 
 }  // namespace
 
 template <typename R>
-cudaError_t launch_step(bool rev, int form, int G, int unroll, bool shift, int n_blk, int threads,
-                        const StepArgs &a, const NbConsts<R> &nb, const BondConsts &bc,
-                        cudaStream_t st) {
+cudaError_t launch_step(bool rev, int form, int G, int unroll, int n_blk, int mols, const StepArgs &a,
+                        const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st) {
     switch (form) {
-        case F_LJ: return launch_form<R, F_LJ>(rev, G, unroll, shift, n_blk, threads, a, nb, bc, st);
-        case F_DEXP: return launch_form<R, F_DEXP>(rev, G, unroll, shift, n_blk, threads, a, nb, bc, st);
-        case F_BUCK: return launch_form<R, F_BUCK>(rev, G, unroll, shift, n_blk, threads, a, nb, bc, st);
-        case F_LJSC: return launch_form<R, F_LJSC>(rev, G, unroll, shift, n_blk, threads, a, nb, bc, st);
-        case F_BUFF: return launch_form<R, F_BUFF>(rev, G, unroll, shift, n_blk, threads, a, nb, bc, st);
-        case F_LJ_MLP: return launch_form<R, F_LJ_MLP>(rev, G, unroll, shift, n_blk, threads, a, nb, bc, st);
+        case F_LJ: return launch_form<R, F_LJ>(rev, G, unroll, n_blk, mols, a, nb, bc, st);
+        case F_DEXP: return launch_form<R, F_DEXP>(rev, G, unroll, n_blk, mols, a, nb, bc, st);
+        case F_BUCK: return launch_form<R, F_BUCK>(rev, G, unroll, n_blk, mols, a, nb, bc, st);
+        case F_LJSC: return launch_form<R, F_LJSC>(rev, G, unroll, n_blk, mols, a, nb, bc, st);
+        case F_BUFF: return launch_form<R, F_BUFF>(rev, G, unroll, n_blk, mols, a, nb, bc, st);
+        case F_LJ_MLP: return launch_form<R, F_LJ_MLP>(rev, G, unroll, n_blk, mols, a, nb, bc, st);
     }
     return cudaErrorInvalidValue;
 }
@@ -193,9 +192,9 @@ cudaError_t launch_half(bool rev, int form, int G, int n_blk, int threads, const
     return cudaErrorInvalidValue;
 }
 
-template cudaError_t launch_step<float>(bool, int, int, int, bool, int, int, const StepArgs &,
+template cudaError_t launch_step<float>(bool, int, int, int, int, int, const StepArgs &,
                                         const NbConsts<float> &, const BondConsts &, cudaStream_t);
-template cudaError_t launch_step<double>(bool, int, int, int, bool, int, int, const StepArgs &,
+template cudaError_t launch_step<double>(bool, int, int, int, int, int, const StepArgs &,
                                          const NbConsts<double> &, const BondConsts &, cudaStream_t);
 
 cudaError_t launch_pack(int N, int prec, const double *x, const double *C, double mO, double mH,

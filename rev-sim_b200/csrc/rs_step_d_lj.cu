@@ -2,6 +2,6 @@
 #include "rs_step_impl.cuh"
 
 namespace rs {
-template cudaError_t launch_form<double, F_LJ>(bool, int, int, bool, int, int, const StepArgs &,
+template cudaError_t launch_form<double, F_LJ>(bool, int, int, int, int, const StepArgs &,
                                            const NbConsts<double> &, const BondConsts &, cudaStream_t);
 }  // namespace rs

@@ -11,11 +11,13 @@
 //
 // Work decomposition: a group of G lanes owns one molecule; the lanes stride over
 // the molecule's neighbour row (entries of 3 atoms each), accumulate the forces of
-// the 3 own atoms in registers, and reduce them with a fixed xor butterfly.  Lanes
-// 0..2 then finish one atom each (bonded terms in FP64, integrator in FP64).  Every
-// atom's force is computed by exactly one group in a fixed order, so there are no
-// atomics and the forward and reverse kernels produce bit-identical forces.
+// the 3 own atoms in registers, and reduce them in the order of a fixed xor butterfly.
+// Further warps of the CTA, one lane per atom, form the bonded terms meanwhile and then run
+// the FP64 integrator.  Every atom's force is computed by exactly one group in a fixed order,
+// so there are no atomics and the forward and reverse kernels produce bit-identical forces.
 #pragma once
+
+#include <type_traits>
 
 #include "rs_internal.h"
 #include "rs_pack.cuh"
@@ -247,208 +249,27 @@ __device__ __forceinline__ void mlp_adjoint(double *madj, int QI, int gi, R na, 
 // every slot and which needs n . a per slot anyway.
 __host__ __device__ constexpr bool charge_from_forces(int form) { return form != F_LJ_MLP; }
 
-// The O-O Lennard-Jones form of pair_form on both halves of a register pair at once (the
-// packed instructions round each half as the scalar ones do, so the halves carry the bits of
-// pair_form<R, F_LJ>).  c[0] = sigma^2, c[1] = 24 eps, c[2] = 144 eps / sigma, c[3] = 1/eps.
-template <typename R, bool GRAD>
-__device__ __forceinline__ void lj_form2(const FormConsts<R> &fc, typename PkT<R>::T rinv,
-                                         typename PkT<R>::T invr2, typename PkT<R>::T &F,
-                                         typename PkT<R>::T &dF, typename PkT<R>::T g[2]) {
-    using P = typename PkT<R>::T;
-    P six = xmul(pk1(fc.c[0]), invr2);
-    six = xmul(xmul(six, six), six);
-    const P twelve = xmul(six, six);
-    F = xmul(xmul(pk1(fc.c[1]), rinv), xsub(xadd(twelve, twelve), six));
-    if (GRAD) {
-        dF = xneg(xmul(xmul(pk1(fc.c[1]), invr2), xsub(xmul(pk1(R(26)), twelve), xmul(pk1(R(7)), six))));
-        g[0] = xmul(xmul(pk1(fc.c[2]), rinv), xsub(xmul(pk1(R(4)), twelve), six));
-        g[1] = xmul(F, pk1(fc.c[3]));
-    }
-}
-
-// Two-entry form (FP32 kernels).  One (own atom KA, neighbour atom KB) slot of two neighbour
-// entries at once: the .x halves of the displacement (dx, dy, dz), of the VJP differences
-// (ex, ey, ez) = w_b - w_a, of the accumulators and of every intermediate belong to entry
-// "x", the .y halves to entry "y" (rs_pack.cuh).  Evaluated unconditionally: pairs outside the
-// neighbour mask or the cutoff contribute exact zeros, so the nine slots of an entry pair run
-// as straight-line code with no divergence between the lanes of a warp.
+// One (own atom KA, neighbour atom KB) slot with displacement (dx, dy, dz), evaluated
+// unconditionally: pairs outside the neighbour mask or the cutoff contribute exact zeros, so
+// the nine slots of an entry run as straight-line code with no divergence between the lanes of
+// a warp (each lane holds a different neighbour).
 //
 // The slot works with A = F/r and B = (dF/dr - F/r) / r^2 of the radial force F(r): the force
 // on the own atom is -A d, the force Jacobian is M = -(B d d^T + A I), so the VJP adds
-// -(B (d . e) d + A e), and the contraction of dF/dtheta with the adjoint a is
+// -(B (d . e) d + A e), e = w_b - w_a, and the contraction of dF/dtheta with the adjoint a is
 // -(dF/dtheta / r) (d . a).  For the reaction-field Coulomb term F = qq (1/r^2 - 2 k_rf r),
-// A = qq (1/r^3 - 2 k_rf) and B = -3 qq / r^5 in closed form (no separate r, dF or 1/r
-// scaling of the dot products); the O-O form and the learned term add their own A and B.
-// The accumulators receive -A and -B times the vectors ("mA", "mB").
+// A = qq (1/r^3 - 2 k_rf) and B = -3 qq / r^5 in closed form; the O-O form and the learned
+// term add their own A and B.  The accumulators receive -A and -B times the vectors ("mA",
+// "mB").  A dead slot is a zero charge product and a zero weight z on the other terms (its own
+// r is finite: a molecule is never its own neighbour).
+//
+// One entry per lane in both precisions.  FP32 took two entries per lane in packed arithmetic
+// before: that halves the instructions but not the FMA pipe's time, and the second entry's
+// operands held the reverse kernel at 168 registers, 12 warps an SM and 35 % issue (16 x 895
+// waters at 16 lanes: 108 us a reverse and 66 us a forward step); one entry runs at 96
+// registers, 20 warps and 65 % issue (90 and 52 us).
 template <typename R, int FORM, bool REV, int KA, int KB>
-__device__ __forceinline__ void pair_term(bool bitx, bool bity, typename PkT<R>::T dx,
-                                          typename PkT<R>::T dy, typename PkT<R>::T dz,
-                                          typename PkT<R>::T ex, typename PkT<R>::T ey,
-                                          typename PkT<R>::T ez, const R ca[3],
-                                          const NbConsts<R> &nb, typename PkT<R>::T f[3],
-                                          typename PkT<R>::T g[3], typename PkT<R>::T *th,
-                                          typename PkT<R>::T fnc[3], double *madj) {
-    using P = typename PkT<R>::T;
-    constexpr int NF = FormInfo<FORM>::NP;
-    constexpr int PF = FORM == F_LJ_MLP ? F_LJ : FORM;   // the O-O pair form
-    constexpr int QI = (KA > 0) + (KB > 0);
-    constexpr bool OO = KA == 0 && KB == 0;
-    constexpr bool CHG_F = charge_from_forces(FORM);
-    const P r2 = xfma(dz, dz, xfma(dy, dy, xmul(dx, dx)));
-    const bool onx = bitx && r2.x <= nb.rc2;
-    const bool ony = bity && r2.y <= nb.rc2;
-    const R qq = nb.qq[QI];
-    // dead slots: 1/r of r = 1 (finite) and a zero charge product
-    const P rinv = xrsqrt(pk(onx ? r2.x : R(1), ony ? r2.y : R(1)));
-    const P qz = pk(onx ? qq : R(0), ony ? qq : R(0));
-    const P invr2 = xmul(rinv, rinv);
-    const P rinv3 = xmul(invr2, rinv);
-    const P mAc = xmul(qz, xsub(pk1(nb.krf2), rinv3));   // -A of the Coulomb term
-    P mA = mAc;
-    P mB = pk1(R(0));
-    if (REV) mB = xmul(xmul(qz, pk1(R(3))), xmul(rinv3, invr2));   // 3 qq / r^5 = -B
-    P gf[4];
-    if (OO || FORM == F_LJ_MLP) {
-        const P z = pk(onx ? R(1) : R(0), ony ? R(1) : R(0));
-        const P r = xmul(pk(onx ? r2.x : R(1), ony ? r2.y : R(1)), rinv);
-        P Ff = pk1(R(0)), dFf = pk1(R(0));
-        bool have = false;
-        if (OO && nb.fc.on) {
-            have = true;
-            if constexpr (PF == F_LJ) {
-                lj_form2<R, REV>(nb.fc, rinv, invr2, Ff, dFf, gf);
-            } else {
-                // the other O-O forms per half with the scalar code
-                R Fx, Fy, dFx = R(0), dFy = R(0), gx[4], gy[4];
-                pair_form<R, PF, REV>(nb.fc, r.x, rinv.x, invr2.x, Fx, dFx, gx);
-                pair_form<R, PF, REV>(nb.fc, r.y, rinv.y, invr2.y, Fy, dFy, gy);
-                Ff = pk(Fx, Fy);
-                if (REV) {
-                    dFf = pk(dFx, dFy);
-#pragma unroll
-                    for (int p = 0; p < NF; p++) gf[p] = pk(gx[p], gy[p]);
-                }
-            }
-        }
-        int gix = 0, giy = 0;
-        R smx = R(0), smy = R(0);
-        if constexpr (FORM == F_LJ_MLP) {
-            // the learned correction: F -= u'(r), dF/dr -= u''(r)
-            R d1x, d1y, d2x, d2y;
-            mlp_segment<R, REV>(nb, QI, r.x, gix, smx, d1x, d2x);
-            mlp_segment<R, REV>(nb, QI, r.y, giy, smy, d1y, d2y);
-            Ff = xsub(Ff, pk(d1x, d1y));
-            if (REV) dFf = xsub(dFf, pk(d2x, d2y));
-            have = true;
-        }
-        if (have) {
-            Ff = xmul(Ff, z);
-            const P Af = xmul(Ff, rinv);
-            mA = xsub(mA, Af);
-            if (REV) mB = xfma(xsub(Af, xmul(dFf, z)), invr2, mB);
-            if (REV && CHG_F) {
-                // the O-O form's share of the own-atom force, so that the Coulomb share is
-                // known after the row (charge_contraction)
-                fnc[0] = xfma(Af, dx, fnc[0]);
-                fnc[1] = xfma(Af, dy, fnc[1]);
-                fnc[2] = xfma(Af, dz, fnc[2]);
-            }
-        }
-        if (REV) {
-            const P dca = xfma(dz, pk1(ca[2]), xfma(dy, pk1(ca[1]), xmul(dx, pk1(ca[0]))));
-            const P na = xmul(xmul(rinv, dca), z);   // n . a
-            if (OO && nb.fc.on) {
-#pragma unroll
-                for (int p = 0; p < NF; p++) th[p] = xfma(xneg(gf[p]), na, th[p]);
-            }
-            if constexpr (FORM == F_LJ_MLP) {
-                if (onx) mlp_adjoint<R>(madj, QI, gix, na.x, smx, nb.mlp_hinv);
-                if (ony) mlp_adjoint<R>(madj, QI, giy, na.y, smy, nb.mlp_hinv);
-            }
-            // charge, per slot when the learned term is on: acoef . dF/dq_O = (2 / q_O) (-A_c) (d . a)
-            if (!CHG_F) th[NF] = xfma(xmul(mAc, pk1(nb.twoinvq)), dca, th[NF]);
-        }
-    }
-    // force on the own atom: -A d
-    f[0] = xfma(mA, dx, f[0]);
-    f[1] = xfma(mA, dy, f[1]);
-    f[2] = xfma(mA, dz, f[2]);
-    if (REV) {
-        // VJP: -(B (d . e) d + A e)
-        const P mt = xmul(mB, xfma(dz, ez, xfma(dy, ey, xmul(dx, ex))));
-        g[0] = xfma(mt, dx, xfma(mA, ex, g[0]));
-        g[1] = xfma(mt, dy, xfma(mA, ey, g[1]));
-        g[2] = xfma(mt, dz, xfma(mA, ez, g[2]));
-    }
-}
-
-// Displacement of one slot for both entries (FP32 kernels): cx / cy = the neighbour atom's
-// gather coordinate in entry x / y, c = the own atom's; formed per half (the two results land
-// in one register pair) and packed from there on.  The gather coordinates are offsets from
-// per-molecule cell origins (gather_f32) and s carries the entries' origin differences (exact
-// multiples of 0.5 nm).  SHIFT: s also carries one periodic image per molecule pair (chosen
-// from the O-O vector) for all nine atom pairs, the minimum one for every pair within the
-// cutoff whenever L > 2 (cutoff + 2 * max O-H distance); s stays exact, so d + s is the one
-// rounding of a vector within the cutoff.  Otherwise the image is chosen per slot from d + s
-// and applied to s first (s - L rint((d + s) / L), exact), then added to d.
-template <typename R, bool SHIFT>
-__device__ __forceinline__ typename PkT<R>::T slot_d(R c, R cx, R cy, typename PkT<R>::T s, R L, R invL) {
-    using P = typename PkT<R>::T;
-    const P d = pk(xsub(cx, c), xsub(cy, c));
-    if (SHIFT) return xadd(d, s);
-    const P q = xmul(xadd(d, s), pk1(invL));
-    return xadd(d, xfma(pk(-r_rint(q.x), -r_rint(q.y)), pk1(L), s));
-}
-
-template <typename R>
-__device__ __forceinline__ R image_shift(R d, R L, R hL) {
-    return d > hL ? -L : (d < -hL ? L : R(0));
-}
-
-// The three slots of own atom KA against the three atoms of the two neighbour molecules
-// (entry x: pbx, wbx; entry y: pby, wby).
-template <typename R, int FORM, bool REV, bool SHIFT, int KA>
-__device__ __forceinline__ void pair_row(uint32_t maskx, uint32_t masky, const typename V4T<R>::T &pa,
-                                         const typename V4T<R>::T pbx[3],
-                                         const typename V4T<R>::T pby[3],
-                                         const typename V4T<R>::T &wa,
-                                         const typename V4T<R>::T wbx[3],
-                                         const typename V4T<R>::T wby[3], const R ca[3],
-                                         const typename PkT<R>::T sh[3], R L, R invL,
-                                         const NbConsts<R> &nb, typename PkT<R>::T f[3],
-                                         typename PkT<R>::T g[3], typename PkT<R>::T *th,
-                                         typename PkT<R>::T fnc[3], double *madj) {
-    using P = typename PkT<R>::T;
-#define RS_SLOT(KB)                                                                               \
-    {                                                                                             \
-        P ex = pk1(R(0)), ey = pk1(R(0)), ez = pk1(R(0));                                         \
-        if (REV) {                                                                                \
-            ex = pk(xsub(wbx[KB].x, wa.x), xsub(wby[KB].x, wa.x));                                \
-            ey = pk(xsub(wbx[KB].y, wa.y), xsub(wby[KB].y, wa.y));                                \
-            ez = pk(xsub(wbx[KB].z, wa.z), xsub(wby[KB].z, wa.z));                                \
-        }                                                                                         \
-        pair_term<R, FORM, REV, KA, KB>((maskx >> (3 * KA + KB)) & 1u, (masky >> (3 * KA + KB)) & 1u, \
-                                        slot_d<R, SHIFT>(pa.x, pbx[KB].x, pby[KB].x, sh[0], L, invL), \
-                                        slot_d<R, SHIFT>(pa.y, pbx[KB].y, pby[KB].y, sh[1], L, invL), \
-                                        slot_d<R, SHIFT>(pa.z, pbx[KB].z, pby[KB].z, sh[2], L, invL), \
-                                        ex, ey, ez, ca, nb, f, g, th, fnc, madj);                 \
-    }
-    RS_SLOT(0);
-    RS_SLOT(1);
-    RS_SLOT(2);
-#undef RS_SLOT
-}
-
-// Single-entry form of the slots, used by the FP64 kernels (no packed FP64 arithmetic, and
-// two entries per lane would exceed their registers).
-// One (own atom KA, neighbour atom KB) interaction with displacement (dx, dy, dz),
-// evaluated unconditionally: pairs outside the neighbour mask or the cutoff
-// contribute exact zeros, so the nine slots of an entry run as straight-line code with
-// no divergence between the lanes of a warp (each lane holds a different neighbour).
-// Same A / B formulation as the two-entry form.
-template <typename R, int FORM, bool REV, int KA, int KB>
-__device__ __forceinline__ void pair_term1(bool bit, R dx, R dy, R dz,
-                                          const typename V4T<R>::T &wa,
+__device__ __forceinline__ void pair_term(bool bit, R dx, R dy, R dz, const typename V4T<R>::T &wa,
                                           const typename V4T<R>::T &wb, const R ca[3],
                                           const NbConsts<R> &nb, R f[3], R g[3], R *th,
                                           R fnc[3], double *madj) {
@@ -459,8 +280,7 @@ __device__ __forceinline__ void pair_term1(bool bit, R dx, R dy, R dz,
     constexpr bool CHG_F = charge_from_forces(FORM);
     const R r2 = xfma(dz, dz, xfma(dy, dy, xmul(dx, dx)));
     const bool on = bit && r2 <= nb.rc2;
-    const R r2s = on ? r2 : R(1);
-    const R rinv = xrsqrt(r2s);
+    const R rinv = xrsqrt(r2);
     const R qz = on ? nb.qq[QI] : R(0);
     const R invr2 = xmul(rinv, rinv);
     const R rinv3 = xmul(invr2, rinv);
@@ -472,29 +292,21 @@ __device__ __forceinline__ void pair_term1(bool bit, R dx, R dy, R dz,
     if (REV && (OO || !CHG_F)) dca = xfma(dz, ca[2], xfma(dy, ca[1], xmul(dx, ca[0])));
     if (OO || FORM == F_LJ_MLP) {
         const R z = on ? R(1) : R(0);
-        const R r = xmul(r2s, rinv);
+        const R r = xmul(r2, rinv);
         R Ff = R(0), dFf = R(0), gf[4];
         bool have = false;
         if (OO && nb.fc.on) {
             have = true;
             pair_form<R, PF, REV>(nb.fc, r, rinv, invr2, Ff, dFf, gf);
         }
-        // Learned pair correction: the cubic segment of interval gi of type QI (O-O, O-H,
-        // H-H), F -= u'(r) = (c1 + 2 c2 s + 3 c3 s^2) / h, dF/dr -= (2 c2 + 6 c3 s) / h^2.
         int gi = 0;
         R sm = R(0);
         if constexpr (FORM == F_LJ_MLP) {
-            using V4m = typename V4T<R>::T;
-            const R q = xmul(r, nb.mlp_hinv);
-            gi = min((int)q, MLP_NG - 1);
-            sm = xsub(q, (R)gi);
-            const V4m cf = reinterpret_cast<const V4m *>(nb.mlp_tab)[QI * MLP_NG + gi];
-            const R d1 = xmul(xfma(sm, xfma(xmul(R(3), sm), cf.w, xmul(R(2), cf.z)), cf.y), nb.mlp_hinv);
+            // the learned correction: F -= u'(r), dF/dr -= u''(r)
+            R d1, d2;
+            mlp_segment<R, REV>(nb, QI, r, gi, sm, d1, d2);
             Ff = xsub(Ff, d1);
-            if (REV) {
-                const R d2 = xmul(xmul(xfma(xmul(R(6), sm), cf.w, xmul(R(2), cf.z)), nb.mlp_hinv), nb.mlp_hinv);
-                dFf = xsub(dFf, d2);
-            }
+            if (REV) dFf = xsub(dFf, d2);
             have = true;
         }
         if (have) {
@@ -503,6 +315,8 @@ __device__ __forceinline__ void pair_term1(bool bit, R dx, R dy, R dz,
             mA = xsub(mA, Af);
             if (REV) mB = xfma(xsub(Af, xmul(dFf, z)), invr2, mB);
             if (REV && CHG_F) {
+                // the O-O form's share of the own-atom force, so that the Coulomb share is
+                // known after the row
                 fnc[0] = xfma(Af, dx, fnc[0]);
                 fnc[1] = xfma(Af, dy, fnc[1]);
                 fnc[2] = xfma(Af, dz, fnc[2]);
@@ -515,14 +329,7 @@ __device__ __forceinline__ void pair_term1(bool bit, R dx, R dy, R dz,
                 for (int p = 0; p < NF; p++) th[p] = xfma(-gf[p], na, th[p]);
             }
             if constexpr (FORM == F_LJ_MLP) {
-                // -(dF/dc_k) (n . acoef_a) for the interval's coefficients c1, c2, c3
-                if (on) {
-                    const double v = (double)na * (double)nb.mlp_hinv, s1 = (double)sm;
-                    double *adj = madj + ((size_t)QI * MLP_NG + gi) * 4;
-                    atomicAdd(adj + 1, v);
-                    atomicAdd(adj + 2, 2.0 * s1 * v);
-                    atomicAdd(adj + 3, 3.0 * s1 * s1 * v);
-                }
+                if (on) mlp_adjoint<R>(madj, QI, gi, na, sm, nb.mlp_hinv);
             }
         }
     }
@@ -542,33 +349,47 @@ __device__ __forceinline__ void pair_term1(bool bit, R dx, R dy, R dz,
     }
 }
 
-// Displacement of one slot.  SHIFT: one periodic image per molecule pair (chosen from
-// the O-O vector) is applied to all nine atom pairs; d + s rounds exactly as Molly's
-// (c2 - c1) -/+ L, and the image is the minimum one for every pair within the cutoff
-// whenever L > 2 (cutoff + 2 * max O-H distance).  Otherwise per-slot vec_mi.
+// Nearest integer of a small FP32 value by the rounding of a sum with 1.5 x 2^23 (two FMA-pipe
+// instructions; rint is a slow conversion).  It differs from rint only on ties.
+__device__ __forceinline__ float near_int(float a, float b) {
+    return xsub(xfma(a, b, 12582912.f), 12582912.f);
+}
+
+// Displacement of one slot.  SHIFT: one periodic image per molecule pair, chosen from the O-O
+// vector and the minimum one for every pair within the cutoff whenever L > 2 (cutoff + 2 * max
+// O-H distance).  Otherwise the image is chosen per slot.  FP64: d + s rounds exactly as Molly's
+// (c2 - c1) -/+ L; vec_mi per slot.  FP32: the gather coordinates are offsets from per-molecule
+// cell origins (gather_f32) and s carries the origins' difference (an exact multiple of 0.5 nm)
+// and, with SHIFT, the image; s stays exact, so d + s is the one rounding of a vector within the
+// cutoff.
 template <typename R, bool SHIFT>
-__device__ __forceinline__ R slot_d1(R ca_, R cb_, R s, R L, R invL) {
-    if (SHIFT) return xadd(xsub(cb_, ca_), s);
+__device__ __forceinline__ R slot_d(R ca_, R cb_, R s, R L, R invL) {
+    const R d = xsub(cb_, ca_);
+    if (SHIFT) return xadd(d, s);
+    if constexpr (sizeof(R) == 4) return xadd(d, xfma(-near_int(xadd(d, s), invL), L, s));
     return vec_mi(ca_, cb_, L, invL);
 }
 
-template <typename R, bool SHIFT>
-__device__ __forceinline__ R image_shift1(R d, R L, R hL) {
-    return d > hL ? -L : (d < -hL ? L : R(0));
+// The image shift of the O-O vector d, added to the origins' difference o (FP64: no origins).
+__device__ __forceinline__ float image_of(float d, float o, float L, float invL) {
+    return xfma(-near_int(d, invL), L, o);
+}
+__device__ __forceinline__ double image_of(double d, double, double L, double) {
+    return d > 0.5 * L ? -L : (d < -0.5 * L ? L : 0.0);
 }
 
 template <typename R, int FORM, bool REV, bool SHIFT, int KA>
-__device__ __forceinline__ void pair_row1(uint32_t mask, const typename V4T<R>::T &pa,
+__device__ __forceinline__ void pair_row(uint32_t mask, const typename V4T<R>::T &pa,
                                          const typename V4T<R>::T pb[3],
                                          const typename V4T<R>::T &wa,
                                          const typename V4T<R>::T wb[3], const R ca[3],
                                          const R sh[3], R L, R invL, const NbConsts<R> &nb,
                                          R f[3], R g[3], R *th, R fnc[3], double *madj) {
 #define RS_SLOT(KB)                                                                             \
-    pair_term1<R, FORM, REV, KA, KB>((mask >> (3 * KA + KB)) & 1u,                               \
-                                    slot_d1<R, SHIFT>(pa.x, pb[KB].x, sh[0], L, invL),           \
-                                    slot_d1<R, SHIFT>(pa.y, pb[KB].y, sh[1], L, invL),           \
-                                    slot_d1<R, SHIFT>(pa.z, pb[KB].z, sh[2], L, invL), wa, wb[KB], \
+    pair_term<R, FORM, REV, KA, KB>((mask >> (3 * KA + KB)) & 1u,                               \
+                                    slot_d<R, SHIFT>(pa.x, pb[KB].x, sh[0], L, invL),           \
+                                    slot_d<R, SHIFT>(pa.y, pb[KB].y, sh[1], L, invL),           \
+                                    slot_d<R, SHIFT>(pa.z, pb[KB].z, sh[2], L, invL), wa, wb[KB], \
                                     ca, nb, f, g, th, fnc, madj)
     RS_SLOT(0);
     RS_SLOT(1);
@@ -576,12 +397,67 @@ __device__ __forceinline__ void pair_row1(uint32_t mask, const typename V4T<R>::
 #undef RS_SLOT
 }
 
+// What an atom's update reads besides its force: the FP64 state and the step's noise.  Loaded
+// before the force is known (atom_load), so that the loads and the noise draw are off the
+// step's critical path, and every load precedes the atom's stores (the state arrays are
+// distinct, but the compiler cannot know that and would otherwise serialise the components).
+struct AtomState {
+    double x[3], v[3], B[3], A[3], D[3], C[3], xi[3];
+};
+
+template <bool REV>
+__device__ __forceinline__ void atom_load(const StepArgs &a, int I, int k, int rep, AtomState &s) {
+    const size_t ia = 3 * (size_t)I + k;
+#pragma unroll
+    for (int u = 0; u < 3; u++) {
+        s.x[u] = a.x[3 * ia + u];
+        s.xi[u] = 0.0;
+    }
+    if (a.mode & MODE_FORCES_ONLY) return;
+    const bool fuse = !REV || (a.mode & MODE_FUSE_NEXT) != 0;
+#pragma unroll
+    for (int u = 0; u < 3; u++) {
+        const size_t e = 3 * ia + u;
+        s.v[u] = a.v[e];
+        if (REV) {
+            if (!(a.mode & MODE_DEFER_BA)) {
+                s.B[u] = a.B[e];
+                s.A[u] = a.A[e];
+            }
+            if (fuse) {
+                s.D[u] = a.D[e];
+                s.C[u] = a.C[e];
+            }
+        }
+    }
+    // noise of this step (forward) or of the next reverse step (fused part 1)
+    if (fuse && a.s != 0.0) {
+        const double *given = REV ? a.noise_next : a.noise_cur;
+        if (given) {
+#pragma unroll
+            for (int u = 0; u < 3; u++) s.xi[u] = given[3 * ia + u];
+        } else {
+            const uint32_t la = (uint32_t)(ia - a.rep_atom0[rep]);
+            atom_noise(REV ? a.seed_next[rep] : a.seed_cur[rep], la, k == 0 ? a.rep_sdO[rep] : a.rep_sdH[rep], s.xi);
+        }
+    }
+}
+
+// wrap1d without its division for a coordinate already inside the box (floor(c / L) is 0
+// there: c / L < 1 rounds below 1), which all but a few atoms of a step are.
+__device__ __forceinline__ double wrap_near(double c, double L) {
+    return c >= 0.0 && c < L ? c : wrap1d(c, L);
+}
+__device__ __forceinline__ double wrap_exact_near(double c, double L) {
+    return c >= 0.0 && c < L ? c : wrap_exact(c, L);
+}
+
 // The per-atom update of a step after the pair, bonded and reduction phases: forces F and
 // VJP Gv of atom k of molecule I (FP64 sums), then forces-only output, the forward B-A-O-A
 // update or the reverse un-kick with the adjoint updates and the next step's part 1.
 // n2 receives |Gv|^2, xn the new FP64 position when wpos.
 template <typename R, bool REV>
-__device__ __forceinline__ void atom_update(const StepArgs &a, int I, int k, int rep, double Ld,
+__device__ __forceinline__ void atom_finish(const StepArgs &a, int I, int k, double Ld, const AtomState &s,
                                             const double F[3], const double Gv[3], double &n2,
                                             double xn[3], bool &wpos) {
     using V4 = typename V4T<R>::T;
@@ -592,7 +468,6 @@ __device__ __forceinline__ void atom_update(const StepArgs &a, int I, int k, int
     // divides as water.jl does.
     const double dtm = k == 0 ? a.dtm_O : a.dtm_H, invm = k == 0 ? a.invm_O : a.invm_H;
     if (!isfinite(F[0]) || !isfinite(F[1]) || !isfinite(F[2])) atomicOr(a.status, ST_NAN);
-    const double xk[3] = {a.x[3 * ia], a.x[3 * ia + 1], a.x[3 * ia + 2]};
     if (a.mode & MODE_FORCES_ONLY) {
 #pragma unroll
         for (int u = 0; u < 3; u++) {
@@ -601,32 +476,19 @@ __device__ __forceinline__ void atom_update(const StepArgs &a, int I, int k, int
         }
     } else if (!REV) {
         // B-A-O-A (water.jl:1032-1037)
-        const uint32_t la = (uint32_t)(ia - a.rep_atom0[rep]);
-        // every load before the first store: the state arrays are distinct, but the compiler
-        // cannot know that, and would otherwise serialise the three components
-        const double vk[3] = {a.v[3 * ia], a.v[3 * ia + 1], a.v[3 * ia + 2]};
-        double xi[3] = {0.0, 0.0, 0.0};
-        if (a.s != 0.0) {
-            if (a.noise_cur) {
-#pragma unroll
-                for (int u = 0; u < 3; u++) xi[u] = a.noise_cur[3 * ia + u];
-            } else {
-                atom_noise(a.seed_cur[rep], la, k == 0 ? a.rep_sdO[rep] : a.rep_sdH[rep], xi);
-            }
-        }
         const bool ex = a.exact != 0;
 #pragma unroll
         for (int u = 0; u < 3; u++) {
-            double v = vk[u], x = xk[u];
+            double v = s.v[u], x = s.x[u];
             const double kick = ex ? __dmul_rn(F[u], dtm) : __ddiv_rn(__dmul_rn(F[u], a.dt), m);
             v = __dadd_rn(v, ex ? qgrid(kick) : kick);
             const double h1 = __dmul_rn(__dmul_rn(v, a.dt), 0.5);
             x = __dadd_rn(x, ex ? qgrid(h1) : h1);
-            v = __dadd_rn(__dmul_rn(v, a.c), __dmul_rn(xi[u], a.s));
+            v = __dadd_rn(__dmul_rn(v, a.c), __dmul_rn(s.xi[u], a.s));
             if (ex) v = qgrid(v);
             const double h2 = __dmul_rn(__dmul_rn(v, a.dt), 0.5);
             x = __dadd_rn(x, ex ? qgrid(h2) : h2);
-            x = ex ? wrap_exact(x, Ld) : wrap1d(x, Ld);
+            x = ex ? wrap_exact_near(x, Ld) : wrap_near(x, Ld);
             a.v[3 * ia + u] = v;
             a.x[3 * ia + u] = x;
             xn[u] = x;
@@ -636,31 +498,6 @@ __device__ __forceinline__ void atom_update(const StepArgs &a, int I, int k, int
         const double dt2 = __dmul_rn(a.dt, a.dt);
         const bool fuse = (a.mode & MODE_FUSE_NEXT) != 0;
         const bool defer = (a.mode & MODE_DEFER_BA) != 0;
-        // every load before the first store (as in the forward branch)
-        double vk[3], Bk[3], Ak[3], Dk[3], Ck[3];
-#pragma unroll
-        for (int u = 0; u < 3; u++) {
-            const size_t e = 3 * ia + u;
-            vk[u] = a.v[e];
-            if (!defer) {
-                Bk[u] = a.B[e];
-                Ak[u] = a.A[e];
-            }
-            if (fuse) {
-                Dk[u] = a.D[e];
-                Ck[u] = a.C[e];
-            }
-        }
-        double xi[3] = {0.0, 0.0, 0.0};
-        if (fuse && a.s != 0.0) {
-            if (a.noise_next) {
-#pragma unroll
-                for (int u = 0; u < 3; u++) xi[u] = a.noise_next[3 * ia + u];
-            } else {
-                const uint32_t la = (uint32_t)(ia - a.rep_atom0[rep]);
-                atom_noise(a.seed_next[rep], la, k == 0 ? a.rep_sdO[rep] : a.rep_sdH[rep], xi);
-            }
-        }
         double Cm[3];
 #pragma unroll
         for (int u = 0; u < 3; u++) {
@@ -669,28 +506,28 @@ __device__ __forceinline__ void atom_update(const StepArgs &a, int I, int k, int
             n2 = __dadd_rn(n2, __dmul_rn(Gv[u], Gv[u]));
             // v_{n-1} = v' - F dt / m (water.jl:1516)
             const double kick = a.exact ? __dmul_rn(F[u], dtm) : __ddiv_rn(__dmul_rn(F[u], a.dt), m);
-            double v = __dsub_rn(vk[u], a.exact ? qgrid(kick) : kick);
+            double v = __dsub_rn(s.v[u], a.exact ? qgrid(kick) : kick);
             if (!defer) {
                 // water.jl:1520-1521
-                const double B = __dadd_rn(__dmul_rn(a.c, Bk[u]), __dmul_rn(dt2, Gv[u]));
+                const double B = __dadd_rn(__dmul_rn(a.c, s.B[u]), __dmul_rn(dt2, Gv[u]));
                 a.B[e] = B;
-                a.A[e] = __dadd_rn(Ak[u], B);
+                a.A[e] = __dadd_rn(s.A[u], B);
             }
             if (fuse) {
                 // part 1 of the next reverse step (water.jl:1496-1502)
-                double x = xk[u];
+                double x = s.x[u];
                 const double h2 = __dmul_rn(__dmul_rn(v, a.dt), 0.5);
                 x = __dsub_rn(x, a.exact ? qgrid(h2) : h2);
-                v = __dsub_rn(v, __dmul_rn(xi[u], a.s));
+                v = __dsub_rn(v, __dmul_rn(s.xi[u], a.s));
                 if (a.c != 1.0) v = __ddiv_rn(v, a.c);   // v / 1 is v: the same bits at gamma = 0
                 if (a.exact) v = qgrid(v);
                 const double h1 = __dmul_rn(__dmul_rn(v, a.dt), 0.5);
                 x = __dsub_rn(x, a.exact ? qgrid(h1) : h1);
-                x = a.exact ? wrap_exact(x, Ld) : wrap1d(x, Ld);
+                x = a.exact ? wrap_exact_near(x, Ld) : wrap_near(x, Ld);
                 // (dt^2 G (1 + c)) / 2, the halving as the (exact) product with 0.5
-                const double D = __dadd_rn(__dmul_rn(a.c, Dk[u]),
+                const double D = __dadd_rn(__dmul_rn(a.c, s.D[u]),
                                            __dmul_rn(__dmul_rn(__dmul_rn(dt2, Gv[u]), __dadd_rn(1.0, a.c)), 0.5));
-                const double C = __dadd_rn(Ck[u], D);
+                const double C = __dadd_rn(s.C[u], D);
                 a.D[e] = D;
                 a.C[e] = C;
                 a.x[e] = x;
@@ -711,118 +548,235 @@ __device__ __forceinline__ void atom_update(const StepArgs &a, int I, int k, int
     }
 }
 
+// Sum N values over the G lanes of a group, each total left in one lane: at every level a lane
+// gives away half of its values and adds the other half of its partner's, so N values cost
+// about N + log2 G shuffles instead of N log2 G.  The pairs added at each level are those of
+// group_sum's butterfly, so the totals are the same bits.  On return v[0 .. M) (M = N halved
+// log2 G times, rounded up) hold the totals of values base .. min(base + M, end).
+template <int G, int N, typename R>
+struct GroupScatter {
+    static constexpr int HALF = (N + 1) / 2;
+    static constexpr int M = GroupScatter<G / 2, HALF, R>::M;
+    static __device__ __forceinline__ void run(R *v, int lane, int &base, int &end) {
+        const bool up = (lane & (G / 2)) != 0;
+#pragma unroll
+        for (int i = 0; i < HALF; i++) {
+            const R hi = i + HALF < N ? v[i + HALF] : R(0);
+            const R send = up ? v[i] : hi;
+            v[i] = xadd(up ? hi : v[i], __shfl_xor_sync(0xffffffffu, send, G / 2));
+        }
+        if (up) base += HALF;
+        else end = min(end, base + HALF);
+        GroupScatter<G / 2, HALF, R>::run(v, lane, base, end);
+    }
+};
+template <int N, typename R>
+struct GroupScatter<1, N, R> {
+    static constexpr int M = N;
+    static __device__ __forceinline__ void run(R *, int, int &, int &) {}
+};
+
 // Register budget per thread: step_nreg (rs_internal.h).
 template <typename R, bool REV, int U>
 constexpr int step_maxnreg() {
     return step_nreg(sizeof(R) == 4, REV, U);
 }
 
-// U = 1: one neighbour entry (FP32: entry pair) per lane per iteration; 2: two, all loads
+// U = 1: one neighbour entry per lane per iteration; 2: two, all loads
 // issued first; 3: one, with the next one's indices and coordinates loaded while the
-// current one is computed (software pipelining; launched with at most 256 threads).  Every
+// current one is computed (software pipelining; launched with at most 256 pair threads).  Every
 // form sums a lane's entries in the same order, so at one lane count they give the same bits.
-template <typename R, int FORM, int G, bool REV, bool SHIFT, int U>
+//
+// Pair warps and update warps.  The first n_pair threads of a CTA are the pair lanes (G per
+// molecule): they walk the rows, reduce the molecule's sums and leave them in shared memory.
+// The warps behind them own the molecules' remaining work, ten molecules a warp, one lane per
+// atom: while the pair warps walk the rows they load the FP64 state, draw the noise and (first
+// lane of each molecule) form the bonded terms; after the CTA's barrier they run the
+// integrator.  With all of that on lanes 0-2 of every pair group, a molecule cost ~2,300 warp
+// instructions outside its row at 32 lanes (5,080 in all, reverse, ncu on 16 x 895 waters),
+// nearly all with 1-3 lanes active, and its latency came before and after the row's.
+//
+// Bound by instruction issue (65 % at 16 x 895 waters, FMA pipe 47 %) where molecules are many
+// and by the latency of one row where they are few.  Event-timed us per forward | reverse step
+// at the default shapes, with the former kernels and now: mixed 895 waters 16.8 | 21.8 -> 12.8 |
+// 16.7, 3,000 27.2 | 42 -> 18.8 | 29, 16 x 895 85 | 150 -> 52 | 90; FP64 895 25 | 43 -> 16.6 |
+// 20.9, 3,000 47.5 | 97 -> 29 | 50, 16 x 895 159 | 338 -> 90 | 185.
+template <typename R, int FORM, int G, bool REV, int U>
 __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a, NbConsts<R> nb,
                                                                       BondConsts bc) {
     using V4 = typename V4T<R>::T;
     constexpr int NF = FormInfo<FORM>::NP;
     constexpr int NTH = NF + 1;
-    // dynamic shared memory: [groups][22] bonded results (R): forces (9), VJP (9), dtheta (4)
+    constexpr int NS = REV ? 18 + NTH : 9;   // sums per molecule: forces, VJP, dtheta
+    // dynamic shared memory: [molecules][NS] sums, then [molecules][22] bonded results:
+    // forces (9), VJP (9), dtheta (4)
     extern __shared__ double s_dyn[];
+    R *s_sum = (R *)s_dyn, *s_bonded = s_sum + NS * (a.n_pair / G);
     chain_enter();
 
-    const int grp = threadIdx.x / G;
-    const int lane = threadIdx.x % G;
     const int blk = blockIdx.x;
     const int rep = a.blk_rep[blk];
-    const int I = a.blk_mol0[blk] + grp;
-    const bool active = grp < a.blk_nmol[blk];
+    const int mol0 = a.blk_mol0[blk], nmol = a.blk_nmol[blk];
     const double Ld = a.rep_box[rep];
+    const V4 *__restrict__ wgt = (const V4 *)a.wgt_in;
+
+    if ((int)threadIdx.x >= a.n_pair) {
+        // ---------------------------------------------------------------- update warps
+        const int l = threadIdx.x & 31;
+        const int mol = ((int)threadIdx.x - a.n_pair) / 32 * kMolsPerUpdateWarp + l / 3, k = l % 3;
+        const bool live = l < 3 * kMolsPerUpdateWarp && mol < nmol;
+        const int I = mol0 + (live ? mol : 0);
+        R *sb = s_bonded + 22 * mol;
+        AtomState st;
+        constexpr int NPT = NF + 5;   // classical parameters, NPL of them per lane
+        constexpr int NPL = (NPT + 2) / 3;
+        double pold[NPL];
+        if (live) {
+            if (k == 0) {
+                double xm[9];
+#pragma unroll
+                for (int u = 0; u < 9; u++) xm[u] = a.x[9 * (size_t)I + u];
+                R w[9], ac[9];
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    V4 wq;
+                    wq.x = wq.y = wq.z = R(0);
+                    if (REV) wq = wgt[3 * I + q];
+                    w[3 * q] = wq.x;
+                    w[3 * q + 1] = wq.y;
+                    w[3 * q + 2] = wq.z;
+                    const double sc = q == 0 ? a.acoefO : a.acoefH;
+#pragma unroll
+                    for (int u = 0; u < 3; u++)
+                        ac[3 * q + u] = REV ? (R)__dmul_rn(a.A[9 * (size_t)I + 3 * q + u], sc) : R(0);
+                }
+                R Fb[9], Gb[9], tb[4];
+                bonded<R, REV>(xm, Ld, bc, w, ac, Fb, Gb, tb);
+#pragma unroll
+                for (int u = 0; u < 9; u++) {
+                    sb[u] = Fb[u];
+                    if (REV) sb[9 + u] = Gb[u];
+                }
+                if (REV) {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) sb[18 + q] = tb[q];
+                }
+            }
+            atom_load<REV>(a, I, k, rep, st);
+            if (REV) {
+#pragma unroll
+                for (int q = 0; q < NPL; q++) {
+                    const int p = k + 3 * q;
+                    pold[q] = p < NPT ? a.part[(size_t)I * NPT + p] : 0.0;
+                }
+            }
+        }
+        __syncthreads();   // the pair warps' sums; every read of the old state and adjoints
+
+        double n2 = 0.0;
+        double xn[3] = {0.0, 0.0, 0.0};   // new FP64 position of the lane's atom
+        bool wpos = false;
+        const R *ss = s_sum + NS * mol;
+        if (live) {
+            double F[3], Gv[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                F[u] = __dadd_rn((double)ss[3 * k + u], (double)sb[3 * k + u]);
+                if (REV) Gv[u] = __dadd_rn((double)ss[9 + 3 * k + u], (double)sb[9 + 3 * k + u]);
+            }
+            atom_finish<R, REV>(a, I, k, Ld, st, F, Gv, n2, xn, wpos);
+        }
+        // Gather buffer of the next step: H atoms are written next to their O (the molecule's
+        // first lane), so that molecules are contiguous (gather_coord).
+        const int src = l - k;
+        const double o0 = __shfl_sync(0xffffffffu, xn[0], src);
+        const double o1 = __shfl_sync(0xffffffffu, xn[1], src);
+        const double o2 = __shfl_sync(0xffffffffu, xn[2], src);
+        if (wpos) {
+            V4 po;
+            if constexpr (sizeof(R) == 4) {
+                const double xo[3] = {o0, o1, o2};
+                po = gather_f32(xo, xn, k, Ld);   // offsets from the molecule's cell origin
+            } else {
+                po.x = (R)gather_coord(o0, xn[0], k != 0, Ld);
+                po.y = (R)gather_coord(o1, xn[1], k != 0, Ld);
+                po.z = (R)gather_coord(o2, xn[2], k != 0, Ld);
+                po.w = R(0);
+            }
+            ((V4 *)a.pos_out)[3 * (size_t)I + k] = po;
+        }
+        if (REV) {
+            // This molecule's dtheta contributions and |dl_dfi|^2, into its own slots: one
+            // group per molecule and step, so every slot sums its steps in step order.
+            const double n2a = __shfl_sync(0xffffffffu, n2, src + 1 < 32 ? src + 1 : 31);
+            const double n2b = __shfl_sync(0xffffffffu, n2, src + 2 < 32 ? src + 2 : 31);
+            if (live) {
+#pragma unroll
+                for (int q = 0; q < NPL; q++) {
+                    const int p = k + 3 * q;
+                    if (p < NPT)
+                        a.part[(size_t)I * NPT + p] =
+                            __dadd_rn(pold[q], (double)(p < NTH ? ss[18 + p] : sb[18 + p - NTH]));
+                }
+                if (k == 0 && a.norm2) a.norm2[I] = __dadd_rn(__dadd_rn(n2, n2a), n2b);
+            }
+        }
+        return;
+    }
+
+    // -------------------------------------------------------------------- pair warps
+    const int grp = threadIdx.x / G;
+    const int lane = threadIdx.x % G;
+    const int I = mol0 + grp;
+    const bool active = grp < nmol;
     const R L = (R)Ld;
     const R invL = (R)(1.0 / Ld);
     const V4 *__restrict__ pos = (const V4 *)a.pos_in;
-    const V4 *__restrict__ wgt = (const V4 *)a.wgt_in;
     // this replica's accumulator of the learned term's interval-coefficient adjoints
     double *madj = FORM == F_LJ_MLP && REV
                        ? nb.mlp_adj + ((size_t)rep * MLP_NCOPY + (blk % MLP_NCOPY)) * MLP_NT * MLP_NG * 4
                        : nullptr;
 
-    // FP32: two entries per lane step in packed arithmetic (rs_pack.cuh), accumulated in
-    // the halves of f2, g2, th2 and combined after the row loop; FP64: one entry per step
-    // into f, g, th.
-    constexpr bool PACKED = sizeof(R) == 4;
-    using P = typename PkT<R>::T;
-    P f2[3][3], g2[3][3], th2[NTH], fnc2[3];
     R f[3][3], g[3][3], th[NTH], fnc[3];
 #pragma unroll
     for (int k = 0; k < 3; k++)
 #pragma unroll
         for (int u = 0; u < 3; u++) {
-            f2[k][u] = pk1(R(0));
-            g2[k][u] = pk1(R(0));
             f[k][u] = R(0);
             g[k][u] = R(0);
         }
 #pragma unroll
-    for (int p = 0; p < NTH; p++) {
-        th2[p] = pk1(R(0));
-        th[p] = R(0);
-    }
+    for (int p = 0; p < NTH; p++) th[p] = R(0);
 #pragma unroll
-    for (int u = 0; u < 3; u++) {
-        fnc2[u] = pk1(R(0));
-        fnc[u] = R(0);
-    }
+    for (int u = 0; u < 3; u++) fnc[u] = R(0);
 
-    V4 pa[3], wa[3];
-    R ca[3][3];
-    // Bonded terms first, by lane 0 of each group into shared memory, so that their
-    // latency overlaps the neighbour loops of the other lanes and warps.
-    R *s_bond = (R *)s_dyn + 22 * grp;
     if (active) {
+        const uint32_t *__restrict__ row = a.nbr + (size_t)I * a.cap;
+        const int cnt = min(a.nbr_cnt[I], a.cap);
+        // padding entries (past the row end): the row's first neighbour with an empty mask
+        const uint32_t pad = cnt > 0 ? __ldg(row) & 0x7FFFFFu : 0u;
+        auto ent_at = [&](int e) { return e < cnt ? __ldg(row + e) : pad; };
+        // the lane's first row entries (lane + q G, q < 4 covers every loop form)
+        uint32_t first[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) first[q] = ent_at(lane + q * G);
+        V4 pa[3], wa[3];
+        // the contraction weights A dt^2 / (2 m): the row needs the O's (the pair form's slot;
+        // all three with the learned term), the rest are read after it
+        R ca[3][3];
+        auto load_ca = [&](int k) {
+            const double sc = k == 0 ? a.acoefO : a.acoefH;
+#pragma unroll
+            for (int u = 0; u < 3; u++) ca[k][u] = (R)__dmul_rn(a.A[9 * (size_t)I + 3 * k + u], sc);
+        };
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             pa[k] = pos[3 * I + k];
             if (REV) {
                 wa[k] = wgt[3 * I + k];
-                const double sc = k == 0 ? a.acoefO : a.acoefH;
-#pragma unroll
-                for (int u = 0; u < 3; u++) ca[k][u] = (R)__dmul_rn(a.A[9 * (size_t)I + 3 * k + u], sc);
+                if (k == 0 || !charge_from_forces(FORM)) load_ca(k);
             }
         }
-        const uint32_t *__restrict__ row = a.nbr + (size_t)I * a.cap;
-        const int cnt = min(a.nbr_cnt[I], a.cap);
-        // padding entries (past the row end) read molecule 0 with an empty mask
-        auto ent_at = [&](int e) { return e < cnt ? __ldg(row + e) : 0u; };
-        // the lane's first row entries, loaded before the bonded terms so that their latency
-        // overlaps lane 0's bonded arithmetic (entries lane + q G, q < 4 covers every loop form)
-        uint32_t first[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) first[q] = ent_at(lane + q * G);
-        if (lane == 0) {
-            double xm[9];
-#pragma unroll
-            for (int u = 0; u < 9; u++) xm[u] = a.x[9 * (size_t)I + u];
-            R w[9], ac[9];
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                w[3 * k] = REV ? wa[k].x : R(0);
-                w[3 * k + 1] = REV ? wa[k].y : R(0);
-                w[3 * k + 2] = REV ? wa[k].z : R(0);
-#pragma unroll
-                for (int u = 0; u < 3; u++) ac[3 * k + u] = REV ? ca[k][u] : R(0);
-            }
-            R Fb[9], Gb[9], tb[4];
-            bonded<R, REV>(xm, Ld, bc, w, ac, Fb, Gb, tb);
-#pragma unroll
-            for (int u = 0; u < 9; u++) {
-                s_bond[u] = Fb[u];
-                s_bond[9 + u] = Gb[u];
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) s_bond[18 + q] = tb[q];
-        }
-        const R hL = xmul(L, R(0.5));
         auto fetch = [&](uint32_t ent, V4 pbq[3], V4 wbq[3]) {
             const int J = (int)(ent & 0x7FFFFFu);
 #pragma unroll
@@ -831,117 +785,29 @@ __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a
                 if (REV) wbq[k] = wgt[3 * J + k];
             }
         };
-        if constexpr (PACKED) {
-            // Entries e and e + G of the row as one pair (halves x and y); a lane takes the
-            // pairs starting at lane, lane + 2G, lane + 4G, ...
-            auto entry2 = [&](uint32_t ex, uint32_t ey, const V4 pbx[3], const V4 wbx[3], const V4 pby[3],
-                              const V4 wby[3]) {
-                // the entries' cell origins relative to the own molecule's (exact multiples of
-                // 0.5 nm, gather_f32) and, with SHIFT, the periodic image from the O-O vector:
-                // s = origin difference + image shift, exact, added to each slot's offset difference
-                R ox[3], oy[3];
-#pragma unroll
-                for (int u = 0; u < 3; u++) {
-                    ox[u] = xsub(pbx[u].w, pa[u].w);
-                    oy[u] = xsub(pby[u].w, pa[u].w);
-                }
-                P sh[3] = {pk(ox[0], oy[0]), pk(ox[1], oy[1]), pk(ox[2], oy[2])};
-                if (SHIFT) {
-                    sh[0] = pk(xadd(ox[0], image_shift(xadd(xsub(pbx[0].x, pa[0].x), ox[0]), L, hL)),
-                               xadd(oy[0], image_shift(xadd(xsub(pby[0].x, pa[0].x), oy[0]), L, hL)));
-                    sh[1] = pk(xadd(ox[1], image_shift(xadd(xsub(pbx[0].y, pa[0].y), ox[1]), L, hL)),
-                               xadd(oy[1], image_shift(xadd(xsub(pby[0].y, pa[0].y), oy[1]), L, hL)));
-                    sh[2] = pk(xadd(ox[2], image_shift(xadd(xsub(pbx[0].z, pa[0].z), ox[2]), L, hL)),
-                               xadd(oy[2], image_shift(xadd(xsub(pby[0].z, pa[0].z), oy[2]), L, hL)));
-                }
-                const uint32_t mx = ex >> 23, my = ey >> 23;
-                pair_row<R, FORM, REV, SHIFT, 0>(mx, my, pa[0], pbx, pby, wa[0], wbx, wby, ca[0], sh, L, invL, nb,
-                                                 f2[0], g2[0], th2, fnc2, madj);
-                pair_row<R, FORM, REV, SHIFT, 1>(mx, my, pa[1], pbx, pby, wa[1], wbx, wby, ca[1], sh, L, invL, nb,
-                                                 f2[1], g2[1], th2, fnc2, madj);
-                pair_row<R, FORM, REV, SHIFT, 2>(mx, my, pa[2], pbx, pby, wa[2], wbx, wby, ca[2], sh, L, invL, nb,
-                                                 f2[2], g2[2], th2, fnc2, madj);
-            };
-            if (U == 3) {
-                // one entry pair per iteration, the next pair's indices and coordinates
-                // loaded while the current pair is computed
-                uint32_t nx = first[0], ny = first[1];
-                V4 pnx[3], wnx[3], pny[3], wny[3];
-                fetch(nx, pnx, wnx);
-                fetch(ny, pny, wny);
-                for (int e = lane; e < cnt; e += 2 * G) {
-                    const uint32_t ex = nx, ey = ny;
-                    V4 pbx[3], wbx[3], pby[3], wby[3];
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        pbx[k] = pnx[k];
-                        pby[k] = pny[k];
-                        if (REV) {
-                            wbx[k] = wnx[k];
-                            wby[k] = wny[k];
-                        }
-                    }
-                    if (e + 2 * G < cnt) {
-                        nx = ent_at(e + 2 * G);
-                        ny = ent_at(e + 3 * G);
-                        fetch(nx, pnx, wnx);
-                        fetch(ny, pny, wny);
-                    }
-                    entry2(ex, ey, pbx, wbx, pby, wby);
-                }
-            } else {
-                // U entry pairs per lane per iteration: all their loads are issued first, and
-                // the row entries are loaded RS_ROW_AHEAD iterations ahead
-                constexpr int UP = U == 3 ? 1 : U;
-                constexpr int D = RS_ROW_AHEAD;
-                constexpr int STEP = 2 * U * G;
-                uint32_t nx[D][UP], ny[D][UP];
-#pragma unroll
-                for (int d = 0; d < D; d++)
-#pragma unroll
-                    for (int q = 0; q < UP; q++) {
-                        nx[d][q] = d == 0 ? first[2 * q] : ent_at(lane + d * STEP + 2 * q * G);
-                        ny[d][q] = d == 0 ? first[2 * q + 1] : ent_at(lane + d * STEP + (2 * q + 1) * G);
-                    }
-                for (int e0 = lane; e0 < cnt; e0 += STEP) {
-                    uint32_t ex[UP], ey[UP];
-#pragma unroll
-                    for (int q = 0; q < UP; q++) {
-                        ex[q] = nx[0][q];
-                        ey[q] = ny[0][q];
-#pragma unroll
-                        for (int d = 0; d + 1 < D; d++) {
-                            nx[d][q] = nx[d + 1][q];
-                            ny[d][q] = ny[d + 1][q];
-                        }
-                        nx[D - 1][q] = ent_at(e0 + D * STEP + 2 * q * G);
-                        ny[D - 1][q] = ent_at(e0 + D * STEP + (2 * q + 1) * G);
-                    }
-                    V4 pbx[UP][3], wbx[UP][3], pby[UP][3], wby[UP][3];
-#pragma unroll
-                    for (int q = 0; q < UP; q++) {
-                        fetch(ex[q], pbx[q], wbx[q]);
-                        fetch(ey[q], pby[q], wby[q]);
-                    }
-#pragma unroll
-                    for (int q = 0; q < UP; q++) entry2(ex[q], ey[q], pbx[q], wbx[q], pby[q], wby[q]);
-                }
-            }
-        } else {
+        // One periodic image per molecule pair where the replica's box allows it (a.shift_box)
+        auto walk = [&](auto shift) {
+        constexpr bool SHIFT = decltype(shift)::value;
+        {
             // one neighbour entry: displacement image and the nine slots
             auto entry = [&](uint32_t ent, const V4 pbq[3], const V4 wbq[3]) {
                 const uint32_t mask = ent >> 23;
                 R sh[3] = {R(0), R(0), R(0)};
-                if (SHIFT) {
-                    sh[0] = image_shift1<R, SHIFT>(xsub(pbq[0].x, pa[0].x), L, hL);
-                    sh[1] = image_shift1<R, SHIFT>(xsub(pbq[0].y, pa[0].y), L, hL);
-                    sh[2] = image_shift1<R, SHIFT>(xsub(pbq[0].z, pa[0].z), L, hL);
+                if constexpr (sizeof(R) == 4) {
+#pragma unroll
+                    for (int u = 0; u < 3; u++) sh[u] = xsub(pbq[u].w, pa[u].w);
                 }
-                pair_row1<R, FORM, REV, SHIFT, 0>(mask, pa[0], pbq, wa[0], wbq, ca[0], sh, L, invL, nb, f[0],
+                if (SHIFT) {
+                    const R dO[3] = {xsub(pbq[0].x, pa[0].x), xsub(pbq[0].y, pa[0].y), xsub(pbq[0].z, pa[0].z)};
+#pragma unroll
+                    for (int u = 0; u < 3; u++)
+                        sh[u] = image_of(sizeof(R) == 4 ? xadd(dO[u], sh[u]) : dO[u], sh[u], L, invL);
+                }
+                pair_row<R, FORM, REV, SHIFT, 0>(mask, pa[0], pbq, wa[0], wbq, ca[0], sh, L, invL, nb, f[0],
                                                   g[0], th, fnc, madj);
-                pair_row1<R, FORM, REV, SHIFT, 1>(mask, pa[1], pbq, wa[1], wbq, ca[1], sh, L, invL, nb, f[1],
+                pair_row<R, FORM, REV, SHIFT, 1>(mask, pa[1], pbq, wa[1], wbq, ca[1], sh, L, invL, nb, f[1],
                                                   g[1], th, fnc, madj);
-                pair_row1<R, FORM, REV, SHIFT, 2>(mask, pa[2], pbq, wa[2], wbq, ca[2], sh, L, invL, nb, f[2],
+                pair_row<R, FORM, REV, SHIFT, 2>(mask, pa[2], pbq, wa[2], wbq, ca[2], sh, L, invL, nb, f[2],
                                                   g[2], th, fnc, madj);
             };
             if (U == 3) {
@@ -963,16 +829,16 @@ __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a
             } else {
                 // U entries per lane per iteration: all their loads are issued first, and the
                 // next iteration's row entries are loaded one iteration ahead
-                constexpr int UE = U == 3 ? 1 : U;
+                constexpr int UE = step_entries(sizeof(R) == 4, REV, U);
                 uint32_t nxt[UE];
 #pragma unroll
                 for (int q = 0; q < UE; q++) nxt[q] = first[q];
-                for (int e0 = lane; e0 < cnt; e0 += U * G) {
+                for (int e0 = lane; e0 < cnt; e0 += UE * G) {
                     uint32_t ent[UE];
 #pragma unroll
                     for (int q = 0; q < UE; q++) {
                         ent[q] = nxt[q];
-                        nxt[q] = ent_at(e0 + U * G + q * G);
+                        nxt[q] = ent_at(e0 + UE * G + q * G);
                     }
                     V4 pb[UE][3], wb[UE][3];
 #pragma unroll
@@ -982,159 +848,83 @@ __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a
                 }
             }
         }
-    }
+        };
+        if (Ld > a.shift_box) walk(std::true_type{});
+        else walk(std::false_type{});
 
     // The charge contraction from the forces (charge_from_forces), per lane on its partial
     // sums: (2 / q_O) sum_k a_k . (F_k - F_form,k), F_form only on the O atom.
     if constexpr (REV && charge_from_forces(FORM)) {
-        if (active) {
-            if constexpr (PACKED) {
-                P q = pk1(R(0));
+        {
+            load_ca(1);
+            load_ca(2);
+            R q = R(0);
 #pragma unroll
-                for (int k = 0; k < 3; k++)
+            for (int k = 0; k < 3; k++)
 #pragma unroll
-                    for (int u = 0; u < 3; u++)
-                        q = xfma(pk1(ca[k][u]), k == 0 ? xadd(f2[0][u], fnc2[u]) : f2[k][u], q);
-                th2[NF] = xfma(pk1(nb.twoinvq), q, th2[NF]);
-            } else {
-                R q = R(0);
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-#pragma unroll
-                    for (int u = 0; u < 3; u++)
-                        q = xfma(ca[k][u], k == 0 ? xadd(f[0][u], fnc[u]) : f[k][u], q);
-                th[NF] = xfma(nb.twoinvq, q, th[NF]);
-            }
+                for (int u = 0; u < 3; u++)
+                    q = xfma(ca[k][u], k == 0 ? xadd(f[0][u], fnc[u]) : f[k][u], q);
+            th[NF] = xfma(nb.twoinvq, q, th[NF]);
         }
     }
+    }   // active
 
-    // FP32: the lane's two halves.  Then a fixed butterfly over the group: every lane ends
-    // with the same totals.
-    if constexpr (PACKED) {
+    // The group's totals, each in one lane, to shared memory.
+    R v[NS];
 #pragma unroll
-        for (int k = 0; k < 3; k++)
-#pragma unroll
-            for (int u = 0; u < 3; u++) {
-                f[k][u] = xadd(f2[k][u].x, f2[k][u].y);
-                g[k][u] = xadd(g2[k][u].x, g2[k][u].y);
-            }
-#pragma unroll
-        for (int p = 0; p < NTH; p++) th[p] = xadd(th2[p].x, th2[p].y);
+    for (int q = 0; q < 9; q++) {
+        v[q] = f[q / 3][q % 3];
+        if (REV) v[9 + q] = g[q / 3][q % 3];
     }
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-        for (int u = 0; u < 3; u++) {
-            f[k][u] = group_sum<G>(f[k][u]);
-            if (REV) g[k][u] = group_sum<G>(g[k][u]);
-        }
     if (REV) {
 #pragma unroll
-        for (int p = 0; p < NTH; p++) th[p] = group_sum<G>(th[p]);
+        for (int p = 0; p < NTH; p++) v[18 + p] = th[p];
     }
-    // Every read of the molecule's FP64 state (bonded terms above) precedes the
-    // per-atom writes below, and lane 0's bonded results are visible to lanes 1, 2.
-    __syncwarp();
-
-    double n2 = 0.0;
-    double xn[3] = {0.0, 0.0, 0.0};   // new FP64 position of the lane's atom
-    bool wpos = false;
-    if (active && lane < 3) {
-        const int k = lane;
-        double F[3], Gv[3] = {0.0, 0.0, 0.0};
+    int base = 0, end = NS;
+    using Sc = GroupScatter<G, NS, R>;
+    Sc::run(v, lane, base, end);
+    if (active) {
 #pragma unroll
-        for (int u = 0; u < 3; u++) {
-            F[u] = __dadd_rn((double)pick3(k, f[0][u], f[1][u], f[2][u]), (double)s_bond[3 * k + u]);
-            if (REV)
-                Gv[u] = __dadd_rn((double)pick3(k, g[0][u], g[1][u], g[2][u]), (double)s_bond[9 + 3 * k + u]);
-        }
-        atom_update<R, REV>(a, I, k, rep, Ld, F, Gv, n2, xn, wpos);
+        for (int q = 0; q < Sc::M; q++)
+            if (base + q < end) s_sum[NS * grp + base + q] = v[q];
     }
-
-    // Gather buffer of the next step: H atoms are written next to their O (lane 0 of
-    // the group), so that molecules are contiguous (gather_coord).
-    {
-        const int src = (threadIdx.x & 31) - lane;
-        const double o0 = __shfl_sync(0xffffffffu, xn[0], src);
-        const double o1 = __shfl_sync(0xffffffffu, xn[1], src);
-        const double o2 = __shfl_sync(0xffffffffu, xn[2], src);
-        if (wpos) {
-            const bool is_h = lane != 0;
-            V4 po;
-            if constexpr (sizeof(R) == 4) {
-                const double xo[3] = {o0, o1, o2};
-                po = gather_f32(xo, xn, lane, Ld);   // offsets from the molecule's cell origin
-            } else {
-                po.x = (R)gather_coord(o0, xn[0], is_h, Ld);
-                po.y = (R)gather_coord(o1, xn[1], is_h, Ld);
-                po.z = (R)gather_coord(o2, xn[2], is_h, Ld);
-                po.w = R(0);
-            }
-            ((V4 *)a.pos_out)[3 * (size_t)I + lane] = po;
-        }
-    }
-
-    if (REV) {
-        // This molecule's dtheta contributions and |dl_dfi|^2, into its own slots: one group
-        // per molecule and step, so every slot sums its steps in step order.
-        const int P = a.P;
-        // lanes 0..2 hold per-atom |G|^2; fold them into lane 0's in order
-        const double n2a = __shfl_sync(0xffffffffu, n2, (threadIdx.x & 31) - lane + 1);
-        const double n2b = __shfl_sync(0xffffffffu, n2, (threadIdx.x & 31) - lane + 2);
-        if (active && lane == 0) {
-            double *pm = a.part + (size_t)I * P;
-#pragma unroll
-            for (int p = 0; p < NTH; p++) pm[p] = __dadd_rn(pm[p], (double)th[p]);
-#pragma unroll
-            for (int q = 0; q < 4; q++) pm[NF + 1 + q] = __dadd_rn(pm[NF + 1 + q], (double)s_bond[18 + q]);
-            if (a.norm2) a.norm2[I] = __dadd_rn(__dadd_rn(n2, n2a), n2b);
-        }
-    }
+    __syncthreads();
 }
 
-// Launch of one (precision, pair form): dispatch on lanes per molecule, image mode
-// and entries per iteration.
-template <typename R, int FORM, int G, bool SHIFT, int U>
-cudaError_t launch_one(bool rev, int n_blk, int threads, const StepArgs &a, const NbConsts<R> &nb,
+// Launch of one (precision, pair form): dispatch on lanes per molecule and entries per
+// iteration; mols = molecules per CTA (a.n_pair = G mols pair threads, then the update warps).
+template <typename R, int FORM, int G, int U>
+cudaError_t launch_one(bool rev, int n_blk, int mols, const StepArgs &a, const NbConsts<R> &nb,
                        const BondConsts &bc, cudaStream_t st) {
-    const size_t smem = sizeof(R) * 22 * (size_t)(threads / G);
+    const int threads = a.n_pair + 32 * update_warps(mols);
+    const size_t smem = sizeof(R) * (size_t)mols * (22 + (rev ? 19 + FormInfo<FORM>::NP : 9));
     if (rev)
-        return launch_chained(k_water_step<R, FORM, G, true, SHIFT, U>, dim3(n_blk), dim3(threads), smem,
-                              st, a, nb, bc);
-    return launch_chained(k_water_step<R, FORM, G, false, SHIFT, U>, dim3(n_blk), dim3(threads), smem, st,
-                          a, nb, bc);
-}
-
-template <typename R, int FORM, int G, bool SHIFT>
-cudaError_t launch_u(bool rev, int unroll, int n_blk, int threads, const StepArgs &a,
-                     const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st) {
-    switch (unroll) {
-        case 1: return launch_one<R, FORM, G, SHIFT, 1>(rev, n_blk, threads, a, nb, bc, st);
-        case 2: return launch_one<R, FORM, G, SHIFT, 2>(rev, n_blk, threads, a, nb, bc, st);
-        case 3:
-            if (threads > 256) return cudaErrorInvalidValue;
-            return launch_one<R, FORM, G, SHIFT, 3>(rev, n_blk, threads, a, nb, bc, st);
-    }
-    return cudaErrorInvalidValue;
+        return launch_chained(k_water_step<R, FORM, G, true, U>, dim3(n_blk), dim3(threads), smem, st, a, nb, bc);
+    return launch_chained(k_water_step<R, FORM, G, false, U>, dim3(n_blk), dim3(threads), smem, st, a, nb, bc);
 }
 
 template <typename R, int FORM, int G>
-cudaError_t launch_g(bool rev, bool shift, int unroll, int n_blk, int threads, const StepArgs &a,
-                     const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st) {
-    if (shift) return launch_u<R, FORM, G, true>(rev, unroll, n_blk, threads, a, nb, bc, st);
-    return launch_u<R, FORM, G, false>(rev, unroll, n_blk, threads, a, nb, bc, st);
+cudaError_t launch_u(bool rev, int unroll, int n_blk, int mols, const StepArgs &a, const NbConsts<R> &nb,
+                     const BondConsts &bc, cudaStream_t st) {
+    switch (unroll) {
+        case 1: return launch_one<R, FORM, G, 1>(rev, n_blk, mols, a, nb, bc, st);
+        case 2: return launch_one<R, FORM, G, 2>(rev, n_blk, mols, a, nb, bc, st);
+        case 3:
+            if (a.n_pair > 256) return cudaErrorInvalidValue;
+            return launch_one<R, FORM, G, 3>(rev, n_blk, mols, a, nb, bc, st);
+    }
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
 template <typename R, int FORM>
-cudaError_t launch_form(bool rev, int G, int unroll, bool shift, int n_blk, int threads,
-                        const StepArgs &a, const NbConsts<R> &nb, const BondConsts &bc,
-                        cudaStream_t st) {
+cudaError_t launch_form(bool rev, int G, int unroll, int n_blk, int mols, const StepArgs &a,
+                        const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st) {
     switch (G) {
-        case 8: return launch_g<R, FORM, 8>(rev, shift, unroll, n_blk, threads, a, nb, bc, st);
-        case 16: return launch_g<R, FORM, 16>(rev, shift, unroll, n_blk, threads, a, nb, bc, st);
-        case 32: return launch_g<R, FORM, 32>(rev, shift, unroll, n_blk, threads, a, nb, bc, st);
+        case 8: return launch_u<R, FORM, 8>(rev, unroll, n_blk, mols, a, nb, bc, st);
+        case 16: return launch_u<R, FORM, 16>(rev, unroll, n_blk, mols, a, nb, bc, st);
+        case 32: return launch_u<R, FORM, 32>(rev, unroll, n_blk, mols, a, nb, bc, st);
     }
     return cudaErrorInvalidValue;
 }
