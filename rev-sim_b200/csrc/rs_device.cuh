@@ -27,9 +27,11 @@ constexpr int ST_ROW_ASYM = 64;   // half-shell split: a row member whose row la
 // be scheduled, so that its CTAs become resident while this one runs and wait at the same
 // point.  Called first, by every thread, before any read of device state or any write.
 // Without the launch attribute both instructions return at once.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    chain_wait();
+    chain_next();
 }
 
 // ---------------------------------------------------------------- arithmetic

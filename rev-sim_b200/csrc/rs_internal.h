@@ -128,25 +128,39 @@ constexpr int step_cta_mols(bool fp32, bool rev, int U, int G, int mols) {
 constexpr int half_nreg(bool rev) { return rev ? RS_NREG_HALF_REV : 128; }
 constexpr int half_max_threads(bool rev) { return max_threads_for(half_nreg(rev)); }
 
+// Molecules per CTA that leave the busiest SM the fewest molecules when all M run as one wave of
+// CTAs, at G lanes each; 0 when no count fits one wave (by the registers).
+constexpr int one_wave_mols(bool fp32, bool rev, int U, int G, int M) {
+    const int cap = step_max_threads(fp32, rev, U) / 32;   // warps an SM holds
+    int best = 0, load = 0;
+    for (int m = 32 / G; m <= 32; m += 32 / G) {
+        const int ctas = ((M + m - 1) / m + 147) / 148, warps = m * G / 32 + update_warps(m);
+        if (ctas * warps > cap || (best && ctas * m > load)) continue;
+        best = m;
+        load = ctas * m;
+    }
+    return best;
+}
+
 // The shape a handle's step kernels start with (revsim_set_launch_shape and revsim_autotune
 // replace it): lanes per molecule G (one count for both directions), loop form U and molecules
-// per CTA, by the molecules M of all replicas.  Few molecules: 32 lanes each and one CTA per SM,
-// as many molecules as that takes (at least three, so that an update warp is not alone); from
-// there on 16 lanes (fewer idle lanes at the rows' ends) in CTAs of four or five pair warps that
-// fill the register file.  The lines lie between the sizes measured (event-timed us per step,
-// 32 | 16 lanes, forward + reverse): mixed 895 12.8 + 16.7 | 15.1 + 19.2, 1,500 14.7 + 19.5 |
-// 16.8 + 22.8, 3,000 20.9 + 31.1 | 18.8 + 28.9, 14,320 56 + 101 | 52 + 90, 73,720 244 + 515 |
-// 224 + 425; FP64 895 16.5 + 20.9 | 18.8 + 25, 2,001 22.9 + 39 | 25 + 40, 3,000 29 + 50 | 28 + 54,
-// 14,320 98 + 205 | 90 + 185.  Before: 32 lanes and eight molecules at every size.
+// per CTA, by the molecules M of all replicas.  While one wave holds them at 32 lanes, 32 lanes;
+// then 16 (fewer idle lanes at the rows' ends), in one wave as long as that goes, else in CTAs of
+// four or five pair warps that fill the register file.  Within one wave the busiest SM sets the
+// time, hence one_wave_mols (3,000 waters, mixed, 16 lanes: 22 molecules in 137 CTAs 17.7 | 23.7
+// us a forward | reverse step, 8 in 375 18.3 | 26.1, 12 in 250 19.5 | 28.0; 2,001 at 32 lanes: 14
+// 13.7 | 16.9, 4 14.9 | 19.2).  FP64's reverse kernel holds seven molecules an SM with the
+// registers it wants, and stays at 32 lanes up to 4,000 all the same (3,000: 26 | 45 at 32 lanes,
+// 25 | 49 at 16; 14,320: 98 | 205 and 90 | 185).  Before: 32 lanes and eight molecules always.
 struct StepShape {
     int G, U, cta;
 };
 constexpr StepShape step_default(bool fp32, bool rev, int M) {
-    const bool few = M <= (fp32 ? 2200 : 4000);
-    const int per_sm = (M + 147) / 148;
-    if (!few) return {16, 1, !fp32 && rev ? 10 : 8};
-    const int U = rev && (!fp32 || M <= 1200) ? 2 : 1;
-    return {32, U, step_cta_mols(fp32, rev, U, 32, per_sm < 3 ? 3 : (per_sm > 14 ? 14 : per_sm))};
+    const int G = (fp32 ? one_wave_mols(true, true, 1, 32, M) > 0 : M <= 4000) ? 32 : 16;
+    const int U = rev && G == 32 && (!fp32 || M <= 1200) ? 2 : 1;
+    const int m = one_wave_mols(fp32, rev, U, G, M);
+    const int fill = G == 32 ? 7 : (!fp32 && rev ? 10 : 8);
+    return {G, U, m ? m : fill};
 }
 
 // Everything the step kernels read or write.
@@ -174,6 +188,7 @@ struct StepArgs {
     const double *noise_cur, *noise_next;
     int mode;
     int n_pair;        // pair threads per CTA (step kernels; the update warps follow them)
+    int chain_early;   // let the next step's CTAs in at the start of this one (see launch_step_k)
     double shift_box;  // replicas in boxes above it take one periodic image per molecule pair
     int exact;         // 1: the exactly reversible integrator (grid increments, rs_device.cuh)
     // Half-shell pair evaluation (FP32 kernels, rs_half.cu): each unordered molecule pair is

@@ -612,7 +612,8 @@ __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a
     // forces (9), VJP (9), dtheta (4)
     extern __shared__ double s_dyn[];
     R *s_sum = (R *)s_dyn, *s_bonded = s_sum + NS * (a.n_pair / G);
-    chain_enter();
+    chain_wait();
+    if (a.chain_early) chain_next();
 
     const int blk = blockIdx.x;
     const int rep = a.blk_rep[blk];
@@ -672,6 +673,7 @@ __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a
             }
         }
         __syncthreads();   // the pair warps' sums; every read of the old state and adjoints
+        if (!a.chain_early) chain_next();
 
         double n2 = 0.0;
         double xn[3] = {0.0, 0.0, 0.0};   // new FP64 position of the lane's atom
@@ -889,6 +891,7 @@ __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a
             if (base + q < end) s_sum[NS * grp + base + q] = v[q];
     }
     __syncthreads();
+    if (!a.chain_early) chain_next();
 }
 
 // Launch of one (precision, pair form): dispatch on lanes per molecule and entries per
