@@ -79,6 +79,7 @@ struct revsim_handle {
     double *d_mlp_r = nullptr, *d_mlp_u = nullptr;   // revsim_mlp_eval buffers
     size_t mlp_eval_cap = 0;
     double *d_epart = nullptr;   // [M][P + 1] energy-gradient partials
+    double *d_sums = nullptr;    // [R][P + 1] per-replica sums of partials
     bool have_params = false, have_state = false;
 
     // Launch shapes of the step kernels, [0] reverse and [1] forward, each with its own
@@ -858,7 +859,7 @@ int replica_energies(revsim_handle *h, const uint32_t *nbr, const int *cnt, std:
     EnergyArgs a = energy_args(h, nbr, cnt);
     a.grads = 0;
     CK(launch_energy_grads(h->mlp ? (int)F_LJ_MLP : h->form, h->prec, a, h->st));
-    CK(launch_rep_energy(h->R, h->d_rep_atom0, h->d_rep_nmol, h->d_epart, h->P, h->d_repE, h->st));
+    CK(launch_rep_sums(h->R, h->d_rep_atom0, h->d_rep_nmol, h->d_epart, h->P + 1, 1, h->d_repE, h->st));
     h->launches += 2;
     E.assign(h->R, 0.0);
     CK(cudaMemcpyAsync(E.data(), h->d_repE, sizeof(double) * h->R, cudaMemcpyDeviceToHost, h->st));
@@ -1142,14 +1143,22 @@ int collect_kernel_times(revsim_handle *h) {
     return REVSIM_OK;
 }
 
-// Sum the dtheta partials per replica (FP64, in slot order).
+// Sum the dtheta partials per replica: on the device for the per-molecule slots, in slot order
+// here for the half-shell kernels' per-CTA slots.
 int reduce_part(revsim_handle *h, std::vector<double> &out) {
+    out.assign((size_t)h->R * h->P, 0.0);
+    if (!half_eff(h)) {
+        CK(launch_rep_sums(h->R, h->d_rep_atom0, h->d_rep_nmol, h->d_part, h->P, h->P, h->d_sums, h->st));
+        h->launches++;
+        CK(cudaMemcpyAsync(out.data(), h->d_sums, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, h->st));
+        CK(cudaStreamSynchronize(h->st));
+        return REVSIM_OK;
+    }
     std::vector<int> owner;
     if (int rc = slot_owner(h, owner)) return fail(h, rc, "block table copy failed");
     std::vector<double> part(owner.size() * h->P);
     CK(cudaMemcpyAsync(part.data(), h->d_part, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
-    out.assign((size_t)h->R * h->P, 0.0);
     for (size_t b = 0; b < owner.size(); b++)
         for (int p = 0; p < h->P; p++) out[(size_t)owner[b] * h->P + p] += part[b * h->P + p];
     return REVSIM_OK;
@@ -1162,7 +1171,7 @@ void free_all(revsim_handle *h) {
         dfree(sh.d_blk_nmol);
     }
     void *mptrs[] = {h->d_mlp_theta, h->d_mlp_adj, h->d_mlp_scratch, h->d_mlp_grad, h->d_mlp_tab,
-                     h->d_epart, h->d_mlp_tc, h->d_mlp_r, h->d_mlp_u};
+                     h->d_epart, h->d_sums, h->d_mlp_tc, h->d_mlp_r, h->d_mlp_u};
     for (void *p : mptrs) dfree(p);
     free_half(h);
     void *ptrs[] = {h->d_mol_rep, h->d_atom_rep,
@@ -1313,7 +1322,8 @@ int32_t revsim_create(const revsim_system_desc *d, revsim_handle **out) {
               dalloc(&h->d_scale, 2 * h->R) == cudaSuccess && dalloc(&h->d_status, 1) == cudaSuccess &&
               dalloc(&h->d_maxcnt, 2) == cudaSuccess && dalloc(&h->d_count, 1) == cudaSuccess &&
               dalloc(&h->d_loss, h->R) == cudaSuccess && dalloc(&h->d_loss_acc, h->R) == cudaSuccess &&
-              dalloc(&h->d_cell_rep, ncell) == cudaSuccess;
+              dalloc(&h->d_cell_rep, ncell) == cudaSuccess &&
+              dalloc(&h->d_sums, (size_t)h->R * (h->P + 1)) == cudaSuccess;
     if (!ok) return cfail("alloc");
     std::vector<int> rep_nmol(h->nmol.begin(), h->nmol.end());
     ok = cudaMemcpy(h->d_mol_rep, mol_rep.data(), sizeof(int) * h->M, cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -1613,16 +1623,15 @@ int32_t revsim_energy_grad(revsim_handle *h, double *energy, double *dEdtheta) {
     cudaError_t e = launch_energy_grads(h->mlp ? (int)F_LJ_MLP : h->form, h->prec, a, h->st);
     h->launches++;
     if (e != cudaSuccess) return fail(h, REVSIM_ERR_CUDA, std::string("energy gradient: ") + cudaGetErrorString(e));
-    std::vector<double> part((size_t)h->M * (h->P + 1));
-    std::vector<int> mol_rep(h->M);
-    CK(cudaMemcpyAsync(part.data(), h->d_epart, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, h->st));
-    CK(cudaMemcpyAsync(mol_rep.data(), h->d_mol_rep, sizeof(int) * h->M, cudaMemcpyDeviceToHost, h->st));
+    CK(launch_rep_sums(h->R, h->d_rep_atom0, h->d_rep_nmol, h->d_epart, h->P + 1, h->P + 1, h->d_sums, h->st));
+    h->launches++;
+    std::vector<double> sums((size_t)h->R * (h->P + 1));
+    CK(cudaMemcpyAsync(sums.data(), h->d_sums, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     std::vector<double> E(h->R, 0.0), cl((size_t)h->R * h->P, 0.0), ml;
-    for (int I = 0; I < h->M; I++) {
-        const int r = mol_rep[I];
-        E[r] += part[(size_t)I * (h->P + 1)];
-        for (int p = 0; p < h->P; p++) cl[(size_t)r * h->P + p] += part[(size_t)I * (h->P + 1) + 1 + p];
+    for (int r = 0; r < h->R; r++) {
+        E[r] = sums[(size_t)r * (h->P + 1)];
+        for (int p = 0; p < h->P; p++) cl[(size_t)r * h->P + p] = sums[(size_t)r * (h->P + 1) + 1 + p];
     }
     if (h->mlp && (rc = mlp_grads(h, ml))) return rc;
     if (energy) std::memcpy(energy, E.data(), sizeof(double) * h->R);

@@ -300,7 +300,7 @@ template <typename R, int FORM>
 cudaError_t launch_form(bool rev, int G, int unroll, int n_blk, int mols, const StepArgs &a,
                         const NbConsts<R> &nb, const BondConsts &bc, cudaStream_t st);
 
-// Potential energy and its parameter gradient (rs_energy.cu), one thread per molecule.
+// Potential energy and its parameter gradient (rs_energy.cu), one warp per molecule.
 struct EnergyArgs {
     int M, P, cap;
     const double *x;
@@ -333,9 +333,10 @@ struct EnthArgs {
     double *acc, *ev_acc, *k, *dgrad;
 };
 cudaError_t launch_enth_finalize(const EnthArgs &a, cudaStream_t st);
-// E[r] = the replica's sum of part[I][0] (fixed-order tree), r < R.
-cudaError_t launch_rep_energy(int R, const int *rep_atom0, const int *rep_nmol, const double *part, int P,
-                              double *E, cudaStream_t st);
+// out[r][c] = the sum over replica r's molecules I of part[I * stride + c], c < ncol <= 10, in a
+// fixed order.
+cudaError_t launch_rep_sums(int R, const int *rep_atom0, const int *rep_nmol, const double *part, int stride,
+                            int ncol, double *out, cudaStream_t st);
 // dLdx[i] += k[replica of atom i / 3] * F[i], i < 3N (dl_ev/dx = (2 e / n) F).
 cudaError_t launch_enth_dldx(int N, const int *atom_rep, const double *k, const double *F, double *dLdx,
                              cudaStream_t st);
