@@ -67,6 +67,7 @@ struct revsim_gas_handle {
         int off = 0;
         double *d_target = nullptr, *d_sum = nullptr, *d_wt = nullptr;   // d_sum: slice sums, then pre
         rs::RdfDen den;
+        std::vector<double> target;   // what the device holds
     };
     std::vector<RdfDev> rdf;
     int *d_rdf_int = nullptr;
@@ -677,6 +678,16 @@ int32_t revsim_gas_set_rdf(revsim_gas_handle *h, int32_t n_terms, const revsim_r
     }
     if (n_terms > 0 && h->nw < 1) return fail(h, REVSIM_ERR_BADARG, "the RDF term needs water molecules");
     CK(cudaSetDevice(h->dev));
+    // the same terms again: nothing to do (forward_sim sets them on every call)
+    bool same = (int)h->rdf.size() == n_terms;
+    for (int i = 0; same && i < n_terms; i++) {
+        const revsim_rdf_term &t = terms[i], &o = h->rdf[i].t;
+        same = t.sel1 == o.sel1 && t.sel2 == o.sel2 && t.x_min == o.x_min && t.step == o.step && t.width == o.width &&
+               t.exp_cutoff == o.exp_cutoff && t.n_grid == o.n_grid && t.slice_start == o.slice_start &&
+               t.slice_stride == o.slice_stride && t.n_target == o.n_target && t.norm == o.norm &&
+               t.weight == o.weight && std::equal(h->rdf[i].target.begin(), h->rdf[i].target.end(), targets[i]);
+    }
+    if (same) return REVSIM_OK;
     CK(cudaStreamSynchronize(h->st));
     free_rdf(h);
     const double pi = 3.14159265358979323846;
@@ -698,6 +709,7 @@ int32_t revsim_gas_set_rdf(revsim_gas_handle *h, int32_t n_terms, const revsim_r
         const double pre = h->L * h->L * h->L / (4 * pi * n1 * n2 * t.step);
         CK(cudaMemcpy(D.d_target, targets[i], sizeof(double) * t.n_target, cudaMemcpyHostToDevice));
         CK(cudaMemcpy(D.d_sum + t.n_target, &pre, sizeof(double), cudaMemcpyHostToDevice));
+        D.target.assign(targets[i], targets[i] + t.n_target);
     }
     return REVSIM_OK;
 }

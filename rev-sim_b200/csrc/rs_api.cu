@@ -52,7 +52,14 @@ struct Term {
     double *d_hist = nullptr;     // [R * n_grid + R]  (histogram, then pre[R])
     double *d_wt = nullptr;       // [R * n_target] gradient weights of the slice points
     RdfDen den;
+    std::vector<double> target, pre;   // what the device holds
 };
+
+bool same_term(const revsim_rdf_term &a, const revsim_rdf_term &b) {
+    return a.sel1 == b.sel1 && a.sel2 == b.sel2 && a.x_min == b.x_min && a.step == b.step && a.width == b.width &&
+           a.exp_cutoff == b.exp_cutoff && a.n_grid == b.n_grid && a.slice_start == b.slice_start &&
+           a.slice_stride == b.slice_stride && a.n_target == b.n_target && a.norm == b.norm && a.weight == b.weight;
+}
 
 }  // namespace
 
@@ -1493,50 +1500,82 @@ int32_t revsim_set_loss(revsim_handle *h, int32_t n_terms, const revsim_rdf_term
                         const double *const *targets) {
     if (!h || n_terms < 0 || (n_terms > 0 && (!terms || !targets))) return REVSIM_ERR_BADARG;
     CK(cudaSetDevice(h->dev));
-    for (Term &T : h->terms) {
+    // A term keeps the buffers of the one it replaces when their sizes are equal, and what they
+    // hold already is not uploaded again: forward_sim and reverse_sim set the same terms on every
+    // call, and six cudaMalloc / cudaFree pairs and the copies took 100-200 us of a pass.
+    std::vector<Term> old;
+    old.swap(h->terms);
+    if ((int)old.size() != n_terms) h->gen++;
+    auto release = [](Term &T) {
         dfree(T.d_target);
         dfree(T.d_hist);
         dfree(T.d_wt);
-    }
-    h->terms.clear();
-    for (int i = 0; i < n_terms; i++) {
+        T.d_target = T.d_hist = T.d_wt = nullptr;
+    };
+    int rc = REVSIM_OK;
+    for (int i = 0; i < n_terms && !rc; i++) {
         const revsim_rdf_term &t = terms[i];
         if (t.n_grid < 1 || !(t.step > 0) || !(t.width > 0) || !(t.exp_cutoff >= 0) || t.n_target < 0 ||
             t.slice_start < 0 || (t.n_target > 0 && (t.slice_stride < 1 ||
                                                      t.slice_start + (long long)(t.n_target - 1) * t.slice_stride >= t.n_grid)) ||
             (t.norm != 1 && t.norm != 2) || (t.sel1 != 0 && t.sel1 != 1) || (t.sel2 != 0 && t.sel2 != 1) ||
-            !targets[i])
-            return fail(h, REVSIM_ERR_BADARG, "bad loss term");
+            !targets[i]) {
+            rc = fail(h, REVSIM_ERR_BADARG, "bad loss term");
+            break;
+        }
         const double q = t.x_min / t.step;
-        if (std::fabs(q - std::llround(q)) > 1e-6)
-            return fail(h, REVSIM_ERR_BADARG, "x_min must be a multiple of step (water.jl:660)");
-        if (!rdf_term_recurrence_ok(t.step, t.width, t.exp_cutoff))
-            return fail(h, REVSIM_ERR_BADARG, "width too small for the grid step and window");
+        if (std::fabs(q - std::llround(q)) > 1e-6) {
+            rc = fail(h, REVSIM_ERR_BADARG, "x_min must be a multiple of step (water.jl:660)");
+            break;
+        }
+        if (!rdf_term_recurrence_ok(t.step, t.width, t.exp_cutoff)) {
+            rc = fail(h, REVSIM_ERR_BADARG, "width too small for the grid step and window");
+            break;
+        }
         Term T;
+        if (i < (int)old.size()) std::swap(T, old[i]);
+        if (!T.d_hist || T.t.n_grid != t.n_grid || T.t.n_target != t.n_target) {
+            release(T);
+            T.target.clear();
+            T.pre.clear();
+            if (dalloc(&T.d_target, (size_t)h->R * std::max(t.n_target, 1)) != cudaSuccess ||
+                dalloc(&T.d_hist, (size_t)h->R * t.n_grid + h->R) != cudaSuccess ||
+                dalloc(&T.d_wt, (size_t)h->R * std::max(t.n_target, 1)) != cudaSuccess) {
+                cudaGetLastError();
+                release(T);
+                rc = fail(h, REVSIM_ERR_NOMEM, "loss buffers");
+                break;
+            }
+            T.den = rdf_den_poly(t.step, t.width, t.exp_cutoff);
+            h->gen++;   // a captured graph holds the term's constants and buffers
+        } else if (!same_term(T.t, t)) {
+            T.den = rdf_den_poly(t.step, t.width, t.exp_cutoff);
+            h->gen++;
+        }
         T.t = t;
         T.off = (int)std::llround(q) - 1;
-        T.den = rdf_den_poly(t.step, t.width, t.exp_cutoff);
-        if (dalloc(&T.d_target, (size_t)h->R * std::max(t.n_target, 1)) != cudaSuccess ||
-            dalloc(&T.d_hist, (size_t)h->R * t.n_grid + h->R) != cudaSuccess ||
-            dalloc(&T.d_wt, (size_t)h->R * std::max(t.n_target, 1)) != cudaSuccess) {
-            dfree(T.d_target);
-            dfree(T.d_hist);
-            dfree(T.d_wt);
-            return fail(h, REVSIM_ERR_NOMEM, "loss buffers");
-        }
-        h->terms.push_back(T);
-        if (t.n_target > 0)
-            CK(cudaMemcpy(T.d_target, targets[i], sizeof(double) * (size_t)h->R * t.n_target, cudaMemcpyHostToDevice));
-        std::vector<double> pre(h->R);
+        std::vector<double> target(targets[i], targets[i] + (size_t)h->R * t.n_target), pre(h->R);
         for (int r = 0; r < h->R; r++) {
             const double n1 = t.sel1 == 0 ? h->nmol[r] : 2.0 * h->nmol[r];
             const double n2 = t.sel2 == 0 ? h->nmol[r] : 2.0 * h->nmol[r];
             const double V = h->box[r] * h->box[r] * h->box[r];
             pre[r] = V / (4 * 3.14159265358979323846 * n1 * n2 * t.step);
         }
-        CK(cudaMemcpy(T.d_hist + (size_t)h->R * t.n_grid, pre.data(), sizeof(double) * h->R, cudaMemcpyHostToDevice));
+        const bool up_t = target != T.target, up_p = pre != T.pre;
+        T.target.swap(target);
+        T.pre.swap(pre);
+        h->terms.push_back(T);
+        const Term &D = h->terms.back();
+        if (up_t && t.n_target > 0 &&
+            cudaMemcpy(D.d_target, D.target.data(), sizeof(double) * D.target.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            rc = fail(h, REVSIM_ERR_CUDA, "loss targets");
+        if (!rc && up_p &&
+            cudaMemcpy(D.d_hist + (size_t)h->R * t.n_grid, D.pre.data(), sizeof(double) * h->R, cudaMemcpyHostToDevice) !=
+                cudaSuccess)
+            rc = fail(h, REVSIM_ERR_CUDA, "loss normalisers");
     }
-    return REVSIM_OK;
+    for (Term &T : old) release(T);
+    return rc;
 }
 
 int32_t revsim_neighbor_pairs(revsim_handle *h, int32_t replica, int32_t *pairs, int64_t cap,
