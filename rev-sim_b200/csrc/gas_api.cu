@@ -49,8 +49,9 @@ struct revsim_gas_handle {
     // gather buffers (32 B per atom: double4 in FP64, float4 in mixed precision) and the FP64
     // copy pos64 of the positions (aliases d_pos in FP64)
     void *d_pos[2] = {nullptr, nullptr}, *d_wgt[2] = {nullptr, nullptr};
-    double4 *d_pos64[2] = {nullptr, nullptr};
-    double4 *d_p64own[2] = {nullptr, nullptr};   // allocations of pos64 in mixed precision
+    double *d_pos64[2] = {nullptr, nullptr};
+    double *d_p64own[2] = {nullptr, nullptr};   // allocations of pos64 in mixed precision
+    float4 *d_posf[2] = {nullptr, nullptr};      // FP32 test positions
     // forward record
     double *d_snap_x = nullptr, *d_snap_v = nullptr;
     size_t snap_cap = 0;   // snapshots
@@ -237,6 +238,8 @@ GasArgs args(revsim_gas_handle *h) {
     a.wgt_out = h->d_wgt[h->cur ^ 1];
     a.pos64_in = h->d_pos64[h->cur];
     a.pos64_out = h->d_pos64[h->cur ^ 1];
+    a.posf_in = h->d_posf[h->cur];
+    a.posf_out = h->d_posf[h->cur ^ 1];
     a.x = h->d_x;
     a.v = h->d_v;
     a.A = h->d_A;
@@ -252,6 +255,9 @@ GasArgs args(revsim_gas_handle *h) {
     a.mH = h->mH;
     a.sdO = std::sqrt(h->kB * h->temp / h->mO);
     a.sdH = std::sqrt(h->kB * h->temp / h->mH);
+    // the cutoff widened by the FP32 distances' error (test_slack) and its own rounding
+    const double rt = h->rc + 2e-6 * h->L;
+    a.rc2_test = (float)(rt * rt * (1 + 1e-6));
     a.bw = h->bw;
     a.kb_g = h->kbg;
     a.r0_g = h->r0g;
@@ -265,6 +271,7 @@ int rebuild(revsim_gas_handle *h) {
     r.L = h->L;
     r.rc_nl2 = h->rc_nl * h->rc_nl;
     r.x = h->d_x;
+    r.posf = h->d_posf[h->cur];
     r.rows = h->d_rows;
     r.cnt = h->d_cnt;
     r.cap = h->cap;
@@ -276,7 +283,7 @@ int rebuild(revsim_gas_handle *h) {
 }
 
 int pack(revsim_gas_handle *h) {
-    launch_gas_pack(h->mixed, h->N, h->d_x, h->d_pos[h->cur], h->d_pos64[h->cur], h->st);
+    launch_gas_pack(h->mixed, h->N, h->nw3, h->L, h->d_x, h->d_pos[h->cur], h->d_pos64[h->cur], h->d_posf[h->cur], h->st);
     h->launches++;
     CK(cudaGetLastError());
     return REVSIM_OK;
@@ -561,7 +568,8 @@ int32_t revsim_gas_destroy(revsim_gas_handle *h) {
     void *bufs[] = {h->d_rows, h->d_cnt, h->d_status, h->d_x, h->d_v, h->d_A, h->d_B, h->d_C,
                     h->d_D, h->d_G, h->d_F, h->d_g, h->d_w, h->d_ac, h->d_part, h->d_epart,
                     h->d_direct, h->d_gtail, h->d_Eloss, h->d_pos[0], h->d_pos[1], h->d_wgt[0],
-                    h->d_wgt[1], h->d_snap_x, h->d_snap_v, h->d_p64own[0], h->d_p64own[1]};
+                    h->d_wgt[1], h->d_snap_x, h->d_snap_v, h->d_p64own[0], h->d_p64own[1],
+                    h->d_posf[0], h->d_posf[1]};
     for (void *p : bufs)
         if (p) cudaFree(p);
     free_rdf(h);
@@ -633,20 +641,21 @@ int32_t revsim_gas_create(const revsim_gas_desc *d, revsim_gas_handle **out) {
         bad(dalloc(&h->d_g, n3)) || bad(dalloc(&h->d_w, n3)) || bad(dalloc(&h->d_ac, n3)) ||
         bad(dalloc(&h->d_part, N * kMaxP)) || bad(dalloc(&h->d_epart, N * (kMaxP + 1))) ||
         bad(dalloc(&h->d_direct, kMaxP + 1)) || bad(dalloc(&h->d_gtail, 6 * (size_t)h->ng)) ||
-        bad(dalloc((double4 **)&h->d_pos[0], N)) || bad(dalloc((double4 **)&h->d_pos[1], N)) ||
-        bad(dalloc((double4 **)&h->d_wgt[0], N)) || bad(dalloc((double4 **)&h->d_wgt[1], N)) ||
-        (h->mixed && (bad(dalloc(&h->d_p64own[0], N)) || bad(dalloc(&h->d_p64own[1], N)))) ||
+        bad(dalloc((double **)&h->d_pos[0], n3)) || bad(dalloc((double **)&h->d_pos[1], n3)) ||
+        bad(dalloc((double **)&h->d_wgt[0], n3)) || bad(dalloc((double **)&h->d_wgt[1], n3)) ||
+        (h->mixed && (bad(dalloc(&h->d_p64own[0], n3)) || bad(dalloc(&h->d_p64own[1], n3)))) ||
+        bad(dalloc(&h->d_posf[0], N)) || bad(dalloc(&h->d_posf[1], N)) ||
         bad(dalloc(&h->d_rdf_int, 2)) ||
         bad(dalloc(&h->d_rdf_box, 1)) || bad(dalloc(&h->d_rdf_dx, 9 * (size_t)h->nw)) ||
         bad(dalloc(&h->d_rdf_tmp, 1)) || bad(cudaMemset(h->d_status, 0, sizeof(int))) ||
-        bad(cudaMemset(h->d_wgt[0], 0, N * sizeof(double4))) ||
-        bad(cudaMemset(h->d_wgt[1], 0, N * sizeof(double4)))) {
+        bad(cudaMemset(h->d_wgt[0], 0, n3 * sizeof(double))) ||
+        bad(cudaMemset(h->d_wgt[1], 0, n3 * sizeof(double)))) {
         cudaGetLastError();
         revsim_gas_destroy(h);
         return REVSIM_ERR_NOMEM;
     }
     for (int b = 0; b < 2; b++)
-        h->d_pos64[b] = h->mixed ? h->d_p64own[b] : static_cast<double4 *>(h->d_pos[b]);
+        h->d_pos64[b] = h->mixed ? h->d_p64own[b] : static_cast<double *>(h->d_pos[b]);
     const int tab[2] = {0, h->nw};
     if (bad(cudaMemcpy(h->d_rdf_int, tab, sizeof(tab), cudaMemcpyHostToDevice)) ||
         bad(cudaMemcpy(h->d_rdf_box, &h->L, sizeof(double), cudaMemcpyHostToDevice))) {
@@ -1018,6 +1027,7 @@ int32_t revsim_gas_reverse(revsim_gas_handle *h, const uint64_t *seeds, double g
             a.seed_next = seeds[s_start - 1];
             a.pos_out = h->d_pos[h->cur];
             a.pos64_out = h->d_pos64[h->cur];
+            a.posf_out = h->d_posf[h->cur];
             a.wgt_out = h->d_wgt[h->cur];
             launch_gas_part1(h->mixed, a, h->st);
             h->launches++;

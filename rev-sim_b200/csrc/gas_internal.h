@@ -12,7 +12,7 @@ namespace gs {
 using rs::BondConsts;
 using rs::FormConsts;
 
-// One warp per atom; four atoms per CTA.
+// Row and energy kernels: one warp per atom, four atoms per CTA.
 constexpr int kWarpsPerCta = 4;
 constexpr int kThreads = 32 * kWarpsPerCta;
 constexpr int kMaxP = 7;
@@ -40,8 +40,9 @@ struct GasConstsT {
 };
 using GasConsts = GasConstsT<double>;
 
-// Gather buffers: V4T<R>::T per atom (float4 in mixed precision, double4 in FP64) of the
-// positions (pos) and of C/m (wgt); the FP64 state x, v, A-D stays authoritative.
+// Gather buffers: [3][N] components in pair precision (float in mixed precision, double in FP64)
+// of the positions (pos) and of C/m (wgt), atoms ordered by site kind (gather_index); the FP64
+// state x, v, A-D stays authoritative, in atom order.
 struct GasArgs {
     int N, nw3;
     double L, invL;
@@ -52,13 +53,19 @@ struct GasArgs {
     void *pos_out;
     const void *wgt_in;
     void *wgt_out;
-    const double4 *pos64_in;   // FP64 positions for the molecule's bonded terms (the same
-    double4 *pos64_out;        // buffers as pos_in / pos_out in FP64)
+    const float4 *posf_in;     // FP32 positions for the distance tests (test_pos), same order
+    float4 *posf_out;
+    const double *pos64_in;    // FP64 positions for the bonded terms (the same buffers as pos_in /
+    double *pos64_out;         // pos_out in FP64)
     double *x, *v, *A, *B, *C, *D, *G, *F_out;
     const double *acoef_in;   // forces-only reverse mode: the contraction weights [3N]
     double *part;       // [N][P] dtheta partials (accumulated)
     int *status;
     double dt, c, s, mO, mH, sdO, sdH;
+    double cfO, cfH;    // dt^2 / (2 m)
+    float rc2_test;     // FP32 r^2 above which a pair is certainly outside the cutoff
+    int apc;            // atoms per CTA (set by the launcher, as chain_early)
+    int chain_early;    // release the next step's CTAs at the start
     uint64_t seed_cur, seed_next;
     int mode;           // rs::MODE_FORCES_ONLY, rs::MODE_FUSE_NEXT
     BondConsts bw;      // water bonds and angle
@@ -69,6 +76,7 @@ struct GasRowArgs {
     int N, nw3;
     double L, rc_nl2;
     const double *x;    // FP64 state [3N]
+    const float4 *posf; // its test positions
     int *rows, *cnt;
     int cap;
     int *status;
@@ -80,8 +88,9 @@ void launch_gas_step(bool mixed, int form, bool rev, const GasConstsT<float> &kf
                      const GasConstsT<double> &kd, const GasArgs &a, cudaStream_t st);
 // part 1 of a reverse step (diffusion.jl:1566-1572) for every atom, writing pos_out / wgt_out
 void launch_gas_part1(bool mixed, const GasArgs &a, cudaStream_t st);
-// pos[a] = pos64[a] = x[a]
-void launch_gas_pack(bool mixed, int N, const double *x, void *pos, double4 *pos64, cudaStream_t st);
+// x into the gather buffers pos, pos64 and posf
+void launch_gas_pack(bool mixed, int N, int nw3, double L, const double *x, void *pos, double *pos64, float4 *posf,
+                     cudaStream_t st);
 // wgt[a] = w[a] / m_a
 void launch_gas_pack_w(bool mixed, int N, int nw3, const double *w, double mO, double mH, void *wgt,
                        cudaStream_t st);

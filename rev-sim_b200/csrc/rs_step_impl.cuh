@@ -355,6 +355,11 @@ __device__ __forceinline__ float near_int(float a, float b) {
     return xsub(xfma(a, b, 12582912.f), 12582912.f);
 }
 
+// FP64, 1.5 x 2^52.
+__device__ __forceinline__ double near_int(double a, double b) {
+    return xsub(xfma(a, b, 6755399441055744.0), 6755399441055744.0);
+}
+
 // Displacement of one slot.  SHIFT: one periodic image per molecule pair, chosen from the O-O
 // vector and the minimum one for every pair within the cutoff whenever L > 2 (cutoff + 2 * max
 // O-H distance).  Otherwise the image is chosen per slot.  FP64: d + s rounds exactly as Molly's
