@@ -96,12 +96,21 @@ __device__ __forceinline__ void den_sums(const RdfArgs &a, double d, double inv_
 
 // The same sums from the polynomial of the pair's window (RdfDen); false where the window is
 // clipped by the grid, is not one of the four of an unclipped pair, or there is no polynomial.
-__device__ __forceinline__ bool den_poly(const RdfArgs &a, const RdfDen &dn, double d, double &den, double &dden) {
+// The window's ends are those of den_window: a product with 1 / step decides them unless it falls
+// within 1e-6 of an integer (its rounding is below 1e-9 on any grid of less than 10^6 points),
+// where the division does.  The cell only has to hold d to rounding.
+__device__ __forceinline__ bool den_poly(const RdfArgs &a, const RdfDen &dn, double inv_step, double d, double &den,
+                                         double &dden) {
     if (dn.M == 0) return false;
-    const long long s = (long long)ceil(__ddiv_rn(__dsub_rn(d, a.cutoff), a.step));
-    const long long e = (long long)floor(__ddiv_rn(__dadd_rn(d, a.cutoff), a.step));
+    const double da = __dsub_rn(d, a.cutoff), db = __dadd_rn(d, a.cutoff);
+    double qa = __dmul_rn(da, inv_step), qb = __dmul_rn(db, inv_step);
+    if (fabs(__dsub_rn(qa, rint(qa))) < 1e-6 || fabs(__dsub_rn(qb, rint(qb))) < 1e-6 || qb > 1e6) {
+        qa = __ddiv_rn(da, a.step);
+        qb = __ddiv_rn(db, a.step);
+    }
+    const long long s = (long long)ceil(qa), e = (long long)floor(qb);
     if (s - a.off < 1 || e - a.off > a.n_grid) return false;
-    const double j = floor(__ddiv_rn(d, a.step));
+    const double j = floor(__dmul_rn(d, inv_step));
     const int ca = (int)(s - (long long)j) + dn.n, cb = (int)(e - (long long)j) - dn.n;
     if (ca < 0 || ca > 1 || cb < 0 || cb > 1) return false;
     const double u = __dsub_rn(d, __dmul_rn(__dadd_rn(j, 0.5), a.step));
@@ -178,21 +187,37 @@ __global__ void k_rdf(RdfArgs a) {
 // see (an FP32 test with a margin far above its rounding).  The atoms that pass are queued
 // per warp and evaluated 32 at a time in FP64, so the window loops run with full warps
 // whatever the fraction in range (5 % in the 4.5 nm box).  Equal sets take each unordered
-// pair once (half ring: i with the next n/2 atoms, modulo n) and count it twice.  Deposits go
-// to one of a few shared-memory copies of the slice sums (lanes that share a copy are eight
-// apart).  The gradient sums atom i's share in registers.
+// pair once (half ring: i with the next n/2 atoms, modulo n) and count it twice.  The gradient
+// sums atom i's share in registers.
 //
-// Bound by the shared-memory FP64 atomics (value) and the FP64 pipe (gradient).  Smearing every
-// ordered pair over the whole grid, as k_rdf does, took 567 us a value and 535 us a gradient on
-// the 895-water box and the experimental grid (4,801 points, of which the loss reads 248 and
-// 281), and 215 / 298 us on the 3,000-water box with the 200-bin O-O term; this form takes
-// 63 / 44 us and 67 / 76 us (mean over the O-O and O-H terms).
+// The value kernel deposits with PTS = 16 or 32 lanes a pair, a lane per slice point, into
+// copies of the slice sums that no other group of lanes touches: plain additions.  PTS = 0 (the
+// window has more points, the sums are too many for the copies, or the factors too far apart)
+// deposits with a lane per pair, shared-memory FP64 atomics on a copy per lane where they fit.
+//
+// Window ends and normaliser cells come from products with 1 / S and 1 / step: divisions only
+// where those lie within 1e-6 of an integer.  The window's ends take two steps without branches:
+// loops that few lanes repeat left a warp's lanes apart for the whole pair (66 us instead of 38 a
+// gradient on the 895-water box).
+//
+// Bound by FP64 latency at 16 to 24 warps an SM (three CTAs an SM at 80 registers suit PTS = 16
+// only: 60 -> 54 us; the others slow by 3-5 us).  Us per value / gradient, mean over the O-O and O-H
+// terms of the experimental grid (4,801 points, of which the loss reads 248 and 281; 27 a window)
+// on the 895-water box, and the 200-bin O-O term (16 a window) on the 3,000-water box: every
+// ordered pair over the whole grid, as k_rdf does, 567 / 535 and 215 / 298; a lane per pair with
+// atomics on eight copies and divisions 63 / 44 and 67 / 76; now 41 / 38 and 54 / 44.
 constexpr int kRlWarps = 8, kRlTile = 256;
+constexpr size_t kRlSmem = 65536;   // dynamic shared memory of a value CTA at most
 
-template <bool GRAD>
-__global__ void __launch_bounds__(32 * kRlWarps) k_rdf_loss(RdfArgs a, RdfSlice sl, RdfDen dn, int split,
+template <bool GRAD, int PTS>
+__global__ void __launch_bounds__(32 * kRlWarps, PTS == 16 ? 3 : 0) k_rdf_loss(RdfArgs a, RdfSlice sl, RdfDen dn, int split,
                                                             int ncopy) {
-    extern __shared__ double s_sum[];   // GRAD false: [nt][ncopy] partial sums (ncopy 0: none)
+    constexpr bool COOP = PTS > 0;
+    constexpr int NC = COOP ? 64 / PTS : 0;   // pairs deposited at a time, copies of the sums a warp
+    // GRAD false: [nt][ncopy] partial sums (ncopy 0: none; COOP: [warps][NC][nt])
+    extern __shared__ double s_sum[];
+    __shared__ double2 s_g[COOP ? kRlWarps : 1][COOP ? 32 : 1];   // a pair's first point and ratio
+    __shared__ int2 s_t[COOP ? kRlWarps : 1][COOP ? 32 : 1];      // its first point's index and their number
     __shared__ float s_x[3][kRlTile];
     __shared__ int s_q[kRlWarps][64];
     const int r = blockIdx.y, nm = a.rep_nmol[r], atom0 = a.rep_atom0[r];
@@ -212,6 +237,7 @@ __global__ void __launch_bounds__(32 * kRlWarps) k_rdf_loss(RdfArgs a, RdfSlice 
     const float Lf = (float)L, hLf = 0.5f * Lf;
     const double inv_w = __drcp_rn(a.width);
     const double S = __dmul_rn(a.step, (double)sl.sd);   // slice spacing
+    const double inv_step = __drcp_rn(a.step), inv_S = __drcp_rn(S), x0 = grid_x(a, sl.s0);
     const double q1 = exp(-__dmul_rn(__dmul_rn(2.0, __dmul_rn(a.step, a.step)), inv_w));
     const double qS = exp(-__dmul_rn(__dmul_rn(2.0, __dmul_rn(S, S)), inv_w));
     const double dmin = __dsub_rn(__dsub_rn(grid_x(a, sl.s0), a.cutoff), a.step);
@@ -221,7 +247,9 @@ __global__ void __launch_bounds__(32 * kRlWarps) k_rdf_loss(RdfArgs a, RdfSlice 
     const float far = (float)dmax + marg, near = fmaxf(0.f, (float)dmin - marg);
     const float far2 = far * far, near2 = near * near;
     const double pair_w = same ? 2.0 : 1.0;
-    if (!GRAD && ncopy > 0) {
+    if (COOP) {
+        for (int k = threadIdx.x; k < sl.nt * NC * kRlWarps; k += blockDim.x) s_sum[k] = 0.0;
+    } else if (!GRAD && ncopy > 0) {
         for (int k = threadIdx.x; k < sl.nt * ncopy; k += blockDim.x) s_sum[k] = 0.0;
     }
     double xi[3] = {0.0, 0.0, 0.0};
@@ -242,25 +270,82 @@ __global__ void __launch_bounds__(32 * kRlWarps) k_rdf_loss(RdfArgs a, RdfSlice 
     double *sums = sl.sum + (size_t)r * sl.nt;
     const double *wt = sl.wt + (size_t)r * sl.nt;
 
-    auto eval = [&](int j) {
-        const int ib = rdf_atom(a.sel2, atom0, j);
-        const double *xb = a.x + 3 * (size_t)ib;
-        double dr[3];
+    // COOP: lane m of PTS deposits point m of a pair, exp(-(e0 + m S)^2 / w) = exp(-e0^2 / w) r^m A_m
+    // with r = exp(-2 e0 S / w)
+    const int m = COOP ? lane % PTS : 0, group = COOP ? lane / PTS : 0;
+    const double Am = COOP ? exp(-__dmul_rn(__dmul_rn((double)m * S, (double)m * S), inv_w)) : 0.0;
+    double *mine = s_sum + (COOP ? ((size_t)warp * NC + group) * sl.nt : 0);
+
+    // The pair of atom i with atom j: the slice points ta .. tb it reaches, its distance,
+    // displacement and normaliser; false if there are none.
+    auto pair_of = [&](int j, double dr[3], double &d, int &ta, int &tb, double &inv_den, double &dden) {
+        const double *xb = a.x + 3 * (size_t)rdf_atom(a.sel2, atom0, j);
 #pragma unroll
         for (int u = 0; u < 3; u++) dr[u] = vec1d(xi[u], xb[u], L);
-        const double d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dr[0], dr[0]), __dmul_rn(dr[1], dr[1])),
+        d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dr[0], dr[0]), __dmul_rn(dr[1], dr[1])),
                                               __dmul_rn(dr[2], dr[2])));
-        if (d == 0.0 || d < dmin || d > dmax) return;
-        int lo, hi;
-        hist_window(a, d, lo, hi);
-        if (lo > hi) return;
-        // the slice points of the window
-        const int ta = lo <= sl.s0 ? 0 : (lo - sl.s0 + sl.sd - 1) / sl.sd;
-        const int tb = hi < sl.s0 ? -1 : min((hi - sl.s0) / sl.sd, sl.nt - 1);
-        if (ta > tb) return;
-        double den, dden;
-        if (!den_poly(a, dn, d, den, dden)) den_sums(a, d, inv_w, q1, den, dden);
-        const double inv_den = __drcp_rn(den);
+        if (d == 0.0 || d < dmin || d > dmax) return false;
+        // The slice points of the window, x - c <= d <= x + c.  The product with 1 / S, rounded
+        // outwards, is the first (last) of them, the point before it or, within its rounding of a
+        // point, the one before that: two steps inwards without branches.
+        ta = (int)floor(__dmul_rn(__dsub_rn(__dsub_rn(d, a.cutoff), x0), inv_S));
+        tb = (int)ceil(__dmul_rn(__dsub_rn(__dadd_rn(d, a.cutoff), x0), inv_S));
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            ta += d <= __dadd_rn(grid_x(a, sl.s0 + ta * sl.sd), a.cutoff) ? 0 : 1;
+            tb -= d >= __dsub_rn(grid_x(a, sl.s0 + tb * sl.sd), a.cutoff) ? 0 : 1;
+        }
+        ta = max(ta, 0);
+        tb = min(tb, sl.nt - 1);
+        if (ta > tb) return false;
+        double den;
+        if (!den_poly(a, dn, inv_step, d, den, dden)) den_sums(a, d, inv_w, q1, den, dden);
+        inv_den = __drcp_rn(den);
+        return true;
+    };
+    auto eval = [&](int j, bool on) {
+        double dr[3], d = 0.0, inv_den = 0.0, dden = 0.0;
+        int ta = 0, tb = -1;
+        on = on && pair_of(j, dr, d, ta, tb, inv_den, dden);
+        if constexpr (COOP) {
+            double2 g = make_double2(0.0, 1.0);
+            if (on) {
+                const double e0 = __dsub_rn(grid_x(a, sl.s0 + ta * sl.sd), d), c = __dmul_rn(pair_w, inv_den);
+                g.x = __dmul_rn(c, exp(-__dmul_rn(__dmul_rn(e0, e0), inv_w)));
+                g.y = exp(-__dmul_rn(__dmul_rn(__dmul_rn(2.0, e0), S), inv_w));
+                // a window of one point more than the lanes: both its ends on slice points
+                for (int t = ta + PTS; t <= tb; t++) {
+                    const double e = __dsub_rn(grid_x(a, sl.s0 + t * sl.sd), d);
+                    atomicAdd(sums + t, __dmul_rn(c, exp(-__dmul_rn(__dmul_rn(e, e), inv_w))));
+                }
+            }
+            s_g[warp][lane] = g;
+            s_t[warp][lane] = make_int2(ta, tb - ta + 1);
+            __syncwarp();
+            for (int p = 0; p < 32; p += NC) {
+                // NC pairs at a time, two a group of lanes, each into its own copy of the sums
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int q = p + h * (32 / PTS) + group;
+                    const double2 gp = s_g[warp][q];
+                    const int2 tp = s_t[warp][q];
+                    double r = gp.y, v = __dmul_rn(gp.x, Am);
+#pragma unroll
+                    for (int b = 1; b < PTS; b <<= 1) {
+                        v = __dmul_rn(v, m & b ? r : 1.0);
+                        r = __dmul_rn(r, r);
+                    }
+                    if (m < tp.y) {
+                        double *at = mine + (size_t)h * (32 / PTS) * sl.nt + tp.x + m;
+                        *at = __dadd_rn(*at, v);
+                    }
+                }
+                __syncwarp();
+            }
+            return;
+        }
+        if (!on) return;
+        const int ib = rdf_atom(a.sel2, atom0, j);
         Gauss G{0.0, 0.0};
         if (!GRAD) {
             const double c = __dmul_rn(pair_w, inv_den);
@@ -332,12 +417,12 @@ __global__ void __launch_bounds__(32 * kRlWarps) k_rdf_loss(RdfArgs a, RdfSlice 
             __syncwarp();
             if (nq >= 32) {
                 nq -= 32;
-                eval(s_q[warp][nq + lane]);
+                eval(s_q[warp][nq + lane], true);
                 __syncwarp();
             }
         }
     }
-    if (lane < nq) eval(s_q[warp][lane]);
+    if (nq > 0) eval(s_q[warp][min(lane, nq - 1)], lane < nq);
     if (GRAD) {
         __syncwarp();
 #pragma unroll
@@ -346,11 +431,19 @@ __global__ void __launch_bounds__(32 * kRlWarps) k_rdf_loss(RdfArgs a, RdfSlice 
             for (int o = 16; o > 0; o >>= 1) gi[u] += __shfl_xor_sync(0xffffffffu, gi[u], o);
             if (lane == 0 && live && gi[u] != 0.0) atomicAdd(a.dLdx + 3 * (size_t)ia + u, gi[u]);
         }
+    } else if (COOP) {
+        __syncthreads();
+        for (int t = threadIdx.x; t < sl.nt; t += blockDim.x) {
+            double v = 0.0;
+            for (int c = 0; c < NC * kRlWarps; c++) v += s_sum[(size_t)c * sl.nt + t];
+            if (v != 0.0) atomicAdd(sums + t, v);
+        }
     } else if (ncopy > 0) {
         __syncthreads();
         for (int t = threadIdx.x; t < sl.nt; t += blockDim.x) {
             double v = 0.0;
-            for (int c = 0; c < ncopy; c++) v += s_sum[(size_t)t * ncopy + c];
+            // (rotated: the threads of a warp read different banks)
+            for (int c = 0; c < ncopy; c++) v += s_sum[(size_t)t * ncopy + ((c + t) & (ncopy - 1))];
             if (v != 0.0) atomicAdd(sums + t, v);
         }
     }
@@ -460,14 +553,22 @@ cudaError_t launch_rdf_loss(const RdfArgs &a, const RdfSlice &sl, const RdfDen &
     const int tiles = ((a.sel1 == a.sel2 ? max_n1 / 2 + kRlWarps : max_n2) + kRlTile - 1) / kRlTile;
     int split = 1;
     while (split < tiles && (long long)groups * R * split < 2 * 148) split++;
-    int ncopy = 8;
-    while (ncopy > 0 && sizeof(double) * ncopy * (size_t)sl.nt > 32768) ncopy >>= 1;
+    // a lane per slice point of a pair's window where 16 or 32 cover it and the factors stay finite
+    const double points = 2.0 * a.cutoff / (sl.sd * a.step) * (1.0 - 1e-9);
+    const bool finite = 4.0 * a.cutoff * a.cutoff <= 300.0 * a.width;
+    const auto coop_smem = [&](int pts) { return sizeof(double) * (64 / pts) * kRlWarps * (size_t)sl.nt; };
+    const int pts = !finite ? 0 : points <= 16.0 && coop_smem(16) <= kRlSmem ? 16 : points <= 32.0 && coop_smem(32) <= kRlSmem ? 32 : 0;
+    int ncopy = 32;
+    while (ncopy > 0 && sizeof(double) * ncopy * (size_t)sl.nt > kRlSmem) ncopy >>= 1;
+    const auto value = pts == 16 ? k_rdf_loss<false, 16> : pts == 32 ? k_rdf_loss<false, 32> : k_rdf_loss<false, 0>;
+    const size_t smem = pts ? coop_smem(pts) : sizeof(double) * ncopy * (size_t)sl.nt;
     const dim3 grid(groups * split, R);
     cudaError_t e;
+    if ((e = cudaFuncSetAttribute(value, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRlSmem))) return e;
     if ((e = cudaMemsetAsync(sl.sum, 0, sizeof(double) * (size_t)R * sl.nt, st))) return e;
-    k_rdf_loss<false><<<grid, 32 * kRlWarps, sizeof(double) * ncopy * sl.nt, st>>>(a, sl, dn, split, ncopy);
+    value<<<grid, 32 * kRlWarps, smem, st>>>(a, sl, dn, split, ncopy);
     k_rdf_loss_finalize<<<R, 256, 0, st>>>(a, sl, pre, target, norm, weight, loss);
-    if (grad) k_rdf_loss<true><<<grid, 32 * kRlWarps, 0, st>>>(a, sl, dn, split, 0);
+    if (grad) k_rdf_loss<true, 0><<<grid, 32 * kRlWarps, 0, st>>>(a, sl, dn, split, 0);
     return cudaGetLastError();
 }
 

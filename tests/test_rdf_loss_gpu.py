@@ -78,3 +78,40 @@ def test_ragged_replicas():
         assert abs(l[r] - lo) <= 1e-11 * abs(lo)
         assert np.linalg.norm(gx[o:o + 3 * n] - go) <= 1e-11 * np.linalg.norm(go) + 1e-300
         o += 3 * n
+
+
+# the value kernel's forms: 16 or 32 lanes a pair, or a lane a pair -- too many points a window (41),
+# sums too many for 16 lanes' copies (300) and for 32 lanes' (600), factors too far apart
+FORMS = {
+    "16_of_300": (0.005, 0.005, 0.0005, 0.04, 300, 0, 1, 300),
+    "32_of_600": (0.003, 0.003, 0.0005, 0.04, 600, 0, 1, 600),
+    "steep": (0.005, 0.005, 0.00002, 0.04, 200, 0, 1, 200),
+}
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+def test_value_forms(form):
+    GRIDS[form] = FORMS[form]
+    _check(150, 2.6, (0, 0), form, 2)
+    _check(150, 2.6, (0, 1), form, 1)
+
+
+@pytest.mark.parametrize("step", [0.0625, 0.03125])
+def test_window_with_both_ends_on_points(step):
+    """A pair at a distance that is a grid point, with a cutoff of a whole number of steps (all exact
+    in binary): 17 (33) points in the window of 16 (32) steps."""
+    x = np.zeros((6, 3)) + 1.0
+    x[3:, 0] += 1.0
+    x[[1, 4], 1] += 0.0957
+    x[[2, 5], 2] += 0.0957
+    n = int(2.0 / step)
+    args = (0, 0, step, step, 0.05, 0.5, n, 0, 1, np.linspace(0.0, 1.0, n), 2, 1.0)
+    lo, go = orc.loss_grad(orc.make_system(2, 4.0), orc.Loss([orc.RdfTerm(*args)]), x)
+    e = Engine(2, 4.0)
+    e.set_params(C.default_params())
+    e.set_state(x, np.zeros_like(x))
+    e.set_loss([RdfTerm(*args)])
+    l, gx = e.loss_grad()
+    e.close()
+    assert abs(l[0] - lo) <= 1e-11 * abs(lo)
+    assert np.linalg.norm(gx - go) <= 1e-11 * np.linalg.norm(go) + 1e-300
