@@ -266,6 +266,7 @@ bool lane_overflow(revsim_sw_handle *h) {
 int build_list(revsim_sw_handle *h) {
     SwNlArgs a;
     a.N = h->N;
+    a.R = h->R;
     a.n_cells = h->n_cells;
     a.x = h->d_x;
     a.atom_rep = h->d_atom_rep;

@@ -48,7 +48,7 @@ struct SwConsts {
 };
 
 struct SwNlArgs {
-    int N, n_cells;
+    int N, R, n_cells;
     const double *x;
     const int *atom_rep, *rep_nc, *rep_cell_off, *rep_atom0, *rep_n;
     const double *rep_box;

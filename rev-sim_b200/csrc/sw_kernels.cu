@@ -11,98 +11,21 @@ namespace sw {
 
 namespace {
 
-// ------------------------------------------------------------------ duals
-// Forward-mode dual with K tangents (K = 0: a plain value).  Tangent 0 is the
-// position direction (w or S d), tangents 1..3 are a, gamma, sigma.  Every value
-// operation is the same rounding intrinsic whatever K is, so value parts are
-// bit-identical between the forward (K = 0) and reverse (K = 4) kernels.
-template <typename R, int K>
-struct SD {
-    R v;
-    R d[K > 0 ? K : 1];
-};
-
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> sdc(R v) {
-    SD<R, K> r;
-    r.v = v;
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = R(0);
-    return r;
-}
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> operator+(const SD<R, K> &a, const SD<R, K> &b) {
-    SD<R, K> r;
-    r.v = xadd(a.v, b.v);
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = xadd(a.d[k], b.d[k]);
-    return r;
-}
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> operator-(const SD<R, K> &a, const SD<R, K> &b) {
-    SD<R, K> r;
-    r.v = xsub(a.v, b.v);
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = xsub(a.d[k], b.d[k]);
-    return r;
-}
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> operator*(const SD<R, K> &a, const SD<R, K> &b) {
-    SD<R, K> r;
-    r.v = xmul(a.v, b.v);
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = xfma(a.d[k], b.v, xmul(a.v, b.d[k]));
-    return r;
-}
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> operator*(R a, const SD<R, K> &b) {
-    SD<R, K> r;
-    r.v = xmul(a, b.v);
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = xmul(a, b.d[k]);
-    return r;
-}
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> operator/(const SD<R, K> &a, const SD<R, K> &b) {
-    SD<R, K> r;
-    r.v = xdiv(a.v, b.v);
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = xdiv(xsub(a.d[k], xmul(r.v, b.d[k])), b.v);
-    return r;
-}
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> sd_exp(const SD<R, K> &a) {
-    SD<R, K> r;
-    r.v = xexp(a.v);
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = xmul(r.v, a.d[k]);
-    return r;
-}
 __device__ __forceinline__ float xrcp(float a) { return __frcp_rn(a); }
 __device__ __forceinline__ double xrcp(double a) { return __drcp_rn(a); }
 
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> sd_inv(const SD<R, K> &a) {
-    SD<R, K> r;
-    r.v = xrcp(a.v);
-    const R m = -xmul(r.v, r.v);
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = xmul(m, a.d[k]);
-    return r;
-}
-template <typename R, int K>
-__device__ __forceinline__ SD<R, K> sd_neg(const SD<R, K> &a) {
-    SD<R, K> r;
-    r.v = -a.v;
-#pragma unroll
-    for (int k = 0; k < K; k++) r.d[k] = -a.d[k];
-    return r;
-}
-
 __device__ __forceinline__ double dist2(const double *xa, const double *xb, double L, double d[3]) {
-    d[0] = vec1d(xa[0], xb[0], L);
-    d[1] = vec1d(xa[1], xb[1], L);
-    d[2] = vec1d(xa[2], xb[2], L);
+    // (vec1d's first value, c2 - c1, is its result for all that lies well within half a box)
+    bool near = true;
+#pragma unroll
+    for (int u = 0; u < 3; u++) {
+        d[u] = __dsub_rn(xb[u], xa[u]);
+        near = near && fabs(d[u]) < 0.49 * L;
+    }
+    if (!near) {
+#pragma unroll
+        for (int u = 0; u < 3; u++) d[u] = vec1d(xa[u], xb[u], L);
+    }
     return __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
 }
 
@@ -152,28 +75,48 @@ __global__ void k_cell_count(SwNlArgs a) {
     atomicAdd(a.cell_cnt + cell, 1);
 }
 
-__global__ void k_cell_scan(SwNlArgs a) {
-    __shared__ int s_part[1024];
-    __shared__ int s_carry;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    for (int base = 0; base < a.n_cells; base += blockDim.x) {
-        const int i = base + threadIdx.x;
-        const int v = i < a.n_cells ? a.cell_cnt[i] : 0;
-        s_part[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < blockDim.x; off <<= 1) {
-            const int t = threadIdx.x >= off ? s_part[threadIdx.x - off] : 0;
-            __syncthreads();
-            s_part[threadIdx.x] += t;
-            __syncthreads();
+// Exclusive scan of the cell counts, one CTA per replica (its cells hold its atoms, so its scan
+// starts at its first atom): every pass takes two consecutive cells a thread, a shuffle scan a warp
+// and one scan of the warps' sums.  16 replicas of 1,728 cells: under 4 us; 40 us in one CTA with
+// one cell a thread and a barrier per doubling.
+__global__ void __launch_bounds__(1024) k_cell_scan(SwNlArgs a) {
+    constexpr int PER = 2;
+    const int r = blockIdx.x, nc = a.rep_nc[r], first = a.rep_cell_off[r], end = first + nc * nc * nc;
+    __shared__ int s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = a.rep_atom0[r];
+    for (int base = first; base < end; base += 1024 * PER) {
+        const int c0 = base + threadIdx.x * PER;
+        int v[PER], sum = 0;
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            v[k] = c0 + k < end ? a.cell_cnt[c0 + k] : 0;
+            sum += v[k];
         }
-        if (i < a.n_cells) {
-            a.cell_start[i] = s_carry + s_part[threadIdx.x] - v;
-            a.cell_fill[i] = 0;
+        int inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int q = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += q;
         }
+        if (lane == 31) s_warp[warp] = inc;
         __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) s_carry += s_part[threadIdx.x];
+        const int wsum = s_warp[lane];
+        int winc = wsum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int q = __shfl_up_sync(0xffffffffu, winc, o);
+            if (lane >= o) winc += q;
+        }
+        int run = carry + inc - sum + __shfl_sync(0xffffffffu, winc - wsum, warp);
+        carry += __shfl_sync(0xffffffffu, winc, 31);
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (c0 + k < end) {
+                a.cell_start[c0 + k] = run;
+                a.cell_fill[c0 + k] = 0;
+                run += v[k];
+            }
         __syncthreads();
     }
 }
@@ -259,11 +202,16 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS) k_rows(SwNlArgs a) {
 //   alpha_q = dh_q/ds / sigma,  beta_q = 2 h_q / r_q,
 // so T_q = u_q (eps A g2_q / 2 + eps lambda S1) + eps lambda beta_q V with
 // S1 = sum h_q' c3 (c3 alpha_q - cos beta_q), V = sum h_q' c3 u_q'.
+//
+// Bound by instruction issue (65 %; half of a group's lanes hold a slot).  16 x 8,000 atoms, FP32
+// terms, learned pair term, 16 lanes a centre: 140 us with tangents and contraction, 65 us values
+// only.  202 and 74 us with four tangents carried through dual numbers (94 registers, 20 warps an
+// SM) and vec1d's comparisons on every candidate; at 64 registers, some spilled, 32 warps fit (154 ->
+// 149 us).
 template <typename R, int G, int MODE>
-__global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R> p) {
-    constexpr int K = MODE == TM_VALUE ? 0 : 4;
+__global__ void __launch_bounds__(TERM_THREADS, sizeof(R) == 4 && MODE != TM_VALUE ? 8 : 0) k_terms(SwTermArgs t, SwConsts<R> p) {
+    constexpr bool TAN = MODE != TM_VALUE;
     constexpr int GPB = TERM_THREADS / G;
-    using D = SD<R, K>;
     __shared__ double s_d[GPB][G][3];
     __shared__ R s_dd[GPB][G][3];
     __shared__ int s_j[GPB][G];
@@ -272,9 +220,9 @@ __global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R
     // and the 3-body radial factor h with its tangents
     using V4 = typename V4T<R>::T;
     __shared__ V4 s_uh[GPB][G];
-    __shared__ V4 s_ut[GPB][K > 0 ? G : 1];
+    __shared__ V4 s_ut[GPB][TAN ? G : 1];
     chain_enter();
-    __shared__ V4 s_ht[GPB][K > 0 ? G : 1];
+    __shared__ V4 s_ht[GPB][TAN ? G : 1];
     __shared__ double s_red[TERM_THREADS / 32][9];
 
     const int lane = threadIdx.x % G, grp = threadIdx.x / G;
@@ -356,64 +304,92 @@ __global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R
 
     // Phase 2: per-slot quantities (u = d / r, h = exp(gamma / t), alpha = dh/ds / sigma,
     // beta = 2 h / r with s = r / sigma, t = s - a; t from an FP64 difference to keep its
-    // digits near the cutoff).  Divisions are reciprocals.
+    // digits near the cutoff).  Divisions are reciprocals.  Tangents 0 (the position direction), 1
+    // (a), 2 (gamma) and 3 (sigma) follow from those of s (0: r' / sigma, 3: -s / sigma) and t
+    // (those, and 1: -1), in closed form: most of a dual number's tangents would be zeros here.
     const bool own = lane < n;
-    D u[3], alpha = sdc<R, K>(R(0)), beta = sdc<R, K>(R(0)), sD = sdc<R, K>(R(1)),
-            itD = sdc<R, K>(R(0)), it2 = sdc<R, K>(R(0)), g2 = sdc<R, K>(R(0));
-    R gB = R(0);
-    D gm = sdc<R, K>(R(0));   // learned term: u'(r) / 2, the slot's half of the pair
+    R u[3] = {R(0), R(0), R(0)}, alpha = R(0), beta = R(0), g2 = R(0), gB = R(0);
+    R gm = R(0);              // learned term: u'(r) / 2, the slot's half of the pair
     int mg = -1;              // its interval (-1: off) and position in it
     R msv = R(0);
+    R u0[3] = {R(0), R(0), R(0)}, al[4], be[4], g2t[4], gm0 = R(0);   // tangents
+    R z[3] = {R(0), R(0), R(0)};   // the contraction's weights of this slot
+    if (TAN) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) u[k] = sdc<R, K>(R(0));
-    D gam = sdc<R, K>(p.gam), isig = sdc<R, K>(p.isig);
-    if constexpr (K > 0) {
-        gam.d[2] = R(1);
-        isig.d[3] = -xmul(p.isig, p.isig);
+        for (int k = 0; k < 4; k++) al[k] = be[k] = g2t[k] = R(0);
     }
     if (own) {
         double d64[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) d64[k] = s_d[grp][lane][k];
-        t.act_idx[(size_t)c * G + lane] = s_j[grp][lane];
+        const int j = s_j[grp][lane];
+        t.act_idx[(size_t)c * G + lane] = j;
+        if (MODE == TM_REV && t.part) {
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                z[k] = (R)__dsub_rn(__dmul_rn(t.A[3 * (size_t)j + k], t.acoef_scale), ac[k]);
+        } else if (MODE == TM_LOSS && t.part) {
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                z[k] = (R)__dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(S[3 * k], d64[0]), __dmul_rn(S[3 * k + 1], d64[1])),
+                                              __dmul_rn(S[3 * k + 2], d64[2])),
+                                    invV);
+        }
         const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(d64[0], d64[0]), __dmul_rn(d64[1], d64[1])),
                                     __dmul_rn(d64[2], d64[2]));
         const R r = xsqrt((R)r2), ir = xrcp(r);
-        R rdot = R(0);
 #pragma unroll
-        for (int k = 0; k < 3; k++) u[k].v = xmul((R)d64[k], ir);
-        sD.v = xmul(r, p.isig);
+        for (int k = 0; k < 3; k++) u[k] = xmul((R)d64[k], ir);
+        const R sv = xmul(r, p.isig);
         // t = s - a = (r^2 - (a sigma)^2) / (sigma (r + a sigma)), the difference in FP64
-        D tD = sdc<R, K>(xmul((R)__dsub_rn(r2, p.lim2), xrcp(xmul(p.sig, xadd(r, p.asig)))));
-        D irD = sdc<R, K>(ir);
-        if constexpr (K > 0) {
-            // position tangent: r' = u . d'; u' = (d' - u r') / r; s' = r' / sigma;
-            // parameter tangents: dt/da = -1, ds/dsigma = dt/dsigma = -s / sigma
+        const R tv = xmul((R)__dsub_rn(r2, p.lim2), xrcp(xmul(p.sig, xadd(r, p.asig))));
+        const R it = xrcp(tv), it2 = xmul(it, it);
+        const R h = xexp(xmul(p.gam, it));
+        alpha = -xmul(xmul(xmul(p.gam, h), it2), p.isig);
+        beta = xmul(R(2), xmul(h, ir));
+        // 2-body: dE2/dr / (eps A) = e^{1/t} (-4 B s^-5 - (B s^-4 - 1) / t^2) / sigma
+        // (diamond.jl:453), and its B derivative.
+        const R e1 = xexp(it);
+        const R is = xrcp(sv);
+        const R is2 = xmul(is, is), is4 = xmul(is2, is2), is5 = xmul(is4, is);
+        const R B4 = xsub(xmul(p.B, is4), R(1));   // B s^-4 - 1
+        const R gv = xadd(xmul(xmul(R(4), p.B), is5), xmul(B4, it2));
+        g2 = xmul(xmul(e1, -gv), p.isig);
+        gB = xmul(xmul(e1, -xadd(xmul(R(4), is5), xmul(is4, it2))), p.isig);
+        R rdot = R(0), h0 = R(0), hp[3] = {R(0), R(0), R(0)};
+        if constexpr (TAN) {
+            // r' = u . d'; u' = (d' - u r') / r
             R dd[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) dd[k] = s_dd[grp][lane][k];
-            rdot = xfma(u[0].v, dd[0], xfma(u[1].v, dd[1], xmul(u[2].v, dd[2])));
+            rdot = xfma(u[0], dd[0], xfma(u[1], dd[1], xmul(u[2], dd[2])));
 #pragma unroll
-            for (int k = 0; k < 3; k++) u[k].d[0] = xmul(xsub(dd[k], xmul(u[k].v, rdot)), ir);
-            sD.d[0] = xmul(rdot, p.isig);
-            sD.d[3] = -xmul(sD.v, p.isig);
-            tD.d[0] = sD.d[0];
-            tD.d[1] = R(-1);
-            tD.d[3] = sD.d[3];
-            irD.d[0] = -xmul(rdot, xmul(ir, ir));
+            for (int k = 0; k < 3; k++) u0[k] = xmul(xsub(dd[k], xmul(u[k], rdot)), ir);
+            const R s0 = xmul(rdot, p.isig), s3 = -xmul(sv, p.isig);
+            const R it0 = -xmul(it2, s0), it3 = -xmul(it2, s3);   // of 1/t; it2 for a, 0 for gamma
+            const R gh = xmul(p.gam, h);
+            h0 = xmul(gh, it0);
+            hp[0] = xmul(gh, it2);
+            hp[1] = xmul(h, it);
+            hp[2] = xmul(gh, it3);
+            const R A0 = xmul(xmul(p.gam, it2), p.isig), c1 = xmul(xmul(R(2), gh), xmul(p.isig, it));
+            al[0] = -xfma(h0, A0, xmul(c1, it0));
+            al[1] = -xfma(hp[0], A0, xmul(c1, it2));
+            al[2] = -xfma(hp[1], A0, xmul(xmul(h, it2), p.isig));
+            al[3] = -xfma(hp[2], A0, xfma(c1, it3, xmul(alpha, p.isig)));
+            const R b2 = xadd(ir, ir);
+            be[0] = xmul(b2, xfma(-xmul(h, rdot), ir, h0));
+            be[1] = xmul(b2, hp[0]);
+            be[2] = xmul(b2, hp[1]);
+            be[3] = xmul(b2, hp[2]);
+            // d(gv) = gs ds + 2 (B s^-4 - 1) (1/t) d(1/t), d(e^{1/t}) = e^{1/t} d(1/t)
+            const R is3 = xmul(is2, is);
+            const R gs = -xmul(xmul(R(4), p.B), xmul(is2, xfma(R(5), is4, xmul(is3, it2))));
+            const R H = xfma(xmul(R(2), B4), it, gv), E = -xmul(e1, p.isig);
+            g2t[0] = xmul(E, xfma(it0, H, xmul(gs, s0)));
+            g2t[1] = xmul(E, xmul(it2, H));
+            g2t[3] = xsub(xmul(E, xfma(it3, H, xmul(gs, s3))), xmul(g2, p.isig));
         }
-        itD = sd_inv(tD);
-        it2 = itD * itD;
-        const D h = sd_exp(gam * itD);
-        alpha = sd_neg(((gam * h) * it2) * isig);
-        beta = R(2) * (h * irD);
-        // 2-body: dE2/dr / (eps A) = e^{1/t} (-4 B s^-5 - (B s^-4 - 1) / t^2) / sigma
-        // (diamond.jl:453), and its B derivative.
-        const D e1 = sd_exp(itD);
-        const D is = sd_inv(sD);
-        const D is2 = is * is, is4 = is2 * is2, is5 = is4 * is;
-        g2 = (e1 * sd_neg((R(4) * p.B) * is5 + ((p.B * is4) - sdc<R, K>(R(1))) * it2)) * isig;
-        gB = xmul(xmul(e1.v, -xadd(xmul(R(4), is5.v), xmul(is4.v, it2.v))), p.isig);
         if (t.mlp_tab && r2 < p.mlp_rc2) {
             // u'/2 = (c1 + s (2 c2 + 3 s c3)) NG / (2 rc) on the cubic segment of interval
             // g, s = r NG / rc - g; its position tangent u''/2 r' = (c2 + 3 s c3) (NG/rc)^2 r'
@@ -422,24 +398,24 @@ __global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R
             msv = xsub(q, (R)mg);
             const V4 cc = reinterpret_cast<const V4 *>(t.mlp_tab)[mg];
             const R s3 = xmul(R(3), msv);
-            gm.v = xmul(xfma(msv, xfma(s3, cc.w, xmul(R(2), cc.z)), cc.y), p.mlp_hhalf);
-            if constexpr (K > 0) gm.d[0] = xmul(xmul(xfma(s3, cc.w, cc.z), p.mlp_hinv2), rdot);
+            gm = xmul(xfma(msv, xfma(s3, cc.w, xmul(R(2), cc.z)), cc.y), p.mlp_hhalf);
+            if (TAN) gm0 = xmul(xmul(xfma(s3, cc.w, cc.z), p.mlp_hinv2), rdot);
         }
         V4 uh;
-        uh.x = u[0].v;
-        uh.y = u[1].v;
-        uh.z = u[2].v;
-        uh.w = h.v;
+        uh.x = u[0];
+        uh.y = u[1];
+        uh.z = u[2];
+        uh.w = h;
         s_uh[grp][lane] = uh;
-        if constexpr (K > 0) {
+        if constexpr (TAN) {
             V4 ut, ht;
-            ut.x = u[0].d[0];
-            ut.y = u[1].d[0];
-            ut.z = u[2].d[0];
-            ut.w = h.d[0];
-            ht.x = h.d[1];
-            ht.y = h.d[2];
-            ht.z = h.d[3];
+            ut.x = u0[0];
+            ut.y = u0[1];
+            ut.z = u0[2];
+            ut.w = h0;
+            ht.x = hp[0];
+            ht.y = hp[1];
+            ht.z = hp[2];
             ht.w = R(0);
             s_ut[grp][lane] = ut;
             s_ht[grp][lane] = ht;
@@ -448,18 +424,17 @@ __global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R
     __syncwarp(gmask);
 
     // Phase 3: 3-body sums over the other slots.  The value arithmetic is the same
-    // sequence of rounded operations for every K; the tangents use that u and cos
-    // depend on the position direction only (tangent 0), not on the parameters.
-    D S1 = sdc<R, K>(R(0)), V[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) V[k] = sdc<R, K>(R(0));
+    // sequence of rounded operations in every mode.  With w = h' c3 and X = c3 alpha - cos beta
+    // the tangents of S1 = sum w X and V = sum w u' need, besides the position direction's,
+    // only sums that the parameters share: P = sum w c3 and Q = sum w cos multiply the slot's
+    // own alpha', beta'; the neighbours' h' enter the contraction z . T' through
+    // Y_m = sum h'_m c3 (zu X + beta z . u'), zu = z . u.
+    R S1 = R(0), V[3] = {R(0), R(0), R(0)};
+    R S10 = R(0), V0[3] = {R(0), R(0), R(0)}, P = R(0), Q = R(0), Y[3] = {R(0), R(0), R(0)};
+    const R zu = TAN ? xfma(z[2], u[2], xfma(z[1], u[1], xmul(z[0], u[0]))) : R(0);
     if (own) {
         const R third = R(1) / R(3);
-        R ud[3] = {R(0), R(0), R(0)};
-        if constexpr (K > 0) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) ud[k] = u[k].d[0];
-        }
+        R Rc = R(0);   // sum w cos'
         for (int q2 = 0; q2 < n; q2++) {
             // the slot itself enters with weight 0 (its terms are finite), which keeps the
             // lanes of a group on one path
@@ -467,61 +442,62 @@ __global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R
             const V4 uh2 = s_uh[grp][q2];
             const R u2[3] = {uh2.x, uh2.y, uh2.z};
             const R h2 = xmul(uh2.w, one);
-            const R cs = xadd(xadd(xmul(u[0].v, u2[0]), xmul(u[1].v, u2[1])), xmul(u[2].v, u2[2]));
+            const R cs = xadd(xadd(xmul(u[0], u2[0]), xmul(u[1], u2[1])), xmul(u[2], u2[2]));
             const R c3 = xadd(cs, third);
             const R w = xmul(h2, c3);
-            const R X = xsub(xmul(c3, alpha.v), xmul(cs, beta.v));
-            S1.v = xadd(S1.v, xmul(w, X));
+            const R X = xsub(xmul(c3, alpha), xmul(cs, beta));
+            S1 = xadd(S1, xmul(w, X));
 #pragma unroll
-            for (int k = 0; k < 3; k++) V[k].v = xadd(V[k].v, xmul(w, u2[k]));
-            if constexpr (K > 0) {
+            for (int k = 0; k < 3; k++) V[k] = xadd(V[k], xmul(w, u2[k]));
+            if constexpr (TAN) {
                 const V4 ut2 = s_ut[grp][q2], ht2 = s_ht[grp][q2];
-                const R u2d[3] = {ut2.x, ut2.y, ut2.z};
-                const R h2d[4] = {ut2.w, ht2.x, ht2.y, ht2.z};
-                const R csd = xfma(ud[0], u2[0], xfma(u[0].v, u2d[0], xfma(ud[1], u2[1], xfma(u[1].v, u2d[1],
-                                   xfma(ud[2], u2[2], xmul(u[2].v, u2d[2]))))));
-                R wd[K], Xd[K];
-                wd[0] = xfma(xmul(h2d[0], one), c3, xmul(h2, csd));
-                Xd[0] = xsub(xfma(csd, alpha.v, xmul(c3, alpha.d[0])), xfma(csd, beta.v, xmul(cs, beta.d[0])));
+                const R u20[3] = {ut2.x, ut2.y, ut2.z};
+                const R cs0 = xfma(u0[0], u2[0], xfma(u[0], u20[0], xfma(u0[1], u2[1], xfma(u[1], u20[1],
+                                   xfma(u0[2], u2[2], xmul(u[2], u20[2]))))));
+                const R c31 = xmul(c3, one);
+                const R w0 = xfma(ut2.w, c31, xmul(h2, cs0));
+                S10 = xfma(w0, X, S10);
+                Rc = xfma(w, cs0, Rc);
+                P = xfma(w, c3, P);
+                Q = xfma(w, cs, Q);
 #pragma unroll
-                for (int kk = 1; kk < K; kk++) {
-                    wd[kk] = xmul(xmul(h2d[kk], one), c3);
-                    Xd[kk] = xsub(xmul(c3, alpha.d[kk]), xmul(cs, beta.d[kk]));
-                }
-#pragma unroll
-                for (int kk = 0; kk < K; kk++) S1.d[kk] = xfma(wd[kk], X, xfma(w, Xd[kk], S1.d[kk]));
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    V[k].d[0] = xfma(wd[0], u2[k], xfma(w, u2d[k], V[k].d[0]));
-#pragma unroll
-                    for (int kk = 1; kk < K; kk++) V[k].d[kk] = xfma(wd[kk], u2[k], V[k].d[kk]);
-                }
+                for (int k = 0; k < 3; k++) V0[k] = xfma(w0, u2[k], xfma(w, u20[k], V0[k]));
+                const R zu2 = xfma(z[2], u2[2], xfma(z[1], u2[1], xmul(z[0], u2[0])));
+                const R y = xmul(c31, xfma(zu, X, xmul(beta, zu2)));
+                Y[0] = xfma(ht2.x, y, Y[0]);
+                Y[1] = xfma(ht2.y, y, Y[1]);
+                Y[2] = xfma(ht2.z, y, Y[2]);
             }
         }
+        if (TAN) S10 = xadd(xfma(xsub(alpha, beta), Rc, S10), xfma(al[0], P, -xmul(be[0], Q)));
     }
     double d64[3] = {0.0, 0.0, 0.0};
     if (own) {
 #pragma unroll
         for (int k = 0; k < 3; k++) d64[k] = s_d[grp][lane][k];
     }
-    D T[3];
-    const D coef = (p.half_eA * g2 + p.el * S1) + gm;
-    const D elb = p.el * beta;
+    R T[3];
+    const R coef = xadd(xadd(xmul(p.half_eA, g2), xmul(p.el, S1)), gm);
+    const R elb = xmul(p.el, beta);
 #pragma unroll
-    for (int k = 0; k < 3; k++) T[k] = u[k] * coef + elb * V[k];
+    for (int k = 0; k < 3; k++) T[k] = xadd(xmul(u[k], coef), xmul(elb, V[k]));
     if (own) {
-        using V4 = typename V4T<R>::T;
         V4 tv;
-        tv.x = T[0].v;
-        tv.y = T[1].v;
-        tv.z = T[2].v;
+        tv.x = T[0];
+        tv.y = T[1];
+        tv.z = T[2];
         tv.w = R(0);
         reinterpret_cast<V4 *>(t.Tv)[(size_t)c * G + lane] = tv;
-        if constexpr (K > 0) {
+        if constexpr (TAN) {
+            const R coef0 = xadd(xfma(p.half_eA, g2t[0], xmul(p.el, S10)), gm0), elb0 = xmul(p.el, be[0]);
+            R T0[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                T0[k] = xfma(u0[k], coef, xfma(u[k], coef0, xfma(elb0, V[k], xmul(elb, V0[k]))));
             V4 tt;
-            tt.x = T[0].d[0];
-            tt.y = T[1].d[0];
-            tt.z = T[2].d[0];
+            tt.x = T0[0];
+            tt.y = T0[1];
+            tt.z = T0[2];
             tt.w = R(0);
             reinterpret_cast<V4 *>(t.Tt)[(size_t)c * G + lane] = tt;
         }
@@ -529,34 +505,20 @@ __global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R
 
     // Parameter contraction sum_q z_q . dT_q/dtheta (theta order A, B, a, lambda, gamma,
     // sigma, eps); the linear parameters from the value parts.
-    if constexpr (MODE != TM_VALUE) {
+    if constexpr (TAN) {
       if (t.part) {
         double con[NP] = {0, 0, 0, 0, 0, 0, 0};
         if (own) {
-            R z[3];
-            const int j = s_j[grp][lane];
-            if (MODE == TM_REV) {
+            const R zV = xfma(z[2], V[2], xfma(z[1], V[1], xmul(z[0], V[0])));
+            const R zT3 = xfma(zu, S1, xmul(beta, zV));
+            R zd[3];
 #pragma unroll
-                for (int k = 0; k < 3; k++)
-                    z[k] = (R)__dsub_rn(__dmul_rn(t.A[3 * (size_t)j + k], t.acoef_scale), ac[k]);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    z[k] = (R)__dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(S[3 * k], d64[0]),
-                                                            __dmul_rn(S[3 * k + 1], d64[1])),
-                                                  __dmul_rn(S[3 * k + 2], d64[2])),
-                                        invV);
-            }
-            R zu = R(0), zT3 = R(0), zd[3] = {R(0), R(0), R(0)};
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                zu = xfma(z[k], u[k].v, zu);
-                zT3 = xfma(z[k], xfma(u[k].v, S1.v, xmul(beta.v, V[k].v)), zT3);
-#pragma unroll
-                for (int m = 0; m < 3; m++) zd[m] = xfma(z[k], T[k].d[1 + m], zd[m]);
+            for (int m = 0; m < 3; m++) {
+                const R s1 = xsub(xmul(al[1 + m], P), xmul(be[1 + m], Q));
+                zd[m] = xfma(xmul(p.half_eA, g2t[1 + m]), zu, xmul(p.el, xadd(Y[m], xfma(zu, s1, xmul(be[1 + m], zV)))));
             }
             const double sgn = MODE == TM_REV ? -1.0 : 1.0;
-            const double half_g2zu = 0.5 * (double)g2.v * (double)zu;
+            const double half_g2zu = 0.5 * (double)g2 * (double)zu;
             con[0] = sgn * (double)p.eps * half_g2zu;
             con[1] = sgn * (double)p.half_eA * (double)gB * (double)zu;
             con[2] = sgn * (double)zd[0];
@@ -582,7 +544,7 @@ __global__ void __launch_bounds__(TERM_THREADS) k_terms(SwTermArgs t, SwConsts<R
 #pragma unroll
         for (int a = 0; a < 3; a++)
 #pragma unroll
-            for (int bb = 0; bb < 3; bb++) w9[3 * a + bb] = own ? __dmul_rn((double)T[a].v, d64[bb]) : 0.0;
+            for (int bb = 0; bb < 3; bb++) w9[3 * a + bb] = own ? __dmul_rn((double)T[a], d64[bb]) : 0.0;
         cta_sum<9>(s_red, w9, t.wpart + (size_t)b * 9, false);
     }
 }
@@ -904,7 +866,7 @@ cudaError_t launch_sw_nlist(const SwNlArgs &a, cudaStream_t st) {
     cudaError_t e;
     if ((e = cudaMemsetAsync(a.cell_cnt, 0, sizeof(int) * a.n_cells, st))) return e;
     k_cell_count<<<nblk(a.N, 256), 256, 0, st>>>(a);
-    k_cell_scan<<<1, 1024, 0, st>>>(a);
+    k_cell_scan<<<a.R, 1024, 0, st>>>(a);
     k_cell_fill<<<nblk(a.N, 256), 256, 0, st>>>(a);
     k_rows<<<nblk(a.N, ROWS_WARPS), 32 * ROWS_WARPS, 0, st>>>(a);
     return cudaGetLastError();
