@@ -205,15 +205,17 @@ __global__ void k_rdf(RdfArgs a) {
 // terms of the experimental grid (4,801 points, of which the loss reads 248 and 281; 27 a window)
 // on the 895-water box, and the 200-bin O-O term (16 a window) on the 3,000-water box: every
 // ordered pair over the whole grid, as k_rdf does, 567 / 535 and 215 / 298; a lane per pair with
-// atomics on eight copies and divisions 63 / 44 and 67 / 76; now 41 / 38 and 54 / 44.
+// atomics on eight copies and divisions 63 / 44 and 67 / 76; now 41 / 28 and 54 / 44 (the gradient by
+// sums 52 where a window has 16 points, per point 38 where it has 27).
 constexpr int kRlWarps = 8, kRlTile = 256;
 constexpr size_t kRlSmem = 65536;   // dynamic shared memory of a value CTA at most
 
 template <bool GRAD, int PTS>
-__global__ void __launch_bounds__(32 * kRlWarps, PTS == 16 ? 3 : 0) k_rdf_loss(RdfArgs a, RdfSlice sl, RdfDen dn, int split,
+__global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_rdf_loss(RdfArgs a, RdfSlice sl, RdfDen dn, int split,
                                                             int ncopy) {
-    constexpr bool COOP = PTS > 0;
-    constexpr int NC = COOP ? 64 / PTS : 0;   // pairs deposited at a time, copies of the sums a warp
+    constexpr bool COOP = !GRAD && PTS > 0;
+    constexpr int W = PTS ? PTS : 32;   // lanes a pair
+    constexpr int NC = COOP ? 64 / W : 0;   // pairs deposited at a time, copies of the sums a warp
     // GRAD false: [nt][ncopy] partial sums (ncopy 0: none; COOP: [warps][NC][nt])
     extern __shared__ double s_sum[];
     __shared__ double2 s_g[COOP ? kRlWarps : 1][COOP ? 32 : 1];   // a pair's first point and ratio
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(32 * kRlWarps, PTS == 16 ? 3 : 0) k_rdf_loss(R
 
     // COOP: lane m of PTS deposits point m of a pair, exp(-(e0 + m S)^2 / w) = exp(-e0^2 / w) r^m A_m
     // with r = exp(-2 e0 S / w)
-    const int m = COOP ? lane % PTS : 0, group = COOP ? lane / PTS : 0;
+    const int m = COOP ? lane % W : 0, group = COOP ? lane / W : 0;
     const double Am = COOP ? exp(-__dmul_rn(__dmul_rn((double)m * S, (double)m * S), inv_w)) : 0.0;
     double *mine = s_sum + (COOP ? ((size_t)warp * NC + group) * sl.nt : 0);
 
@@ -359,14 +361,35 @@ __global__ void __launch_bounds__(32 * kRlWarps, PTS == 16 ? 3 : 0) k_rdf_loss(R
                 gauss_next(G, qS);
             }
         } else {
-            const double dd2 = __dmul_rn(dden, __dmul_rn(inv_den, inv_den));
+            // dL/dd = sum_t wt (g' / den - g den' / den^2)
             double dLdd = 0.0;
-            for (int t = ta; t <= tb; t++) {
-                if (!sl.recur || ((t - ta) % kGaussAnchor) == 0) gauss_anchor(a, d, sl.s0 + t * sl.sd, S, inv_w, G);
-                const double e = __dsub_rn(grid_x(a, sl.s0 + t * sl.sd), d);
-                const double gp = __dmul_rn(__dmul_rn(__dmul_rn(G.g, 2.0), e), inv_w);
-                dLdd = __fma_rn(wt[t], __dsub_rn(__dmul_rn(gp, inv_den), __dmul_rn(G.g, dd2)), dLdd);
-                gauss_next(G, qS);
+            if constexpr (PTS == 16) {
+                const double dd2 = __dmul_rn(dden, __dmul_rn(inv_den, inv_den));
+                for (int t = ta; t <= tb; t++) {
+                    if (!sl.recur || ((t - ta) % kGaussAnchor) == 0) gauss_anchor(a, d, sl.s0 + t * sl.sd, S, inv_w, G);
+                    const double e = __dsub_rn(grid_x(a, sl.s0 + t * sl.sd), d);
+                    const double gp = __dmul_rn(__dmul_rn(__dmul_rn(G.g, 2.0), e), inv_w);
+                    dLdd = __fma_rn(wt[t], __dsub_rn(__dmul_rn(gp, inv_den), __dmul_rn(G.g, dd2)), dLdd);
+                    gauss_next(G, qS);
+                }
+            } else {
+                // the same from the sums of wt g and wt g e, g' = 2 e g / w: half the instructions a point, at
+                // 113 registers (two CTAs an SM; the other form's 80 hold three)
+                double s0 = 0.0, s1 = 0.0;
+                const double e0 = __dsub_rn(grid_x(a, sl.s0 + ta * sl.sd), d);
+                const int run = sl.recur ? kGaussAnchor : 1;
+                for (int t = ta; t <= tb; t += run) {
+                    gauss_anchor(a, d, sl.s0 + t * sl.sd, S, inv_w, G);
+                    const int t1 = min(t + run - 1, tb);
+                    for (int q = t; q <= t1; q++) {
+                        const double p = __dmul_rn(wt[q], G.g);
+                        s0 = __dadd_rn(s0, p);
+                        s1 = __fma_rn(p, __fma_rn((double)(q - ta), S, e0), s1);
+                        gauss_next(G, qS);
+                    }
+                }
+                dLdd = __dsub_rn(__dmul_rn(__dmul_rn(__dmul_rn(2.0, inv_w), s1), inv_den),
+                                 __dmul_rn(__dmul_rn(s0, dden), __dmul_rn(inv_den, inv_den)));
             }
             if (dLdd != 0.0) {
                 const double s = __ddiv_rn(__dmul_rn(pair_w, dLdd), d);
@@ -568,7 +591,12 @@ cudaError_t launch_rdf_loss(const RdfArgs &a, const RdfSlice &sl, const RdfDen &
     if ((e = cudaMemsetAsync(sl.sum, 0, sizeof(double) * (size_t)R * sl.nt, st))) return e;
     value<<<grid, 32 * kRlWarps, smem, st>>>(a, sl, dn, split, ncopy);
     k_rdf_loss_finalize<<<R, 256, 0, st>>>(a, sl, pre, target, norm, weight, loss);
-    if (grad) k_rdf_loss<true, 0><<<grid, 32 * kRlWarps, 0, st>>>(a, sl, dn, split, 0);
+    if (grad) {
+        if (pts == 16)
+            k_rdf_loss<true, 16><<<grid, 32 * kRlWarps, 0, st>>>(a, sl, dn, split, 0);
+        else
+            k_rdf_loss<true, 32><<<grid, 32 * kRlWarps, 0, st>>>(a, sl, dn, split, 0);
+    }
     return cudaGetLastError();
 }
 
