@@ -1,6 +1,6 @@
 // rs_pack.cuh -- two neighbour entries per lane in one register pair (sm_100a).
 //
-// The FP32 step kernels evaluate the pair terms of two neighbour-row entries at once: the .x
+// The half-shell FP32 kernels evaluate the pair terms of two neighbour-row entries at once: the .x
 // half of every value belongs to one entry, the .y half to the other.  Products, sums and
 // fused multiply-adds are the packed sm_100 instructions (__fadd2_rn, __fmul2_rn, __ffma2_rn:
 // one instruction for both halves, each half rounded exactly as __fadd_rn, __fmul_rn,
