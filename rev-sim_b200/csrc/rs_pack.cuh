@@ -16,10 +16,8 @@ namespace rs {
 
 template <typename R> struct PkT;
 template <> struct PkT<float> { using T = float2; };
-template <> struct PkT<double> { using T = double2; };
 
 __device__ __forceinline__ float2 pk(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ double2 pk(double a, double b) { return make_double2(a, b); }
 __device__ __forceinline__ float2 pk1(float a) { return make_float2(a, a); }
 __device__ __forceinline__ double2 pk1(double a) { return make_double2(a, a); }
 
@@ -33,21 +31,5 @@ __device__ __forceinline__ float2 xsub(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 xneg(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 xrsqrt(float2 a) { return make_float2(xrsqrt(a.x), xrsqrt(a.y)); }
-
-// FP64 (no packed form): per half, for code written once for both precisions.
-__device__ __forceinline__ double2 xadd(double2 a, double2 b) {
-    return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
-}
-__device__ __forceinline__ double2 xmul(double2 a, double2 b) {
-    return make_double2(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y));
-}
-__device__ __forceinline__ double2 xfma(double2 a, double2 b, double2 c) {
-    return make_double2(__fma_rn(a.x, b.x, c.x), __fma_rn(a.y, b.y, c.y));
-}
-__device__ __forceinline__ double2 xsub(double2 a, double2 b) {
-    return make_double2(__dsub_rn(a.x, b.x), __dsub_rn(a.y, b.y));
-}
-__device__ __forceinline__ double2 xneg(double2 a) { return make_double2(-a.x, -a.y); }
-__device__ __forceinline__ double2 xrsqrt(double2 a) { return make_double2(xrsqrt(a.x), xrsqrt(a.y)); }
 
 }  // namespace rs
