@@ -365,30 +365,34 @@ __global__ void __launch_bounds__(TERM_THREADS, sizeof(R) == 4 && MODE != TM_VAL
             rdot = xfma(u[0], dd[0], xfma(u[1], dd[1], xmul(u[2], dd[2])));
 #pragma unroll
             for (int k = 0; k < 3; k++) u0[k] = xmul(xsub(dd[k], xmul(u[k], rdot)), ir);
+            // 1/t' = -s' / t^2.  1/t has no bound (5e15 an ulp of r^2 inside the cutoff) and only
+            // e^{1/t} and h make its powers vanish: FP32 holds its square, so every product takes one
+            // of the two factors (through q, h / t, gamma h) before a second 1 / t^2.
             const R s0 = xmul(rdot, p.isig), s3 = -xmul(sv, p.isig);
-            const R it0 = -xmul(it2, s0), it3 = -xmul(it2, s3);   // of 1/t; it2 for a, 0 for gamma
             const R gh = xmul(p.gam, h);
-            h0 = xmul(gh, it0);
             hp[0] = xmul(gh, it2);
             hp[1] = xmul(h, it);
-            hp[2] = xmul(gh, it3);
+            hp[2] = -xmul(hp[0], s3);
+            h0 = -xmul(hp[0], s0);
             const R A0 = xmul(xmul(p.gam, it2), p.isig), c1 = xmul(xmul(R(2), gh), xmul(p.isig, it));
-            al[0] = -xfma(h0, A0, xmul(c1, it0));
             al[1] = -xfma(hp[0], A0, xmul(c1, it2));
+            al[0] = -xmul(al[1], s0);
             al[2] = -xfma(hp[1], A0, xmul(xmul(h, it2), p.isig));
-            al[3] = -xfma(hp[2], A0, xfma(c1, it3, xmul(alpha, p.isig)));
+            al[3] = -xfma(al[1], s3, xmul(alpha, p.isig));
             const R b2 = xadd(ir, ir);
             be[0] = xmul(b2, xfma(-xmul(h, rdot), ir, h0));
             be[1] = xmul(b2, hp[0]);
             be[2] = xmul(b2, hp[1]);
             be[3] = xmul(b2, hp[2]);
-            // d(gv) = gs ds + 2 (B s^-4 - 1) (1/t) d(1/t), d(e^{1/t}) = e^{1/t} d(1/t)
+            // d(gv) = gs ds + 2 (B s^-4 - 1) (1/t) d(1/t), d(e^{1/t}) = e^{1/t} d(1/t); along s both
+            // s and t move (g2s), along a only t
             const R is3 = xmul(is2, is);
             const R gs = -xmul(xmul(R(4), p.B), xmul(is2, xfma(R(5), is4, xmul(is3, it2))));
-            const R H = xfma(xmul(R(2), B4), it, gv), E = -xmul(e1, p.isig);
-            g2t[0] = xmul(E, xfma(it0, H, xmul(gs, s0)));
-            g2t[1] = xmul(E, xmul(it2, H));
-            g2t[3] = xsub(xmul(E, xfma(it3, H, xmul(gs, s3))), xmul(g2, p.isig));
+            const R H = xfma(xmul(R(2), B4), it, gv), E = -xmul(e1, p.isig), q = xmul(E, it2);
+            const R g2s = xfma(-q, H, xmul(E, gs));
+            g2t[0] = xmul(g2s, s0);
+            g2t[1] = xmul(q, H);
+            g2t[3] = xsub(xmul(g2s, s3), xmul(g2, p.isig));
         }
         if (t.mlp_tab && r2 < p.mlp_rc2) {
             // u'/2 = (c1 + s (2 c2 + 3 s c3)) NG / (2 rc) on the cubic segment of interval
