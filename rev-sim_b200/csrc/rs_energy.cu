@@ -73,11 +73,12 @@ __global__ void __launch_bounds__(EG_THREADS) k_energy_grads(EnergyArgs a) {
                 }
                 const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
                 const bool on = ((mask >> (3 * ka + kb)) & 1u) && r2 <= a.rc2;
-                const double rinv = xrsqrt(on ? r2 : 1.0);
+                const double rinv = rsqrt(on ? r2 : 1.0);
+                const double r = r2 > 0.0 ? r2 * rinv : 0.0;   // overlapping atoms: infinite terms, not 0 x inf
                 const int QI = (ka > 0) + (kb > 0);
                 ec += (on ? qq[QI] : 0.0) * (rinv + a.krf * r2 - a.crf_shift);
                 if (ka == 0 && kb == 0 && gate && on) {
-                    const DN<4> Ef = form_energy<FORM>(a.form_p, r2 * rinv);
+                    const DN<4> Ef = form_energy<FORM>(a.form_p, r);
                     ef += Ef.v;
                     if (a.grads) {
 #pragma unroll
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(EG_THREADS) k_energy_grads(EnergyArgs a) {
                     }
                 }
                 if (FORM == F_LJ_MLP && on) {
-                    const double q = r2 * rinv * a.mlp_hinv;
+                    const double q = r * a.mlp_hinv;
                     const int g = min((int)q, MLP_NG - 1);
                     const double s = q - g;
                     const V4 c = reinterpret_cast<const V4 *>(a.mlp_tab)[QI * MLP_NG + g];
