@@ -280,10 +280,15 @@ __device__ __forceinline__ void pair_term(bool bit, R dx, R dy, R dz, const type
     constexpr bool CHG_F = charge_from_forces(FORM);
     const R r2 = xfma(dz, dz, xfma(dy, dy, xmul(dx, dx)));
     const bool on = bit && r2 <= nb.rc2;
-    const R rinv = xrsqrt(r2);
     const R qz = on ? nb.qq[QI] : R(0);
-    const R invr2 = xmul(rinv, rinv);
-    const R rinv3 = xmul(invr2, rinv);
+    R rinv = R(0), invr2, rinv3;
+    if (OO || FORM == F_LJ_MLP) {
+        rinv = xrsqrt(r2);
+        invr2 = xmul(rinv, rinv);
+        rinv3 = xmul(invr2, rinv);
+    } else {
+        inv_r23(r2, invr2, rinv3);
+    }
     const R mAc = xmul(qz, xsub(nb.krf2, rinv3));   // -A of the Coulomb term
     R mA = mAc;
     R mB = R(0);
