@@ -224,7 +224,7 @@ __device__ __forceinline__ void mlp_segment(const NbConsts<R> &nb, int QI, R r, 
                                             R &d2) {
     using V4m = typename V4T<R>::T;
     const R q = xmul(r, nb.mlp_hinv);
-    gi = min((int)q, MLP_NG - 1);
+    gi = max(min((int)q, MLP_NG - 1), 0);   // (a double NaN, of overlapping atoms, converts to INT_MIN)
     sm = xsub(q, (R)gi);
     const V4m cf = reinterpret_cast<const V4m *>(nb.mlp_tab)[QI * MLP_NG + gi];
     d1 = xmul(xfma(sm, xfma(xmul(R(3), sm), cf.w, xmul(R(2), cf.z)), cf.y), nb.mlp_hinv);

@@ -4,7 +4,7 @@ not NaN (r = 0 is a plain value of every form but those that divide by r)."""
 import numpy as np
 import pytest
 
-from revsim import Engine, constants as C, mlp
+from revsim import Engine, RevsimError, constants as C, mlp
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +45,21 @@ def test_energy_of_overlapping_atoms_with_the_learned_term():
     e.close()
     assert E[0] == np.inf
     assert np.isfinite(g[0, len(C.default_params()):]).all()
+
+
+@pytest.mark.parametrize("a,b", [(0, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("with_mlp", [False, True])
+def test_forces_of_overlapping_atoms_are_an_error(a, b, with_mlp):
+    """An error of the call, also where the NaN distance would be the learned term's table index."""
+    e = Engine(2, 2.6, precision="fp64", mlp=with_mlp)
+    p = C.default_params()
+    e.set_params(np.concatenate([p, mlp.init_params(3)]) if with_mlp else p)
+    x = _pair(a, b)
+    e.set_state(x, np.zeros((6, 3)))
+    with pytest.raises(RevsimError):
+        e.forces()
+    with pytest.raises(RevsimError):
+        e.force_vjp(np.ones_like(x), np.ones_like(x))
+    e.set_state(x + np.arange(6)[:, None] // 3 * 0.5, np.zeros((6, 3)))
+    assert np.isfinite(e.forces()).all()
+    e.close()
