@@ -331,7 +331,8 @@ int32_t revsim_kernel_time(revsim_handle *h, int32_t which, double *total_ms, in
  * its forces are the forward pass's bits); a count the other kernel's shape does not allow
  * returns REVSIM_ERR_BADARG.  A CTA takes as many of the asked molecules as its register budget
  * holds beside the warps that update them.  Until a shape is set the library picks one by the
- * number of molecules.  The FP64 reverse kernel's form 2 takes one entry too, with the registers
+ * number of molecules; molecules per CTA that were never given stay its choice for the lanes and the
+ * loop form in use.  revsim_get_launch_shape returns the shape in use, and that shape can be set.  The FP64 reverse kernel's form 2 takes one entry too, with the registers
  * of two.  revsim_autotune times the allowed shapes on the current state
  * (CTAs of 64-512 threads, plus the molecule counts that spread the CTAs over every SM in
  * one wave of one or two per SM) and keeps the lane count with the smallest forward +

@@ -93,10 +93,9 @@ struct revsim_handle {
     // CTA -> (replica, first molecule, molecule count) table.
     struct Shape {
         int G = 32, mpc = 8, U = 1, n_blk = 0;
-        // molecules per CTA of the table: the default's (step_default) until a shape is set, then
-        // mpc or as many as fit with the update warps
-        int cta = 8;
-        bool set = false;
+        int cta = 0;              // molecules per CTA of the table: mpc, or as many as fit with the update warps
+        bool own = true;          // nothing about the shape was set
+        bool own_mols = true;     // mpc was not set: default_mols at G and U
         int *d_blk_rep = nullptr, *d_blk_mol0 = nullptr, *d_blk_nmol = nullptr;
     } shp[2];
     bool shift_ok = false;   // one periodic image per molecule pair is exact for every box
@@ -386,6 +385,17 @@ size_t cnts_set(const revsim_handle *h) { return (size_t)h->M * (split_rows(h) ?
 // per molecule pair in every box, and no barostat (whose box moves could end that).
 bool half_eff(const revsim_handle *h) { return h->half_req && split_rows(h) && h->shift_ok && !h->baro_on; }
 
+// The library's own launch shapes: the fused kernels' by the number of molecules (step_default);
+// 32 lanes and eight molecules for the half-shell kernels.
+StepShape default_shape(const revsim_handle *h, int dir) {
+    if (h->half_req) return {32, 1};
+    return step_default(h->prec == REVSIM_MIXED, dir == 0, h->M);
+}
+int default_mols(const revsim_handle *h, int dir, int G, int U) {
+    if (h->half_req) return 8;
+    return step_default_mols(h->prec == REVSIM_MIXED, dir == 0, U, G, h->M);
+}
+
 // The step kernels' dtheta partials and |dl_dfi|^2 sums (d_part, d_norm2): one slot per
 // molecule for the both-sides kernels, one per CTA of the reverse block table for the
 // half-shell kernels.  part_slots: the slots to clear; slot_owner: each slot's replica.
@@ -485,7 +495,7 @@ int launch_step_k(revsim_handle *h, bool rev, const StepArgs &a_in) {
 int build_block_table(revsim_handle *h, int dir) {
     revsim_handle::Shape &sh = h->shp[dir];
     std::vector<int> br, bm, bn;
-    if (sh.set) sh.cta = step_cta_mols(h->prec == REVSIM_MIXED, dir == 0, sh.U, sh.G, sh.mpc);
+    sh.cta = step_cta_mols(h->prec == REVSIM_MIXED, dir == 0, sh.U, sh.G, sh.mpc);
     for (int r = 0; r < h->R; r++)
         for (int m = 0; m < h->nmol[r]; m += sh.cta) {
             br.push_back(r);
@@ -1348,10 +1358,10 @@ int32_t revsim_create(const revsim_system_desc *d, revsim_handle **out) {
          cudaMemset(h->d_A, 0, sizeof(double) * n3) == cudaSuccess;
     if (!ok) return cfail("upload");
     for (int dir = 0; dir < 2; dir++) {
-        const StepShape d0 = step_default(h->prec == REVSIM_MIXED, dir == 0, h->M);
+        const StepShape d0 = default_shape(h, dir);
         h->shp[dir].G = d0.G;
         h->shp[dir].U = d0.U;
-        h->shp[dir].cta = d0.cta;
+        h->shp[dir].mpc = default_mols(h, dir, d0.G, d0.U);
     }
     if (build_block_table(h, 0) != REVSIM_OK || build_block_table(h, 1) != REVSIM_OK ||
         alloc_nbr(h, cap) != REVSIM_OK)
@@ -2201,14 +2211,14 @@ int32_t revsim_kernel_time(revsim_handle *h, int32_t which, double *total_ms, in
 namespace {
 
 // An allowed shape of step kernel dir (0 reverse, 1 forward): lanes 8, 16 or 32, whole warps,
-// at most 512 threads and no more than the kernel's register budget lets one CTA have.
+// at most 512 threads and no more than the kernel's register budget lets one CTA have; the
+// library's own choice always.
 bool shape_ok(const revsim_handle *h, int dir, int G, int m, int U) {
     const int thr = G * m;
-    if (!((G == 8 || G == 16 || G == 32) && m >= 1 && thr <= 512 && thr % 32 == 0 && U >= 1 && U <= 3 &&
-          !(U == 3 && thr > 256)))
+    if (!((G == 8 || G == 16 || G == 32) && m >= 1 && thr % 32 == 0 && U >= 1 && U <= 3 && !(U == 3 && thr > 256)))
         return false;
     if (half_eff(h) && thr > half_max_threads(dir == 0)) return false;
-    return thr <= shape_max_threads(h->prec == REVSIM_MIXED, dir == 0, U);
+    return m == default_mols(h, dir, G, U) || thr <= shape_max_threads(h->prec == REVSIM_MIXED, dir == 0, U);
 }
 
 // Shape of one step kernel (dir 0 reverse, 1 forward), after shape_ok.
@@ -2218,7 +2228,6 @@ int set_shape_dir(revsim_handle *h, int dir, int G, int m, int U) {
     sh.G = G;
     sh.U = U;
     sh.mpc = m;
-    sh.set = true;
     if (step_cta_mols(h->prec == REVSIM_MIXED, dir == 0, U, G, m) != sh.cta || !sh.d_blk_rep) return build_block_table(h, dir);
     return REVSIM_OK;
 }
@@ -2238,14 +2247,19 @@ int32_t revsim_set_pair_mode(revsim_handle *h, int32_t mode) {
     h->half_req = want;
     h->gen++;
     h->fwd_valid = false;
-    // the half-shell reverse kernel allows fewer threads per CTA: shrink a shape beyond it (and
-    // give up the default CTA size, which is the fused kernels')
+    // what was never set becomes the mode's default; the half-shell reverse kernel allows fewer
+    // threads per CTA: shrink a set shape beyond it
+    const bool own = h->shp[0].own && h->shp[1].own;   // (both: the lanes are one setting)
     for (int dir = 0; dir < 2; dir++) {
-        revsim_handle::Shape &sh = h->shp[dir];
-        if (shape_ok(h, dir, sh.G, sh.mpc, sh.U) && sh.set) continue;
-        int m = sh.mpc;
-        while (m > 1 && !shape_ok(h, dir, sh.G, m, 1)) m--;
-        if (int rc = set_shape_dir(h, dir, sh.G, m, 1)) return rc;
+        const revsim_handle::Shape &sh = h->shp[dir];
+        const StepShape d0 = default_shape(h, dir);
+        const int G = own ? d0.G : sh.G;
+        int U = sh.own ? d0.U : sh.U, m = sh.own_mols ? default_mols(h, dir, G, U) : sh.mpc;
+        if (!shape_ok(h, dir, G, m, U)) {
+            U = 1;
+            while (m > 1 && !shape_ok(h, dir, G, m, U)) m--;
+        }
+        if (int rc = set_shape_dir(h, dir, G, m, U)) return rc;
     }
     return REVSIM_OK;
 }
@@ -2270,16 +2284,21 @@ int32_t revsim_set_launch_shape(revsim_handle *h, int32_t which, int32_t lanes, 
         const revsim_handle::Shape &sh = h->shp[dir];
         const bool sel = which < 0 || which == dir;
         G[dir] = lanes ? lanes : sh.G;
-        m[dir] = sel && mpc ? mpc : sh.mpc;
         U[dir] = sel && unroll ? unroll : sh.U;
+        m[dir] = sel && mpc ? mpc : (sh.own_mols ? default_mols(h, dir, G[dir], U[dir]) : sh.mpc);
         if (!shape_ok(h, dir, G[dir], m[dir], U[dir]))
             return fail(h, REVSIM_ERR_BADARG,
                         sel ? "unsupported launch shape"
                             : "lanes per molecule apply to both step kernels; the other kernel's "
                               "shape does not allow this count");
     }
-    for (int dir = 0; dir < 2; dir++)
+    for (int dir = 0; dir < 2; dir++) {
+        revsim_handle::Shape &sh = h->shp[dir];
+        const bool sel = which < 0 || which == dir;
+        if (lanes || (sel && (mpc || unroll))) sh.own = false;
+        if (sel && mpc) sh.own_mols = false;
         if (int rc = set_shape_dir(h, dir, G[dir], m[dir], U[dir])) return rc;
+    }
     return REVSIM_OK;
 }
 
@@ -2372,7 +2391,10 @@ int32_t revsim_autotune(revsim_handle *h, double dt) {
             }
         }
     }
-    for (int dir = 0; dir < 2 && !rc; dir++) rc = set_shape_dir(h, dir, bg, bm[dir], bu[dir]);
+    for (int dir = 0; dir < 2 && !rc; dir++) {
+        h->shp[dir].own = h->shp[dir].own_mols = false;
+        rc = set_shape_dir(h, dir, bg, bm[dir], bu[dir]);
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     return rc;

@@ -153,14 +153,17 @@ constexpr int one_wave_mols(bool fp32, bool rev, int U, int G, int M) {
 // registers it wants, and stays at 32 lanes up to 4,000 all the same (3,000: 26 | 45 at 32 lanes,
 // 25 | 49 at 16; 14,320: 98 | 205 and 90 | 185).  Before: 32 lanes and eight molecules always.
 struct StepShape {
-    int G, U, cta;
+    int G, U;
 };
 constexpr StepShape step_default(bool fp32, bool rev, int M) {
     const int G = (fp32 ? one_wave_mols(true, true, 1, 32, M) > 0 : M <= 4000) ? 32 : 16;
-    const int U = rev && G == 32 && (!fp32 || M <= 1200) ? 2 : 1;
-    const int m = one_wave_mols(fp32, rev, U, G, M);
-    const int fill = G == 32 ? 7 : (!fp32 && rev ? 10 : 8);
-    return {G, U, m ? m : fill};
+    return {G, rev && G == 32 && (!fp32 || M <= 1200) ? 2 : 1};
+}
+// Molecules per CTA at those or other lanes and loop forms (form 3 takes 256 pair threads at most).
+constexpr int step_default_mols(bool fp32, bool rev, int U, int G, int M) {
+    const int one = one_wave_mols(fp32, rev, U, G, M), fill = G == 32 ? 7 : (G == 16 && !fp32 && rev ? 10 : 8);
+    const int m = one ? one : fill;
+    return U == 3 && G * m > 256 ? 256 / G : m;
 }
 
 // Everything the step kernels read or write.
