@@ -385,15 +385,22 @@ size_t cnts_set(const revsim_handle *h) { return (size_t)h->M * (split_rows(h) ?
 // per molecule pair in every box, and no barostat (whose box moves could end that).
 bool half_eff(const revsim_handle *h) { return h->half_req && split_rows(h) && h->shift_ok && !h->baro_on; }
 
+// CTAs of m molecules over all replicas.
+int blocks_for(const revsim_handle *h, int m) {
+    int b = 0;
+    for (int n : h->nmol) b += (n + m - 1) / m;
+    return b;
+}
+
 // The library's own launch shapes: the fused kernels' by the number of molecules (step_default);
 // 32 lanes and eight molecules for the half-shell kernels.
 StepShape default_shape(const revsim_handle *h, int dir) {
     if (h->half_req) return {32, 1};
-    return step_default(h->prec == REVSIM_MIXED, dir == 0, h->M);
+    return step_default(h->prec == REVSIM_MIXED, dir == 0, h->M, [h](int m) { return blocks_for(h, m); });
 }
 int default_mols(const revsim_handle *h, int dir, int G, int U) {
     if (h->half_req) return 8;
-    return step_default_mols(h->prec == REVSIM_MIXED, dir == 0, U, G, h->M);
+    return step_default_mols(h->prec == REVSIM_MIXED, dir == 0, U, G, [h](int m) { return blocks_for(h, m); });
 }
 
 // The step kernels' dtheta partials and |dl_dfi|^2 sums (d_part, d_norm2): one slot per
@@ -2328,11 +2335,6 @@ int32_t revsim_autotune(revsim_handle *h, double dt) {
     int bm[2] = {h->shp[0].mpc, h->shp[1].mpc}, bu[2] = {h->shp[0].U, h->shp[1].U}, bg = h->shp[0].G;
     int n_sm = 148;
     CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->dev));
-    auto blocks_for = [&](int m) {
-        long b = 0;
-        for (int r = 0; r < h->R; r++) b += (h->nmol[r] + m - 1) / m;
-        return b;
-    };
     for (int G : {8, 16, 32}) {
         double tot = 0.0;
         int gm[2] = {0, 0}, gu[2] = {1, 1};
@@ -2345,7 +2347,7 @@ int32_t revsim_autotune(revsim_handle *h, double dt) {
         const int mstep = std::max(1, 32 / G);
         for (int k : {1, 2}) {
             int m = mstep;
-            while (m * G <= 512 && blocks_for(m) > (long)k * n_sm) m += mstep;
+            while (m * G <= 512 && blocks_for(h, m) > (long)k * n_sm) m += mstep;
             if (m * G <= 512 && std::find(mpcs.begin(), mpcs.end(), m) == mpcs.end()) mpcs.push_back(m);
         }
         for (int dir = 0; dir < 2 && !rc; dir++) {

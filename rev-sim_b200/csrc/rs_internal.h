@@ -128,13 +128,15 @@ constexpr int step_cta_mols(bool fp32, bool rev, int U, int G, int mols) {
 constexpr int half_nreg(bool rev) { return rev ? RS_NREG_HALF_REV : 128; }
 constexpr int half_max_threads(bool rev) { return max_threads_for(half_nreg(rev)); }
 
-// Molecules per CTA that leave the busiest SM the fewest molecules when all M run as one wave of
-// CTAs, at G lanes each; 0 when no count fits one wave (by the registers).
-constexpr int one_wave_mols(bool fp32, bool rev, int U, int G, int M) {
+// Molecules per CTA that leave the busiest SM the fewest molecules when all run as one wave of
+// CTAs, at G lanes each; 0 when no count fits one wave (by the registers).  blocks(m): the CTAs of m
+// molecules, of which none straddles two replicas.
+template <class F>
+int one_wave_mols(bool fp32, bool rev, int U, int G, const F &blocks) {
     const int cap = step_max_threads(fp32, rev, U) / 32;   // warps an SM holds
     int best = 0, load = 0;
     for (int m = 32 / G; m <= 32; m += 32 / G) {
-        const int ctas = ((M + m - 1) / m + 147) / 148, warps = m * G / 32 + update_warps(m);
+        const int ctas = (blocks(m) + 147) / 148, warps = m * G / 32 + update_warps(m);
         if (ctas * warps > cap || (best && ctas * m > load)) continue;
         best = m;
         load = ctas * m;
@@ -150,18 +152,24 @@ constexpr int one_wave_mols(bool fp32, bool rev, int U, int G, int M) {
 // time, hence one_wave_mols (3,000 waters, mixed, 16 lanes: 22 molecules in 137 CTAs 17.7 | 23.7
 // us a forward | reverse step, 8 in 375 18.3 | 26.1, 12 in 250 19.5 | 28.0; 2,001 at 32 lanes: 14
 // 13.7 | 16.9, 4 14.9 | 19.2).  FP64's reverse kernel holds seven molecules an SM with the
-// registers it wants, and stays at 32 lanes up to 4,000 all the same (3,000: 26 | 45 at 32 lanes,
-// 25 | 49 at 16; 14,320: 98 | 205 and 90 | 185).  Before: 32 lanes and eight molecules always.
+// registers it wants, and stays at 32 lanes up to 4,000 all the same (3,600: 32 | 59 at 32 lanes, 34 | 62
+// at 16; 4,200: 39 | 73 and 37 | 67; 5,000: 42 | 78 and 42 | 82; 6,500: 51 | 101 and 48 | 96).  The FP32
+// reverse kernel's second entry pays while its 128 registers hold the molecules (895: 12.0 and 12.7 with
+// one entry; 1,184: 12.5 and 12.8).  The waves count each replica's CTAs (3 x 394, mixed: 9 molecules
+// 11.6 | 15.0, the 8 of one box of 1,182 are 150 CTAs, 12.4 | 18.9; 16 x 181: 22, 11.8 | 15.7, and 20,
+// 15.0 | 22.6).  Before: 32 lanes and eight molecules always.
 struct StepShape {
     int G, U;
 };
-constexpr StepShape step_default(bool fp32, bool rev, int M) {
-    const int G = (fp32 ? one_wave_mols(true, true, 1, 32, M) > 0 : M <= 4000) ? 32 : 16;
+template <class F>
+StepShape step_default(bool fp32, bool rev, int M, const F &blocks) {
+    const int G = (fp32 ? one_wave_mols(true, true, 1, 32, blocks) > 0 : M <= 4000) ? 32 : 16;
     return {G, rev && G == 32 && (!fp32 || M <= 1200) ? 2 : 1};
 }
 // Molecules per CTA at those or other lanes and loop forms (form 3 takes 256 pair threads at most).
-constexpr int step_default_mols(bool fp32, bool rev, int U, int G, int M) {
-    const int one = one_wave_mols(fp32, rev, U, G, M), fill = G == 32 ? 7 : (G == 16 && !fp32 && rev ? 10 : 8);
+template <class F>
+int step_default_mols(bool fp32, bool rev, int U, int G, const F &blocks) {
+    const int one = one_wave_mols(fp32, rev, U, G, blocks), fill = G == 32 ? 7 : (G == 16 && !fp32 && rev ? 10 : 8);
     const int m = one ? one : fill;
     return U == 3 && G * m > 256 ? 256 / G : m;
 }

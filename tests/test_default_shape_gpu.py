@@ -92,6 +92,15 @@ def test_setting_back_changes_nothing(prec, n, b, mols):
     e.close()
 
 
+@pytest.mark.parametrize("n,reps,rev,fwd", [(394, 3, (32, 9, 2), (32, 9, 1)), (181, 16, (16, 22, 1), (16, 22, 1)),
+                                            (150, 17, (16, 20, 1), (16, 20, 1))])
+def test_one_wave_counts_the_replicas(n, reps, rev, fwd):
+    """No CTA straddles two replicas: 3 boxes of 394 are 150 CTAs of eight molecules, 132 of nine."""
+    e = Engine([n] * reps, [2.6] * reps, precision="mixed")
+    assert (e.launch_shape(0), e.launch_shape(1)) == (rev, fwd)
+    e.close()
+
+
 @pytest.mark.parametrize("n,b", [(400, 2.48), (2600, 4.3), (3000, 4.5)])
 def test_half_shell_and_back(n, b):
     e = _engine(n, b, "mixed")
