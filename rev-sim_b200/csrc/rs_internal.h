@@ -155,9 +155,9 @@ int one_wave_mols(bool fp32, bool rev, int U, int G, const F &blocks) {
 // registers it wants, and stays at 32 lanes up to 4,000 all the same (3,600: 32 | 59 at 32 lanes, 34 | 62
 // at 16; 4,200: 39 | 73 and 37 | 67; 5,000: 42 | 78 and 42 | 82; 6,500: 51 | 101 and 48 | 96).  The FP32
 // reverse kernel's second entry pays while its 128 registers hold the molecules (895: 12.0 and 12.7 with
-// one entry; 1,184: 12.5 and 12.8).  The waves count each replica's CTAs (3 x 394, mixed: 9 molecules
-// 11.6 | 15.0, the 8 of one box of 1,182 are 150 CTAs, 12.4 | 18.9; 16 x 181: 22, 11.8 | 15.7, and 20,
-// 15.0 | 22.6).  Before: 32 lanes and eight molecules always.
+// one entry; 1,184: 12.5 and 12.8).  The waves count each replica's CTAs (3 x 394, mixed: 2 molecules in
+// 591 CTAs, four an SM, 11.6 | 15.0; the 8 of one box of 1,182 are 150 CTAs, 12.4 | 18.9; 16 x 181: 4 in
+// 736 CTAs 11.8 | 15.7, the 20 of one box 15.0 | 22.6).  Before: 32 lanes and eight molecules always.
 struct StepShape {
     int G, U;
 };

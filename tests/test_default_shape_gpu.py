@@ -92,11 +92,11 @@ def test_setting_back_changes_nothing(prec, n, b, mols):
     e.close()
 
 
-@pytest.mark.parametrize("n,reps,rev,fwd", [(394, 3, (32, 9, 2), (32, 9, 1)), (181, 16, (16, 22, 1), (16, 22, 1)),
-                                            (150, 17, (16, 20, 1), (16, 20, 1))])
-def test_one_wave_counts_the_replicas(n, reps, rev, fwd):
-    """No CTA straddles two replicas: 3 boxes of 394 are 150 CTAs of eight molecules, 132 of nine."""
-    e = Engine([n] * reps, [2.6] * reps, precision="mixed")
+@pytest.mark.parametrize("ns,rev,fwd", [([394] * 3, (32, 2, 2), (32, 2, 1)), ([181] * 16, (16, 4, 1), (16, 4, 1)),
+                                        ([150] * 17, (32, 9, 1), (32, 9, 1)), ([700, 1100], (32, 13, 1), (32, 13, 1))])
+def test_one_wave_counts_the_replicas(ns, rev, fwd):
+    """No CTA straddles two replicas: 3 boxes of 394 are 150 CTAs of eight molecules, one too many an SM."""
+    e = Engine(ns, [2.6 if n < 500 else 3.3 for n in ns], precision="mixed")
     assert (e.launch_shape(0), e.launch_shape(1)) == (rev, fwd)
     e.close()
 
