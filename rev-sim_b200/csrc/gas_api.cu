@@ -694,7 +694,8 @@ int32_t revsim_gas_set_rdf(revsim_gas_handle *h, int32_t n_terms, const revsim_r
         same = t.sel1 == o.sel1 && t.sel2 == o.sel2 && t.x_min == o.x_min && t.step == o.step && t.width == o.width &&
                t.exp_cutoff == o.exp_cutoff && t.n_grid == o.n_grid && t.slice_start == o.slice_start &&
                t.slice_stride == o.slice_stride && t.n_target == o.n_target && t.norm == o.norm &&
-               t.weight == o.weight && std::equal(h->rdf[i].target.begin(), h->rdf[i].target.end(), targets[i]);
+               t.weight == o.weight && h->rdf[i].target.size() == (size_t)t.n_target &&
+               std::equal(h->rdf[i].target.begin(), h->rdf[i].target.end(), targets[i]);
     }
     if (same) return REVSIM_OK;
     CK(cudaStreamSynchronize(h->st));
@@ -716,8 +717,12 @@ int32_t revsim_gas_set_rdf(revsim_gas_handle *h, int32_t n_terms, const revsim_r
         // the normaliser V / (4 pi n1 n2 step) behind the slice sums (rdf_differentiable, 725)
         const double n1 = t.sel1 == 0 ? h->nw : 2.0 * h->nw, n2 = t.sel2 == 0 ? h->nw : 2.0 * h->nw;
         const double pre = h->L * h->L * h->L / (4 * pi * n1 * n2 * t.step);
-        CK(cudaMemcpy(D.d_target, targets[i], sizeof(double) * t.n_target, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(D.d_sum + t.n_target, &pre, sizeof(double), cudaMemcpyHostToDevice));
+        if (cudaMemcpyAsync(D.d_target, targets[i], sizeof(double) * t.n_target, cudaMemcpyHostToDevice, h->st) !=
+                cudaSuccess ||
+            cudaMemcpyAsync(D.d_sum + t.n_target, &pre, sizeof(double), cudaMemcpyHostToDevice, h->st) != cudaSuccess) {
+            free_rdf(h);
+            return fail(h, REVSIM_ERR_CUDA, "RDF targets");
+        }
         D.target.assign(targets[i], targets[i] + t.n_target);
     }
     return REVSIM_OK;

@@ -1579,17 +1579,24 @@ int32_t revsim_set_loss(revsim_handle *h, int32_t n_terms, const revsim_rdf_term
             pre[r] = V / (4 * 3.14159265358979323846 * n1 * n2 * t.step);
         }
         const bool up_t = target != T.target, up_p = pre != T.pre;
-        T.target.swap(target);
-        T.pre.swap(pre);
+        // recorded once they are on the device: a copy that fails leaves nothing to skip the next one
+        T.target.clear();
+        T.pre.clear();
         h->terms.push_back(T);
-        const Term &D = h->terms.back();
+        Term &D = h->terms.back();
         if (up_t && t.n_target > 0 &&
-            cudaMemcpy(D.d_target, D.target.data(), sizeof(double) * D.target.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            cudaMemcpyAsync(D.d_target, target.data(), sizeof(double) * target.size(), cudaMemcpyHostToDevice, h->st) !=
+                cudaSuccess) {
             rc = fail(h, REVSIM_ERR_CUDA, "loss targets");
-        if (!rc && up_p &&
-            cudaMemcpy(D.d_hist + (size_t)h->R * t.n_grid, D.pre.data(), sizeof(double) * h->R, cudaMemcpyHostToDevice) !=
-                cudaSuccess)
+            break;
+        }
+        D.target.swap(target);
+        if (up_p && cudaMemcpyAsync(D.d_hist + (size_t)h->R * t.n_grid, pre.data(), sizeof(double) * h->R,
+                                    cudaMemcpyHostToDevice, h->st) != cudaSuccess) {
             rc = fail(h, REVSIM_ERR_CUDA, "loss normalisers");
+            break;
+        }
+        D.pre.swap(pre);
     }
     for (Term &T : old) release(T);
     return rc;
