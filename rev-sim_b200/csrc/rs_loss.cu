@@ -244,7 +244,10 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
     const double qS = exp(-__dmul_rn(__dmul_rn(2.0, __dmul_rn(S, S)), inv_w));
     const double dmin = __dsub_rn(__dsub_rn(grid_x(a, sl.s0), a.cutoff), a.step);
     const double dmax = __dadd_rn(__dadd_rn(grid_x(a, sl.s0 + (sl.nt - 1) * sl.sd), a.cutoff), a.step);
-    // FP32 distances err by < 1e-6 L: a margin that no pair in range can miss
+    // FP32 coordinates of atoms within 16 boxes of the origin (NaN beyond, which decides nothing):
+    // their distances err by < 4e-6 L, a margin that no pair in range can miss
+    const double xmax = 16.0 * L;
+    auto test_x = [xmax](double x) { return fabs(x) <= xmax ? (float)x : __int_as_float(0x7FC00000); };
     const float marg = 1e-3f + 1e-5f * Lf;
     const float far = (float)dmax + marg, near = fmaxf(0.f, (float)dmin - marg);
     const float far2 = far * far, near2 = near * near;
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
 #pragma unroll
         for (int u = 0; u < 3; u++) {
             xi[u] = a.x[3 * (size_t)ia + u];
-            xf[u] = (float)xi[u];
+            xf[u] = test_x(xi[u]);
         }
     }
     // equal sets: atom i takes the pairs (i, i + k mod n), k = 1 .. n/2, the last of them (n
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
         for (int u = 0; u < 3; u++) dr[u] = vec1d(xi[u], xb[u], L);
         d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dr[0], dr[0]), __dmul_rn(dr[1], dr[1])),
                                               __dmul_rn(dr[2], dr[2])));
-        if (d == 0.0 || d < dmin || d > dmax) return false;
+        if (d == 0.0 || !(d >= dmin && d <= dmax)) return false;
         // The slice points of the window, x - c <= d <= x + c.  The product with 1 / S, rounded
         // outwards, is the first (last) of them, the point before it or, within its rounding of a
         // point, the one before that: two steps inwards without branches.
@@ -412,7 +415,7 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
                 const int j = same ? (i0 + 1 + p) % n1 : p;
                 const double *xj = a.x + 3 * (size_t)rdf_atom(a.sel2, atom0, j);
 #pragma unroll
-                for (int u = 0; u < 3; u++) s_x[u][threadIdx.x] = (float)xj[u];
+                for (int u = 0; u < 3; u++) s_x[u][threadIdx.x] = test_x(xj[u]);
             }
         }
         __syncthreads();
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
                     d = d > hLf ? d - Lf : (d < -hLf ? d + Lf : d);
                     r2 = fmaf(d, d, r2);
                 }
-                ok = r2 <= far2 && r2 >= near2;
+                ok = !(r2 > far2) && !(r2 < near2);
             }
             const unsigned m = __ballot_sync(0xffffffffu, ok);
             if (ok) {
