@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(256) k_rdf_loss_finalize(RdfArgs a, RdfSlice s
             l = __dadd_rn(l, __dmul_rn(e, e));
             g = __dmul_rn(weight, __dmul_rn(2.0, e));
         }
-        wt[t] = __ddiv_rn(__dmul_rn(g, pre[r]), x2);
+        wt[t] = g == 0.0 ? 0.0 : __ddiv_rn(__dmul_rn(g, pre[r]), x2);   // (x = 0 with no weight)
     }
     s_l[threadIdx.x] = l;
     __syncthreads();

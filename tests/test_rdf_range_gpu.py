@@ -1,5 +1,6 @@
-"""The RDF loss for atoms far from the origin (the kernels' FP32 distance test must not decide what it
-cannot resolve), against the oracle at the RDF tests' 1e-11, and for non-finite positions."""
+"""The RDF loss away from positions inside the box and grid points above 0: atoms far from the origin
+(the kernels' FP32 distance test must not decide what it cannot resolve), non-finite positions, and a
+grid point at x = 0 that carries no weight.  Against the oracle at the RDF tests' 1e-11."""
 
 import numpy as np
 import pytest
@@ -46,3 +47,12 @@ def test_non_finite_positions_have_no_pairs(bad):
     x[3 * 17] = bad
     l, g = _loss_grad(x, args)
     assert np.isfinite(l) and np.isfinite(g).all() and not g[3 * 17].any()
+
+
+def test_no_weight_at_zero():
+    """Intramolecular O-H pairs reach the point x = 0, where h is infinite; a term of weight 0 has no
+    gradient all the same."""
+    x = systems.water_coords(N_MOL, BOX, seed=3)
+    args = (0, 1, 0.0, 0.005, 0.002, 0.15, 100, 0, 1, np.ones(100), 1, 0.0)
+    _, g = _loss_grad(x, args)
+    assert not g.any()
