@@ -177,7 +177,7 @@ int gas_cta_atoms(int nreg, int N) {
     const int cap = std::min(64, 4 * (512 / nreg));   // warps an SM holds
     int best = 0, load = 0;
     for (int m = 1; m <= 31; m++) {
-        const int ctas = ((N + m - 1) / m + 147) / 148;
+        const int ctas = ((N + m - 1) / m + kSMs - 1) / kSMs;
         if (ctas * (m + 1) > cap || (best && ctas * m > load)) continue;
         best = m;
         load = ctas * m;
@@ -758,7 +758,7 @@ void step_launch(const GasConstsT<R> &k, GasArgs a, cudaStream_t st) {
     a.cfH = a.dt * a.dt / (2.0 * a.mH);
     a.apc = gas_cta_atoms(nreg, a.N);
     const int grid = (a.N + a.apc - 1) / a.apc;
-    a.chain_early = grid <= 148;
+    a.chain_early = grid <= kSMs;
     launch_chained(k_gas_step<R, FORM, REV>, dim3(grid), dim3(32 * (a.apc + 1)),
                    (size_t)a.apc * (NS * sizeof(double) + kQueue * sizeof(int)), st, k, a);
 }

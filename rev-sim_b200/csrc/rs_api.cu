@@ -458,7 +458,7 @@ int launch_step_k(revsim_handle *h, bool rev, const StepArgs &a_in) {
     // an uneven last wave leave the next step uneven too (3,000 waters, mixed: 23.5 | 30.6 us a
     // forward | reverse step with the early release, 18.3 | 25.7 with the late one, 20.0 | 26.6
     // unchained; 895 waters FP64: 12.7 us a forward step early, 15.2 late).
-    a.chain_early = sh.n_blk <= 148;
+    a.chain_early = sh.n_blk <= kSMs;
     const BondConsts bc = bond_consts(h);
     const bool timed = h->ktime && !(a.mode & MODE_FORCES_ONLY);
     const int which = rev ? 0 : 1;
@@ -2340,7 +2340,7 @@ int32_t revsim_autotune(revsim_handle *h, double dt) {
     CK(cudaEventCreate(&e1));
     double best_total = std::numeric_limits<double>::infinity();
     int bm[2] = {h->shp[0].mpc, h->shp[1].mpc}, bu[2] = {h->shp[0].U, h->shp[1].U}, bg = h->shp[0].G;
-    int n_sm = 148;
+    int n_sm = kSMs;
     CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->dev));
     for (int G : {8, 16, 32}) {
         double tot = 0.0;

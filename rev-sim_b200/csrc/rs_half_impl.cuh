@@ -30,46 +30,19 @@ namespace rs {
 
 namespace {
 
-// The O-O Lennard-Jones form of pair_form on both halves of a register pair at once (the
-// packed instructions round each half as the scalar ones do, so the halves carry the bits of
-// pair_form<R, F_LJ>).  c[0] = sigma^2, c[1] = 24 eps, c[2] = 144 eps / sigma, c[3] = 1/eps.
-template <typename R, bool GRAD>
-__device__ __forceinline__ void lj_form2(const FormConsts<R> &fc, typename PkT<R>::T rinv,
-                                         typename PkT<R>::T invr2, typename PkT<R>::T &F,
-                                         typename PkT<R>::T &dF, typename PkT<R>::T g[2]) {
-    using P = typename PkT<R>::T;
-    P six = xmul(pk1(fc.c[0]), invr2);
-    six = xmul(xmul(six, six), six);
-    const P twelve = xmul(six, six);
-    F = xmul(xmul(pk1(fc.c[1]), rinv), xsub(xadd(twelve, twelve), six));
-    if (GRAD) {
-        dF = xneg(xmul(xmul(pk1(fc.c[1]), invr2), xsub(xmul(pk1(R(26)), twelve), xmul(pk1(R(7)), six))));
-        g[0] = xmul(xmul(pk1(fc.c[2]), rinv), xsub(xmul(pk1(R(4)), twelve), six));
-        g[1] = xmul(F, pk1(fc.c[3]));
-    }
+// Displacement of one slot for both entries: cx / cy = the neighbour atom's gather coordinate in
+// entry x / y, c = the own atom's; formed per half (the two results land in one register pair) and
+// packed from there on.  The gather coordinates are offsets from per-molecule cell origins
+// (gather_f32) and s carries the entries' origin differences (exact multiples of 0.5 nm) and one
+// periodic image per molecule pair (chosen from the O-O vector) for all nine atom pairs, the
+// minimum one for every pair within the cutoff whenever L > 2 (cutoff + 2 * max O-H distance); s
+// stays exact, so d + s is the one rounding of a vector within the cutoff.
+__device__ __forceinline__ float2 slot_d2(float c, float cx, float cy, float2 s) {
+    return xadd(pk(xsub(cx, c), xsub(cy, c)), s);
 }
 
-// Displacement of one slot for both entries (FP32 kernels): cx / cy = the neighbour atom's
-// gather coordinate in entry x / y, c = the own atom's; formed per half (the two results land
-// in one register pair) and packed from there on.  The gather coordinates are offsets from
-// per-molecule cell origins (gather_f32) and s carries the entries' origin differences (exact
-// multiples of 0.5 nm).  SHIFT: s also carries one periodic image per molecule pair (chosen
-// from the O-O vector) for all nine atom pairs, the minimum one for every pair within the
-// cutoff whenever L > 2 (cutoff + 2 * max O-H distance); s stays exact, so d + s is the one
-// rounding of a vector within the cutoff.  Otherwise the image is chosen per slot from d + s
-// and applied to s first (s - L rint((d + s) / L), exact), then added to d.
-template <typename R, bool SHIFT>
-__device__ __forceinline__ typename PkT<R>::T slot_d2(R c, R cx, R cy, typename PkT<R>::T s, R L, R invL) {
-    using P = typename PkT<R>::T;
-    const P d = pk(xsub(cx, c), xsub(cy, c));
-    if (SHIFT) return xadd(d, s);
-    const P q = xmul(xadd(d, s), pk1(invL));
-    return xadd(d, xfma(pk(-r_rint(q.x), -r_rint(q.y)), pk1(L), s));
-}
-
-template <typename R>
-__device__ __forceinline__ R image_shift(R d, R L, R hL) {
-    return d > hL ? -L : (d < -hL ? L : R(0));
+__device__ __forceinline__ float image_shift(float d, float L, float hL) {
+    return d > hL ? -L : (d < -hL ? L : 0.f);
 }
 
 // One (own atom KA, partner atom KB) slot of two owned entries (halves x and y): as
@@ -164,9 +137,9 @@ template <int FORM, bool REV, int KB>
 __device__ __forceinline__ void half_col(uint32_t mx, uint32_t my, const float4 pa[3], const float4 &pbx,
                                          const float4 &pby, const float4 wa[3], const float4 &wbx,
                                          const float4 &wby, const float ca[3][3], const float cbx[3],
-                                         const float cby[3], const float2 sh[3], float L, float invL,
-                                         const NbConsts<float> &nb, float2 f[3][3], float2 g[3][3], float2 *th,
-                                         float2 pf[3], float2 pg[3], double *madj) {
+                                         const float cby[3], const float2 sh[3], const NbConsts<float> &nb,
+                                         float2 f[3][3], float2 g[3][3], float2 *th, float2 pf[3], float2 pg[3],
+                                         double *madj) {
     using P = float2;
 #define RS_HSLOT(KA)                                                                                  \
     {                                                                                                 \
@@ -180,10 +153,10 @@ __device__ __forceinline__ void half_col(uint32_t mx, uint32_t my, const float4 
             cz = pk(xsub(ca[KA][2], cbx[2]), xsub(ca[KA][2], cby[2]));                                \
         }                                                                                             \
         half_term<FORM, REV, KA, KB>((mx >> (3 * KA + KB)) & 1u, (my >> (3 * KA + KB)) & 1u,          \
-                                     slot_d2<float, true>(pa[KA].x, pbx.x, pby.x, sh[0], L, invL),     \
-                                     slot_d2<float, true>(pa[KA].y, pbx.y, pby.y, sh[1], L, invL),     \
-                                     slot_d2<float, true>(pa[KA].z, pbx.z, pby.z, sh[2], L, invL), ex, \
-                                     ey, ez, cx, cy, cz, nb, f[KA], g[KA], th, pf, pg, madj);         \
+                                     slot_d2(pa[KA].x, pbx.x, pby.x, sh[0]),                          \
+                                     slot_d2(pa[KA].y, pbx.y, pby.y, sh[1]),                          \
+                                     slot_d2(pa[KA].z, pbx.z, pby.z, sh[2]), ex, ey, ez, cx, cy, cz,  \
+                                     nb, f[KA], g[KA], th, pf, pg, madj);                             \
     }
     RS_HSLOT(0);
     RS_HSLOT(1);
@@ -213,7 +186,6 @@ __global__ void __maxnreg__((half_nreg(REV))) k_water_half(StepArgs a, NbConsts<
     const bool active = grp < a.blk_nmol[blk];
     const double Ld = a.rep_box[rep];
     const R L = (R)Ld;
-    const R invL = (R)(1.0 / Ld);
     const V4 *__restrict__ pos = (const V4 *)a.pos_in;
     const V4 *__restrict__ wgt = (const V4 *)a.wgt_in;
     double *madj = FORM == F_LJ_MLP && REV
@@ -311,8 +283,8 @@ __global__ void __maxnreg__((half_nreg(REV))) k_water_half(StepArgs a, NbConsts<
                 cby[u] = (R)__dmul_rn(a.A[9 * (size_t)Jy + 3 * KB + u], sc);                           \
             }                                                                                          \
         }                                                                                              \
-        half_col<FORM, REV, KB>(mx, my, pa, pbx, pby, wa, wbx, wby, ca, cbx, cby, sh, L,                \
-                                invL, nb, f2, g2, th2, pf, pg, madj);                                  \
+        half_col<FORM, REV, KB>(mx, my, pa, pbx, pby, wa, wbx, wby, ca, cbx, cby, sh,                   \
+                                nb, f2, g2, th2, pf, pg, madj);                                        \
         sf[3 * e + KB] = make_float4(pf[0].x, pf[1].x, pf[2].x, REV ? pg[0].x : R(0));                 \
         if (REV) sg[3 * e + KB] = make_float2(pg[1].x, pg[2].x);                                       \
         if (e2 < cnt) {                                                                                \

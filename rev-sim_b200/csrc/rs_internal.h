@@ -128,6 +128,8 @@ constexpr int step_cta_mols(bool fp32, bool rev, int U, int G, int mols) {
 constexpr int half_nreg(bool rev) { return rev ? RS_NREG_HALF_REV : 128; }
 constexpr int half_max_threads(bool rev) { return max_threads_for(half_nreg(rev)); }
 
+constexpr int kSMs = 148;
+
 // Molecules per CTA that leave the busiest SM the fewest molecules when all run as one wave of
 // CTAs, at G lanes each; 0 when no count fits one wave (by the registers).  blocks(m): the CTAs of m
 // molecules, of which none straddles two replicas.
@@ -136,7 +138,7 @@ int one_wave_mols(bool fp32, bool rev, int U, int G, const F &blocks) {
     const int cap = step_max_threads(fp32, rev, U) / 32;   // warps an SM holds
     int best = 0, load = 0;
     for (int m = 32 / G; m <= 32; m += 32 / G) {
-        const int ctas = (blocks(m) + 147) / 148, warps = m * G / 32 + update_warps(m);
+        const int ctas = (blocks(m) + kSMs - 1) / kSMs, warps = m * G / 32 + update_warps(m);
         if (ctas * warps > cap || (best && ctas * m > load)) continue;
         best = m;
         load = ctas * m;

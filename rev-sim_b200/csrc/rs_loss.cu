@@ -578,7 +578,7 @@ cudaError_t launch_rdf_loss(const RdfArgs &a, const RdfSlice &sl, const RdfDen &
     const int groups = (max_n1 + kRlWarps - 1) / kRlWarps;
     const int tiles = ((a.sel1 == a.sel2 ? max_n1 / 2 + kRlWarps : max_n2) + kRlTile - 1) / kRlTile;
     int split = 1;
-    while (split < tiles && (long long)groups * R * split < 2 * 148) split++;
+    while (split < tiles && (long long)groups * R * split < 2 * kSMs) split++;
     // a lane per slice point of a pair's window where 16 or 32 cover it and the factors stay finite
     const double points = 2.0 * a.cutoff / (sl.sd * a.step) * (1.0 - 1e-9);
     const bool finite = 4.0 * a.cutoff * a.cutoff <= 300.0 * a.width;

@@ -339,7 +339,7 @@ __global__ void k_mlp_wgrad_sum(int C, const double *part, double *dtheta) {
 
 // Scratch of the FP64 network: activations, the weight-gradient partials of one launch (two
 // CTAs per SM), the node arrays u, du, au, ad and the node adjoints of a batch of replicas.
-constexpr int kWgradCtas = 296, kWgradReps = 16;
+constexpr int kWgradCtas = 2 * kSMs, kWgradReps = 16;
 constexpr size_t kActLen = (size_t)MLP_NT * (NG + 1) * NA, kPartLen = (size_t)kWgradCtas * MLP_PER_TYPE,
                  kNodeLen = (size_t)MLP_NT * (NG + 1);
 constexpr size_t kNodesSmem = sizeof(double) * H * kW2Ld,

@@ -599,7 +599,7 @@ cudaError_t launch_mlp_tc_eval(const double *theta, int nt, double rc, double w,
                                double *u, double *du, cudaStream_t st) {
     if (nt < 1 || nt > MLP_NT || n < 1) return cudaErrorInvalidValue;
     const int ntile = (n + 15) / 16;
-    const int blocks = std::min((ntile + 3) / 4, 4 * 148);
+    const int blocks = std::min((ntile + 3) / 4, 4 * kSMs);
     k_mlp_tc_fwd<<<dim3(blocks, nt), 128, 0, st>>>(theta, rc, w, n, r, u, du);
     return cudaGetLastError();
 }

@@ -14,12 +14,8 @@
 
 namespace rs {
 
-template <typename R> struct PkT;
-template <> struct PkT<float> { using T = float2; };
-
 __device__ __forceinline__ float2 pk(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 pk1(float a) { return make_float2(a, a); }
-__device__ __forceinline__ double2 pk1(double a) { return make_double2(a, a); }
 
 // a - b as fma(b, -1, a): b * -1 is exact, so the one rounding gives the bits of
 // __fsub_rn(a, b).
