@@ -46,7 +46,7 @@ struct revsim_gas_handle {
            *d_ac = nullptr, *d_part = nullptr, *d_epart = nullptr, *d_direct = nullptr,
            *d_gtail = nullptr, *d_Eloss = nullptr;
     size_t eloss_cap = 0;
-    // gather buffers (32 B per atom: double4 in FP64, float4 in mixed precision) and the FP64
+    // gather buffers ([3][N] components, double in FP64, float in mixed precision) and the FP64
     // copy pos64 of the positions (aliases d_pos in FP64)
     void *d_pos[2] = {nullptr, nullptr}, *d_wgt[2] = {nullptr, nullptr};
     double *d_pos64[2] = {nullptr, nullptr};

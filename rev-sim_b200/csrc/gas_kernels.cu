@@ -209,8 +209,8 @@ __device__ __forceinline__ void store_pos(int N, int nw3, double L, int i, const
     posf[c] = test_pos(x, atom_mol(i, nw3), L);
 }
 
-// R: pair arithmetic (float in mixed precision, double in FP64).  The pair loop gathers
-// V4T<R> positions and weights; the per-lane sums are R and are combined in FP64; the
+// R: pair arithmetic (float in mixed precision, double in FP64).  The pair loop gathers R
+// positions and weights, [3][N] components; the per-lane sums are R and are combined in FP64; the
 // bonded terms and the integrator run in FP64 on the FP64 gather copy pos64.
 //
 // The first a.apc warps are the pair warps.  Each walks its atom's row in two phases.  Phase 1:
@@ -227,8 +227,8 @@ __device__ __forceinline__ void store_pos(int N, int nw3, double L, int i, const
 // Bound by the latency of a row's gathers and FP64 chains at five warps a scheduler (ncu, forward:
 // 2,670 warp instructions an atom, FP64 pipe 15 %, L1 34 %; loads and fixed latencies are the
 // stalls).  Evaluating two or three queued entries a lane at a time, or testing six or eight entries
-// a lane, changed nothing (13.1-13.8 | 19.7-21.7 us).  2,675 atoms, FP64, LJ: 13.6 us a forward and
-// 19.3 us a reverse step; 19.3 and 32.8 us with the FP64 test on every entry, the displacements in the
+// a lane, changed nothing (13.1-13.8 | 19.7-21.7 us).  2,675 atoms, FP64, LJ: 13.7 us a forward and
+// 19.4 us a reverse step; 19.3 and 32.8 us with the FP64 test on every entry, the displacements in the
 // queue, and the bonded terms and integrator on lane 0 of every pair warp.
 template <typename R, int FORM, bool REV>
 __global__ void __maxnreg__((gas_nreg(sizeof(R) == 4, FORM == F_LJ, REV)))

@@ -455,9 +455,10 @@ int launch_step_k(revsim_handle *h, bool rev, const StepArgs &a_in) {
     a.shift_box = h->shift_min();
     // When the next step's CTAs may become resident: at once if every SM has at most one CTA;
     // otherwise not before this step's CTAs are past their barrier, since CTAs that wait beside
-    // an uneven last wave leave the next step uneven too (3,000 waters, mixed: 23.5 | 30.6 us a
-    // forward | reverse step with the early release, 18.3 | 25.7 with the late one, 20.0 | 26.6
-    // unchained; 895 waters FP64: 12.7 us a forward step early, 15.2 late).
+    // an uneven last wave leave the next step uneven too (3,000 waters, mixed, in 375 CTAs of eight
+    // molecules: 23.5 | 30.6 us a forward | reverse step with the early release, 18.3 | 25.7 with the
+    // late one, 20.0 | 26.6 unchained; 895 waters FP64 in 128 CTAs: 12.7 us a forward step early,
+    // 15.2 late).
     a.chain_early = sh.n_blk <= kSMs;
     const BondConsts bc = bond_consts(h);
     const bool timed = h->ktime && !(a.mode & MODE_FORCES_ONLY);

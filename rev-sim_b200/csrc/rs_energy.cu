@@ -29,7 +29,7 @@ __device__ __forceinline__ double near_int64(double a, double b) {
 // memory and evaluated 32 at a time, the nine atom pairs of an entry as straight-line code with
 // the pairs outside the mask or the cutoff at weight zero.  FP64-pipe bound.  With 16 lanes a
 // molecule, each walking its entries pair by pair past the skipped ones: 124 us on the 895-water
-// box, 133 us on 3,000 waters; this form: 16 and 18 us.
+// box, 133 us on 3,000 waters; this form: 18 and 19 us.
 template <int FORM, typename V4>
 __global__ void __launch_bounds__(EG_THREADS) k_energy_grads(EnergyArgs a) {
     __shared__ uint32_t s_q[EG_WARPS][64];

@@ -77,7 +77,7 @@ struct BondConsts {
 
 // Register budget per thread of the step kernels (__maxnreg__), by precision, direction and
 // loop form U; a scheduler's 16,384 registers then hold: FP32 forward seven warps, reverse five
-// (U = 1) or four; FP64 forward four, reverse three (U = 1) or two.
+// (U = 1) or four; FP64 forward four (U = 3: two), reverse three (U = 1) or two.
 #ifndef RS_NREG_F_FWD
 #define RS_NREG_F_FWD 72
 #endif
@@ -151,9 +151,9 @@ int one_wave_mols(bool fp32, bool rev, int U, int G, const F &blocks) {
 // per CTA, by the molecules M of all replicas.  While one wave holds them at 32 lanes, 32 lanes;
 // then 16 (fewer idle lanes at the rows' ends), in one wave as long as that goes, else in CTAs of
 // four or five pair warps that fill the register file.  Within one wave the busiest SM sets the
-// time, hence one_wave_mols (3,000 waters, mixed, 16 lanes: 22 molecules in 137 CTAs 17.7 | 23.7
+// time, hence one_wave_mols (3,000 waters, mixed, 16 lanes: 22 molecules in 137 CTAs 17.3 | 23.5
 // us a forward | reverse step, 8 in 375 18.3 | 26.1, 12 in 250 19.5 | 28.0; 2,001 at 32 lanes: 14
-// 13.7 | 16.9, 4 14.9 | 19.2).  FP64's reverse kernel holds seven molecules an SM with the
+// 13.4 | 16.9, 4 14.9 | 19.2).  FP64's reverse kernel holds seven molecules an SM with the
 // registers it wants, and stays at 32 lanes up to 4,000 all the same (3,600: 32 | 59 at 32 lanes, 34 | 62
 // at 16; 4,200: 39 | 73 and 37 | 67; 5,000: 42 | 78 and 42 | 82; 6,500: 51 | 101 and 48 | 96).  The FP32
 // reverse kernel's second entry pays while its 128 registers hold the molecules (895: 12.0 and 12.7 with

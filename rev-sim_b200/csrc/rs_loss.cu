@@ -570,7 +570,7 @@ RdfDen rdf_den_poly(double step, double width, double cutoff) {
 }
 
 // split: CTAs per eight first atoms, so that small boxes still fill the SMs; ncopy: as many
-// shared-memory copies of the slice sums (a power of two, at most 8) as 32 KB hold.
+// shared-memory copies of the slice sums (a power of two, at most 32) as kRlSmem holds.
 cudaError_t launch_rdf_loss(const RdfArgs &a, const RdfSlice &sl, const RdfDen &dn, int R, int max_n1, int max_n2,
                             const double *pre, const double *target, int norm, double weight, bool grad,
                             double *loss, cudaStream_t st) {

@@ -212,7 +212,7 @@ __global__ void k_mlp_adj_nodes(const double *cadj, int ncopy, int nt, double rc
 __global__ void __launch_bounds__(kMlpThreads) k_mlp_wgrad(const double *theta, double rc, double w, int nt,
                                                            const double *act, const double *au,
                                                            const double *ad, double *part) {
-    extern __shared__ double s_dyn[];   // W2 [H][kW2Ld], then seven [kNodes][H] arrays
+    extern __shared__ double s_dyn[];   // W2 [H][kW2Ld], then six [kNodes][H] arrays
     double *s_w2 = s_dyn;
     using Row = double[H];
     Row *s_h = (Row *)(s_dyn + H * kW2Ld), *s_dh = s_h + kNodes, *s_z2 = s_dh + kNodes, *s_dz2 = s_z2 + kNodes,

@@ -266,7 +266,7 @@ __host__ __device__ constexpr bool charge_from_forces(int form) { return form !=
 // One entry per lane in both precisions.  FP32 took two entries per lane in packed arithmetic
 // before: that halves the instructions but not the FMA pipe's time, and the second entry's
 // operands held the reverse kernel at 168 registers, 12 warps an SM and 35 % issue (16 x 895
-// waters at 16 lanes: 108 us a reverse and 66 us a forward step); one entry runs at 96
+// waters at 16 lanes, event-timed: 108 us a reverse and 66 us a forward step); one entry runs at 96
 // registers, 20 warps and 65 % issue (90 and 52 us).
 template <typename R, int FORM, bool REV, int KA, int KB>
 __device__ __forceinline__ void pair_term(bool bit, R dx, R dy, R dz, const typename V4T<R>::T &wa,
@@ -607,10 +607,10 @@ constexpr int step_maxnreg() {
 // nearly all with 1-3 lanes active, and its latency came before and after the row's.
 //
 // Bound by instruction issue (65 % at 16 x 895 waters, FMA pipe 47 %) where molecules are many
-// and by the latency of one row where they are few.  Event-timed us per forward | reverse step
-// at the default shapes, with the former kernels and now: mixed 895 waters 16.8 | 21.8 -> 12.8 |
-// 16.7, 3,000 27.2 | 42 -> 18.8 | 29, 16 x 895 85 | 150 -> 52 | 90; FP64 895 25 | 43 -> 16.6 |
-// 20.9, 3,000 47.5 | 97 -> 29 | 50, 16 x 895 159 | 338 -> 90 | 185.
+// and by the latency of one row where they are few.  us per forward | reverse step at the
+// default shapes (a pass's time per step, launches chained), with the former kernels and now: mixed 895
+// waters 13.7 | 17.2 -> 10.0 | 11.9, 3,000 27.0 | 45.8 -> 17.3 | 23.5, 16 x 895 92 | 196 -> 53 | 86; FP64
+// 895 22.7 | 38.5 -> 12.5 | 17.1, 3,000 46.5 | 95.5 -> 25.6 | 47.0, 16 x 895 166 | 337 -> 90 | 182.
 template <typename R, int FORM, int G, bool REV, int U>
 __global__ void __maxnreg__((step_maxnreg<R, REV, U>())) k_water_step(StepArgs a, NbConsts<R> nb,
                                                                       BondConsts bc) {

@@ -77,7 +77,7 @@ __global__ void k_cell_count(SwNlArgs a) {
 
 // Exclusive scan of the cell counts, one CTA per replica (its cells hold its atoms, so its scan
 // starts at its first atom): every pass takes two consecutive cells a thread, a shuffle scan a warp
-// and one scan of the warps' sums.  16 replicas of 1,728 cells: under 4 us; 40 us in one CTA with
+// and one scan of the warps' sums.  16 replicas of 1,331 cells: under 4 us; 40 us in one CTA with
 // one cell a thread and a barrier per doubling.
 __global__ void __launch_bounds__(1024) k_cell_scan(SwNlArgs a) {
     constexpr int PER = 2;
@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS) k_rows(SwNlArgs a) {
 // S1 = sum h_q' c3 (c3 alpha_q - cos beta_q), V = sum h_q' c3 u_q'.
 //
 // Bound by instruction issue (65 %; half of a group's lanes hold a slot).  16 x 8,000 atoms, FP32
-// terms, learned pair term, 16 lanes a centre: 140 us with tangents and contraction, 65 us values
-// only.  202 and 74 us with four tangents carried through dual numbers (94 registers, 20 warps an
+// terms, learned pair term, 16 lanes a centre: 144 us with tangents and contraction, 67 us values
+// only (event-timed).  205 and 75 us with four tangents carried through dual numbers (94 registers, 20 warps an
 // SM) and vec1d's comparisons on every candidate; at 64 registers, some spilled, 32 warps fit (154 ->
 // 149 us).
 template <typename R, int G, int MODE>
