@@ -200,8 +200,8 @@ __global__ void k_rdf(RdfArgs a) {
 // loops that few lanes repeat left a warp's lanes apart for the whole pair (66 us instead of 38 a
 // gradient on the 895-water box).
 //
-// Bound by FP64 latency at 16 to 24 warps an SM (three CTAs an SM at 80 registers suit PTS = 16
-// only: 60 -> 54 us; the others slow by 3-5 us).  Us per value / gradient, mean over the O-O and O-H
+// Bound by FP64 latency at 16 to 24 warps an SM (three CTAs an SM at 80 registers suit PTS = 16, 60 ->
+// 54 us, and PTS = 0, 3,000 waters, O-H, 400 points a window 7.8 -> 4.7 ms; the others slow by 3-5 us).  Us per value / gradient, mean over the O-O and O-H
 // terms of the experimental grid (4,801 points, of which the loss reads 248 and 281; 27 a window)
 // on the 895-water box, and the 200-bin O-O term (16 a window) on the 3,000-water box: every
 // ordered pair over the whole grid, as k_rdf does, 567 / 535 and 215 / 298; a lane per pair with
@@ -211,7 +211,7 @@ constexpr int kRlWarps = 8, kRlTile = 256;
 constexpr size_t kRlSmem = 65536;   // dynamic shared memory of a value CTA at most
 
 template <bool GRAD, int PTS>
-__global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_rdf_loss(RdfArgs a, RdfSlice sl, RdfDen dn, int split,
+__global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS != 32 ? 3 : 0) k_rdf_loss(RdfArgs a, RdfSlice sl, RdfDen dn, int split,
                                                             int ncopy) {
     constexpr bool COOP = !GRAD && PTS > 0;
     constexpr int W = PTS ? PTS : 32;   // lanes a pair
@@ -232,9 +232,10 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
     // tile positions p of the CTA: atom (i0 + 1 + p) mod n for equal sets, atom p otherwise
     const int half = n1 / 2;
     const int np = same ? half + kRlWarps - 1 : n2;
-    const int ntile = (np + kRlTile - 1) / kRlTile;
-    const int t0 = (int)((long long)ntile * part / split), t1 = (int)((long long)ntile * (part + 1) / split);
-    if (t0 >= t1) return;
+    const int nunit = (np + 31) / 32;   // the CTA's share of the positions, in units of a warp's test
+    const int p0 = 32 * (int)((long long)nunit * part / split),
+              p1 = min(np, 32 * (int)((long long)nunit * (part + 1) / split));
+    if (p0 >= p1) return;
     const double L = a.rep_box[r];
     const float Lf = (float)L, hLf = 0.5f * Lf;
     const double inv_w = __drcp_rn(a.width);
@@ -407,11 +408,11 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
     };
 
     int nq = 0;
-    for (int t = t0; t < t1; t++) {
+    for (int pt = p0; pt < p1; pt += kRlTile) {
         __syncthreads();
         {
-            const int p = t * kRlTile + threadIdx.x;
-            if (p < np) {
+            const int p = pt + threadIdx.x;
+            if (p < p1) {
                 const int j = same ? (i0 + 1 + p) % n1 : p;
                 const double *xj = a.x + 3 * (size_t)rdf_atom(a.sel2, atom0, j);
 #pragma unroll
@@ -419,11 +420,11 @@ __global__ void __launch_bounds__(32 * kRlWarps, !GRAD && PTS == 16 ? 3 : 0) k_r
             }
         }
         __syncthreads();
-        for (int b = 0; b < kRlTile; b += 32) {
-            const int p = t * kRlTile + b + lane;
+        for (int b = 0; b < kRlTile && pt + b < p1; b += 32) {
+            const int p = pt + b + lane;
             // equal sets: k = j - i before the ring's wrap
             const int k = i0 + 1 + p - i;
-            bool ok = p < np && (same ? k >= 1 && k <= kmax : live);
+            bool ok = p < p1 && (same ? k >= 1 && k <= kmax : live);
             if (ok) {
                 float r2 = 0.f;
 #pragma unroll
@@ -569,21 +570,30 @@ RdfDen rdf_den_poly(double step, double width, double cutoff) {
     return dn;
 }
 
-// split: CTAs per eight first atoms, so that small boxes still fill the SMs; ncopy: as many
+// split: CTAs per eight first atoms.  Two an SM, of whole tiles while every SM has one at least, else of
+// less (150 waters, O-H, 700 points of which 41 a window, value alone: 51 us a call, 121 with two tiles
+// a group, 53 as k_rdf does it).  A lane per pair evaluates long windows, three CTAs an SM, and their
+// CTAs' times differ: nine an SM (895 waters, O-H, value alone, 200 points a window 572 us a call,
+// 694 with three an SM, 1,009 with two, 724 as k_rdf; 160 points a window of 4,000 785 and 805).  ncopy: as many
 // shared-memory copies of the slice sums (a power of two, at most 32) as kRlSmem holds.
 cudaError_t launch_rdf_loss(const RdfArgs &a, const RdfSlice &sl, const RdfDen &dn, int R, int max_n1, int max_n2,
                             const double *pre, const double *target, int norm, double weight, bool grad,
                             double *loss, cudaStream_t st) {
     if (sl.nt < 1) return cudaSuccess;
     const int groups = (max_n1 + kRlWarps - 1) / kRlWarps;
-    const int tiles = ((a.sel1 == a.sel2 ? max_n1 / 2 + kRlWarps : max_n2) + kRlTile - 1) / kRlTile;
-    int split = 1;
-    while (split < tiles && (long long)groups * R * split < 2 * kSMs) split++;
+    const int np = a.sel1 == a.sel2 ? max_n1 / 2 + kRlWarps : max_n2;
+    const int tiles = (np + kRlTile - 1) / kRlTile, units = (np + 31) / 32;
     // a lane per slice point of a pair's window where 16 or 32 cover it and the factors stay finite
     const double points = 2.0 * a.cutoff / (sl.sd * a.step) * (1.0 - 1e-9);
     const bool finite = 4.0 * a.cutoff * a.cutoff <= 300.0 * a.width;
     const auto coop_smem = [&](int pts) { return sizeof(double) * (64 / pts) * kRlWarps * (size_t)sl.nt; };
     const int pts = !finite ? 0 : points <= 16.0 && coop_smem(16) <= kRlSmem ? 16 : points <= 32.0 && coop_smem(32) <= kRlSmem ? 32 : 0;
+    const auto ctas = [&](int s) { return (long long)groups * R * s; };
+    const int want = (pts ? 2 : 9) * kSMs;
+    int split = 1;
+    while (split < tiles && ctas(split) < want) split++;
+    if (ctas(split) < (pts ? kSMs : want))
+        while (split < units && ctas(split) < want) split++;
     int ncopy = 32;
     while (ncopy > 0 && sizeof(double) * ncopy * (size_t)sl.nt > kRlSmem) ncopy >>= 1;
     const auto value = pts == 16 ? k_rdf_loss<false, 16> : pts == 32 ? k_rdf_loss<false, 32> : k_rdf_loss<false, 0>;

@@ -56,3 +56,20 @@ def test_no_weight_at_zero():
     args = (0, 1, 0.0, 0.005, 0.002, 0.15, 100, 0, 1, np.ones(100), 1, 0.0)
     _, g = _loss_grad(x, args)
     assert not g.any()
+
+
+@pytest.mark.parametrize("n_mol", [31, 33, 257, 300])
+@pytest.mark.parametrize("sel", [(0, 0), (0, 1), (1, 1)])
+def test_long_windows(n_mol, sel):
+    """Windows of 100 points (a lane per pair, CTAs of less than a tile)."""
+    x = systems.water_coords(n_mol, BOX, seed=n_mol)
+    args = (*sel, 0.005, 0.005, 0.002, 0.25, 200, 0, 1, np.random.default_rng(n_mol).uniform(0.2, 1.5, 200), 2, 0.7)
+    lo, go = orc.loss_grad(orc.make_system(n_mol, BOX), orc.Loss([orc.RdfTerm(*args)]), x)
+    e = Engine(n_mol, BOX)
+    e.set_params(C.default_params())
+    e.set_state(x, np.zeros_like(x))
+    e.set_loss([RdfTerm(*args)])
+    l, g = e.loss_grad()
+    e.close()
+    assert abs(l[0] - lo) <= 1e-11 * abs(lo)
+    assert np.linalg.norm(g - go) <= 1e-11 * np.linalg.norm(go)
